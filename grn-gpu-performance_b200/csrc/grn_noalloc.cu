@@ -137,38 +137,45 @@ extern "C" grn_status grn_evaluate_batch_noalloc(
   int n_sm = 0, optin = 0;
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-  const int W = params->dim_x, H = params->dim_y, Wg = (W + 3) / 4, Q = H * Wg;
+  const int W = params->dim_x, H = params->dim_y;
   const bool ragged = (W % 4) != 0;
   const size_t plane_bytes = (size_t)plane_floats(W, H) * sizeof(float);
   const size_t fixed = sim_fixed_smem_bytes();
   int fit = (size_t)optin > fixed ? (int)(((size_t)optin - fixed) / plane_bytes) : 0;
   fit &= ~1;
-  const int gmax = ph.max_genes;
+  const int max_genes = ph.max_genes;
+  // State slots are sized for a class of 4, 8 or 16 genes.
+  const int gmax = max_genes <= 4 ? 4 : max_genes <= 8 ? 8 : GRN_MAX_GENES;
+  const int chunks = strip_chunks(W, H);
   LaunchPlan best{};
   best.cluster = 1;
   double best_score = -1;
   for (int i = 0; i < sim_variant_count(); ++i) {
     const KernelVariant v = sim_variant(i);
-    if (v.cluster || v.trace || v.stream || v.gmax < gmax || v.ragged != ragged || (!v.loop && Q > v.threads * v.items))
-      continue;
-    const int planes = std::min(fit, 2 * gmax);
+    if (v.cluster || v.trace || v.stream || v.ragged != ragged) continue;
+    const int parts = std::min({v.max_threads / 32 / chunks, 4, std::max(1, max_genes)});
+    if (!v.loop && parts < 1) continue;  // more chunks than warps
+    const int threads = v.loop ? v.max_threads : chunks * parts * 32;
+    const int planes = std::min(fit, 2 * max_genes);
     const size_t smem = fixed + planes * plane_bytes;
     int occ = 0;
-    if (sim_occupancy(v, smem, &occ) != cudaSuccess || occ < 1) continue;
-    const double score = (double)occ * std::min(v.threads, Q) * (v.loop ? 1.0 : 1.25) - 1e-3 * v.gmax;
+    if (sim_occupancy(v, threads, smem, &occ) != cudaSuccess || occ < 1) continue;
+    const double score = (double)occ * threads * (v.loop ? 1.0 : 1.25);
     if (score > best_score) {
       best_score = score;
       best.v = v;
       best.schedule = v.loop ? GRN_SCHEDULE_WALK_ITEMS : GRN_SCHEDULE_FIXED_ITEMS;
+      best.threads = threads;
+      best.gmax = gmax;
       best.planes = planes;
       best.smem_bytes = smem;
       best.blocks_per_sm = occ;
-      best.slot_floats = planes / 2 < gmax ? 2LL * v.gmax * plane_floats(W, H) : 0;
+      best.slot_floats = planes / 2 < max_genes ? 2LL * gmax * plane_floats(W, H) : 0;
     }
   }
   if (best_score < 0)
     return put_error(err_buf, err_buf_len, GRN_ERR_CAPACITY,
-                     "no kernel variant holds " + std::to_string(gmax) + " genes on this grid");
+                     "no kernel variant holds " + std::to_string(max_genes) + " genes on this grid");
   int blocks = std::max(1, std::min(batch->n_models, n_sm * best.blocks_per_sm));
   if (best.slot_floats > 0) {
     // As many persistent blocks as the scratch has state slots for.
@@ -202,9 +209,8 @@ extern "C" grn_status grn_evaluate_batch_noalloc(
   a.n_exp = n_experiments;
   a.n_in = params->n_input_morphogens;
   a.n_target = params->n_target_morphogens;
-  a.W = W;
-  a.H = H;
-  a.Wg = Wg;
+  set_geometry(&a, W, H, 1);
+  a.gmax = best.gmax;
   a.n_steps = params->num_sim_steps;
   a.fitness_kind = params->fitness_kind;
   a.planes = best.planes;
@@ -214,6 +220,7 @@ extern "C" grn_status grn_evaluate_batch_noalloc(
   a.dt = (float)params->dt;
   a.min_conc = (float)params->min_conc;
   a.min_conc_change = params->min_conc_change;
+  a.change_bound = float_below(a.min_conc_change);
   a.dist_threshold = params->dist_error_threshold;
   a.initial = d_initial;
   a.target = d_target;

@@ -34,11 +34,10 @@ constexpr int kConstSlot = 255;
 
 // Header flags.
 constexpr uint32_t kFlagNone = 0u;
-// Every link has a finite K > 0, a finite Hill coefficient n <= 32 and
-// 0 < K^n <= 1e300, every gene finite rates, and no (regulator, regulated)
-// pair repeats: on a bounded non-negative state no link term can be NaN, so
-// the kernel may combine terms with min/max over a dense per-gene table of
-// regulator slots (see the kernel's regulation).  pack_batch also clears
+// Every link has a finite K > 0, a finite Hill coefficient 0 < n <= 32 and
+// 0 < K^n <= 1e300, and every gene finite rates: on a bounded non-negative
+// state no link term can be NaN or constant, so the kernel may combine terms
+// with min/max (see the kernel's regulation).  pack_batch also clears
 // the flag where the run's step size could leave the state unbounded
 // (euler_bounded in host/pack.h), so the kernel tests only the flag.
 constexpr uint32_t kFlagFast = 1u;

@@ -7,6 +7,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <cmath>
+
 #include "grn_packed.h"
 
 namespace grn {
@@ -22,6 +24,11 @@ struct SimArgs {
   int32_t n_target;          // target morphogens
   int32_t W, H;              // grid width (x) and height (y)
   int32_t Wg;                // float4 groups per row = ceil(W / 4)
+  uint32_t inv_wg;           // ceil(2^32 / Wg) (unused when Wg is 1)
+  int32_t row_floats, row_bytes;      // one padded state row
+  int32_t plane_floats, plane_bytes;  // one state plane (of a CTA's band)
+  int32_t gmax;              // genes a global state slot (or a streaming
+                             // stage) holds
   int32_t n_steps;           // max Euler steps per experiment
   int32_t fitness_kind;      // grn_fitness_kind
   int32_t planes;            // shared-memory state planes per block (even)
@@ -30,6 +37,8 @@ struct SimArgs {
   float dt;
   float min_conc;
   double min_conc_change;
+  float change_bound;        // the largest float <= min_conc_change: a step's
+                             // change (a float) exceeds both or neither
   double dist_threshold;
   const float *initial;      // [n_exp][n_in][H][W]
   const float *target;       // [n_exp][n_target][H][W]
@@ -56,10 +65,9 @@ constexpr int32_t kHookWithholdBandCopy = 1;  // streaming: band 1's copy is nev
 
 // One compiled kernel variant.
 struct KernelVariant {
-  int threads;  // threads per block
-  int gmax;     // most genes a model may have
-  int items;    // float4 groups each thread owns (fixed items)
-  bool loop;    // threads walk the grid's groups (any grid size)
+  int max_threads;  // most threads per block
+  bool loop;    // warps walk the grid's strips (any grid size); else a warp
+                // owns one chunk of 32 strips (strip_chunks)
   bool ragged;  // compiled for W not a multiple of 4
   bool cluster; // cluster-split: a cluster of CTAs per model, one band of
                 // rows each
@@ -72,6 +80,8 @@ struct KernelVariant {
 struct LaunchPlan {
   KernelVariant v;
   int schedule;          // grn_schedule actually used
+  int threads;           // threads per block (whole warps)
+  int gmax;              // genes per global state slot or streaming stage
   int blocks;            // persistent grid size
   int planes;            // state planes in shared memory (even; may be 0)
   size_t smem_bytes;     // dynamic shared memory
@@ -95,11 +105,46 @@ GRN_HOST_DEVICE inline int row_floats(int W) {
   return 4 * ((W + 3) / 4) + (W % 4 == 0 ? 4 : 0);
 }
 
+// Rows of a strip, the cells one thread computes: 4 columns x 2 rows.
+// Measured on 64 x 64 (2368 models x 400 steps, G cell-updates/s): 1 row
+// 169, 2 rows 189, 4 rows 179 (a 4-row strip needs 120 registers: half the
+// warps).
+constexpr int kStripRows = 2;
+// Rows a plane holds for `rows` rows of the grid: whole strips, so that a
+// thread may read past the last row.
+GRN_HOST_DEVICE inline int strip_rows(int rows) {
+  return (rows + kStripRows - 1) / kStripRows * kStripRows;
+}
+
 // Floats of one state plane of a W x H grid: padded rows plus a zero row
 // above and below (see the kernel's Geom).  With a cluster of C CTAs per
 // model a CTA's plane holds a band of ceil(H / C) rows.
 inline int64_t plane_floats(int W, int H, int cluster = 1) {
-  return (int64_t)((H + cluster - 1) / cluster + 2) * row_floats(W);
+  return (int64_t)(strip_rows((H + cluster - 1) / cluster) + 2) * row_floats(W);
+}
+
+// Chunks of 32 strips of `rows` rows of a W-wide grid: a warp's unit of
+// work.
+inline int strip_chunks(int W, int rows) {
+  return ((strip_rows(rows) / kStripRows) * ((W + 3) / 4) + 31) / 32;
+}
+
+// SimArgs::change_bound.
+inline float float_below(double x) {
+  const float f = (float)x;
+  return (double)f > x ? std::nextafter(f, -HUGE_VALF) : f;
+}
+
+// The launch geometry of a W x H grid split over `cluster` CTAs per model.
+inline void set_geometry(SimArgs *a, int W, int H, int cluster) {
+  a->W = W;
+  a->H = H;
+  a->Wg = (W + 3) / 4;
+  a->inv_wg = a->Wg > 1 ? (uint32_t)((((uint64_t)1 << 32) + a->Wg - 1) / a->Wg) : 0u;
+  a->row_floats = row_floats(W);
+  a->row_bytes = 4 * a->row_floats;
+  a->plane_floats = (int32_t)plane_floats(W, H, cluster);
+  a->plane_bytes = 4 * a->plane_floats;
 }
 
 // Bytes of shared memory a block needs besides the state planes.
@@ -109,16 +154,16 @@ size_t sim_fixed_smem_bytes();
 int sim_variant_count();
 KernelVariant sim_variant(int i);
 
-// Occupancy of a variant with `smem_bytes` dynamic shared memory: resident
+// Occupancy of a variant with blocks of `threads` and `smem_bytes` dynamic shared memory: resident
 // blocks per SM (0 if it does not fit).  Sets the function's max dynamic
 // shared memory attribute as a side effect.
-cudaError_t sim_occupancy(const KernelVariant &v, size_t smem_bytes,
+cudaError_t sim_occupancy(const KernelVariant &v, int threads, size_t smem_bytes,
                           int *blocks_per_sm);
 
 // Cluster-split variant: resident clusters of `cluster` CTAs on the device
 // (0 if it does not fit).
-cudaError_t sim_cluster_occupancy(const KernelVariant &v, size_t smem_bytes, int cluster,
-                                  int *clusters);
+cudaError_t sim_cluster_occupancy(const KernelVariant &v, int threads, size_t smem_bytes,
+                                  int cluster, int *clusters);
 
 // Launches a variant; the caller has zeroed args.work_counter on `stream`.
 cudaError_t sim_launch(const LaunchPlan &plan, const SimArgs &args,

@@ -13,13 +13,15 @@
 //     (one barrier per step); genes that do not fit use the same code on
 //     double-buffered global-memory slots, and grids too large for shared
 //     memory stream bands of rows through it (or split across a cluster);
-//   - each thread owns float4 groups of 4 cells along x; up/down
-//     neighbours come from 128-bit loads, left/right ones from 32-bit loads
-//     next to the group (every padded row ends in zero cells, so a row's
-//     borders read 0 without tests);
-//   - regulation is evaluated in exponent form (grn_packed.h): lg2 once per
-//     regulator gene and cell, one FMA + compare/select per link, and
-//     ex2 + rcp once per regulated gene, on the MUFU pipe;
+//   - the work of a step is cut into warp items: 32 strips of 4 columns x 2
+//     rows, for one gene or all of them (see "the step" below).  A thread
+//     loads its own strip's rows once for both rows' neighbour sums; left and
+//     right neighbours come from 32-bit loads next to the group (every
+//     padded row ends in zero cells, so a row's borders read 0 without
+//     tests);
+//   - regulation is evaluated in exponent form (grn_packed.h): per link lg2
+//     of the regulator's cells, one FMA + min/max, and per regulated gene
+//     ex2 + rcp, on the MUFU pipe;
 //   - the step's max |rate| (early-exit test) is a warp max on the float
 //     bits plus one shared-memory pass; fitness sums are FP64.
 // Semantics follow the reference CPU simulator
@@ -173,26 +175,40 @@ struct ModelSmem {
 constexpr int kModelWords = sizeof(ModelSmem) / 16;
 static_assert(sizeof(ModelSmem) % 16 == 0, "model smem is whole words");
 
-// Dense form of a fast model's regulation, built in shared memory when the
-// model is loaded: for gene p, the regulator slots of its OR links and of
-// its AND links as bitmasks, and the (a, b) of the link from slot k at
-// ab[p][k].  Hill-coefficient-0 links (constant term 0) fold into or_init
-// (min with 0) and and_floor (max with 0).
-struct DenseGene {
-  uint32_t or_slots;
-  uint32_t and_slots;
-  float or_init;    // +inf, or 0 with a constant OR term
-  float and_floor;  // -inf, or 0 with a constant AND term
+// The program in the form the step reads, built in shared memory when a
+// model is loaded.  Coefficients are stored as pairs, so that one load gives
+// the register pairs of the paired FP32 instructions.
+struct GeneSmem {
+  float4 ld;     // lim, lim, -deg, -deg
+  float2 dif;    // dif, dif
+  int ctl;       // GeneCtl fields
+  int pad;
 };
-struct DenseSmem {
-  DenseGene gene[GRN_MAX_GENES];
-  float2 ab[GRN_MAX_GENES][GRN_MAX_GENES];
+struct LinkSmem {
+  float4 ab;     // a, a, b, b
+  int slot;      // regulator, or kConstSlot (exact only)
+  int pad[3];
 };
-static_assert(sizeof(DenseSmem) % 16 == 0, "dense table is whole words");
+struct ProgSmem {
+  GeneSmem gene[GRN_MAX_GENES];      // in the order the splits take them
+  LinkSmem link[GRN_MAX_LINKS + 1];  // the slot after the last is read ahead
+};
+static_assert(sizeof(GeneSmem) == 32 && sizeof(LinkSmem) == 32, "program words");
+
+// GeneSmem::ctl: bits 0-3 the gene, 4 diffuses, 5-12 its first link, 13-20
+// its OR links, 21-28 its links in all (OR first).
+__host__ __device__ constexpr int gene_ctl(int p, bool diffuses, int link, int n_or, int n) {
+  return p | (diffuses ? 16 : 0) | (link << 5) | (n_or << 13) | (n << 21);
+}
+static_assert(GRN_MAX_GENES <= 16 && GRN_MAX_LINKS < 256, "GeneCtl fields");
+
+// A value that is the same in every lane, as one the compiler knows to be:
+// branches on it need no divergence handling.
+__device__ __forceinline__ int uniform(int x) { return __shfl_sync(kFull, x, 0); }
 
 // Fixed shared-memory layout in front of the state planes.
-constexpr size_t kDenseOffset = sizeof(ModelSmem);
-constexpr size_t kRedOffset = kDenseOffset + sizeof(DenseSmem);  // float [2][32]
+constexpr size_t kProgOffset = sizeof(ModelSmem);
+constexpr size_t kRedOffset = kProgOffset + sizeof(ProgSmem);  // float [2][32]
 constexpr size_t kDredOffset = kRedOffset + 2 * 32 * 4;  // double [32]
 constexpr size_t kWorkOffset = kDredOffset + 32 * 8;     // int [2]
 // Cluster exchange slots: per-CTA step maxima float [2][kMaxCluster] (by
@@ -292,6 +308,20 @@ __device__ __forceinline__ float comb_or(float run, float t) { return (run < t) 
 // Reference AND (Hill min) in exponent space.
 __device__ __forceinline__ float comb_and(float run, float t) { return (run > t) ? run : t; }
 
+template <bool B>
+struct Bool {
+  static constexpr bool value = B;
+};
+using True = Bool<true>;
+using False = Bool<false>;
+
+// Hides how a value was computed, so that it stays in a register instead of
+// being computed again at each use (the register-poor variants do that).
+__device__ __forceinline__ int opaque(int x) {
+  asm volatile("" : "+r"(x));
+  return x;
+}
+
 enum CombMode { kOrFast, kAndFast, kOrExact, kAndExact };
 
 template <int MODE>
@@ -302,183 +332,44 @@ __device__ __forceinline__ float comb(float run, float t) {
   else return comb_and(run, t);
 }
 
-template <int MODE>
-__device__ __forceinline__ void comb4(float4 &v, float a, const float4 &x, float b) {
-  v.x = comb<MODE>(v.x, fmaf(a, x.x, b));
-  v.y = comb<MODE>(v.y, fmaf(a, x.y, b));
-  v.z = comb<MODE>(v.z, fmaf(a, x.z, b));
-  v.w = comb<MODE>(v.w, fmaf(a, x.w, b));
-}
-
-// Applies one link to the running exponents of NI groups.  The regulator
-// slot is the same for every thread of the block; each case carries the
-// link's whole work so that the switch stays a (uniform) branch rather than
-// a select chain over all registers.
-template <int NI, int GMAX, int MODE>
-__device__ __forceinline__ void apply_link(float4 (&v)[NI], const PackedLink &lk,
-                                           const float4 (&lg)[NI][GMAX]) {
-#define GRN_CASE(k)                                                   \
-  case k:                                                             \
-    if constexpr (GMAX > k) {                                         \
-      _Pragma("unroll") for (int i = 0; i < NI; ++i)                  \
-          comb4<MODE>(v[i], lk.a, lg[i][k], lk.b);                    \
-    }                                                                 \
-    break;
-  switch (lk.slot) {
-    GRN_CASE(0) GRN_CASE(1) GRN_CASE(2) GRN_CASE(3)
-    GRN_CASE(4) GRN_CASE(5) GRN_CASE(6) GRN_CASE(7)
-    GRN_CASE(8) GRN_CASE(9) GRN_CASE(10) GRN_CASE(11)
-    GRN_CASE(12) GRN_CASE(13) GRN_CASE(14) GRN_CASE(15)
-    default:  // kConstSlot: lg2 value 0, a = b = 0 (Hill coefficient 0)
-#pragma unroll
-      for (int i = 0; i < NI; ++i) comb4<MODE>(v[i], lk.a, f4(0.0f), lk.b);
-      break;
-  }
-#undef GRN_CASE
-}
-
-// Regulation of one gene for NI groups.
-template <int NI, int GMAX, bool EXACT>
-__device__ __forceinline__ void regulation(const ModelSmem &M, const PackedGene &g,
-                                           const float4 (&lg)[NI][GMAX], float4 (&h)[NI]) {
-  const int n_or = g.n_or, n = g.n_or + g.n_and;
-  if (n == 0) {  // OpZero
-#pragma unroll
-    for (int i = 0; i < NI; ++i) h[i] = f4(0.0f);
-    return;
-  }
-  float4 v[NI];
-  // exact: a NaN start makes the first term the initial value; fast: min
-  // over OR terms, then max with each AND term.
-  const float v0 = EXACT ? __int_as_float(0x7fc00000)
-                         : (n_or > 0 ? __int_as_float(0x7f800000) : __int_as_float(0xff800000));
-#pragma unroll
-  for (int i = 0; i < NI; ++i) v[i] = f4(v0);
-  const PackedLink *L = M.links + g.link_begin;
-  int l = 0;
-  for (; l < n_or; ++l) apply_link<NI, GMAX, EXACT ? kOrExact : kOrFast>(v, L[l], lg);
-  for (; l < n; ++l) apply_link<NI, GMAX, EXACT ? kAndExact : kAndFast>(v, L[l], lg);
-#pragma unroll
-  for (int i = 0; i < NI; ++i) {
-    h[i].x = rcp_approx(1.0f + ex2_approx(v[i].x));
-    h[i].y = rcp_approx(1.0f + ex2_approx(v[i].y));
-    h[i].z = rcp_approx(1.0f + ex2_approx(v[i].z));
-    h[i].w = rcp_approx(1.0f + ex2_approx(v[i].w));
-  }
-}
-
-// Regulation of gene p for NI groups from the dense table (fast models):
-// regulator slots are a compile-time loop, so the lg2 values are read with
-// fixed register indices and no per-link dispatch is needed.  The result is
-// the fast combine's: min over OR terms, then max with each AND term (terms
-// are never NaN for fast models, and min/max are order-free).
-// Fast-path combine of one link into 4 running exponents: the terms
-// a * lg2(x) + b for two cells per instruction, then min (OR) or max (AND).
-template <bool AND>
-__device__ __forceinline__ void comb4_fast(float4 &v, float2 ab, const float4 &x) {
-  const float2 t01 = fma2(f2(ab.x), lo2(x), f2(ab.y));
-  const float2 t23 = fma2(f2(ab.x), hi2(x), f2(ab.y));
-  if (AND) {
-    v.x = fmaxf(v.x, t01.x);
-    v.y = fmaxf(v.y, t01.y);
-    v.z = fmaxf(v.z, t23.x);
-    v.w = fmaxf(v.w, t23.y);
-  } else {
-    v.x = fminf(v.x, t01.x);
-    v.y = fminf(v.y, t01.y);
-    v.z = fminf(v.z, t23.x);
-    v.w = fminf(v.w, t23.y);
-  }
-}
-
-template <int NI, int GMAX>
-__device__ __forceinline__ void regulation_dense(const ModelSmem &M, const DenseSmem &D, int p,
-                                                 const float4 (&lg)[NI][GMAX],
-                                                 float4 (&h)[NI]) {
-  const PackedGene &g = M.genes[p];
-  if (g.n_or + g.n_and == 0) {  // OpZero
-#pragma unroll
-    for (int i = 0; i < NI; ++i) h[i] = f4(0.0f);
-    return;
-  }
-  const DenseGene dg = D.gene[p];
-  float4 v[NI];
-#pragma unroll
-  for (int i = 0; i < NI; ++i) v[i] = f4(dg.or_init);
-  const uint32_t os = dg.or_slots, as = dg.and_slots;
-#pragma unroll
-  for (int k = 0; k < GMAX; ++k) {
-    if ((os >> k) == 0u) break;
-    if ((os >> k) & 1u) {
-      const float2 ab = D.ab[p][k];
-#pragma unroll
-      for (int i = 0; i < NI; ++i) comb4_fast<false>(v[i], ab, lg[i][k]);
-    }
-  }
-  if (g.n_or == 0) {
-#pragma unroll
-    for (int i = 0; i < NI; ++i) v[i] = f4(dg.and_floor);
-  } else {
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      v[i].x = fmaxf(v[i].x, dg.and_floor);
-      v[i].y = fmaxf(v[i].y, dg.and_floor);
-      v[i].z = fmaxf(v[i].z, dg.and_floor);
-      v[i].w = fmaxf(v[i].w, dg.and_floor);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < GMAX; ++k) {
-    if ((as >> k) == 0u) break;
-    if ((as >> k) & 1u) {
-      const float2 ab = D.ab[p][k];
-#pragma unroll
-      for (int i = 0; i < NI; ++i) comb4_fast<true>(v[i], ab, lg[i][k]);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < NI; ++i) {
-    const float2 e01 = add2(f2(1.0f), make_float2(ex2_approx(v[i].x), ex2_approx(v[i].y)));
-    const float2 e23 = add2(f2(1.0f), make_float2(ex2_approx(v[i].z), ex2_approx(v[i].w)));
-    h[i].x = rcp_approx(e01.x);
-    h[i].y = rcp_approx(e01.y);
-    h[i].z = rcp_approx(e23.x);
-    h[i].w = rcp_approx(e23.y);
-  }
-}
-
-// Builds the dense table of a fast model (one thread per gene).
-__device__ __forceinline__ void build_dense(const ModelSmem &M, DenseSmem &D, int tid) {
+// Builds the program of the model in M (all threads; a barrier follows).
+// `splits` is the number of warps that share a chunk's genes: the genes are
+// dealt to them in snake order of their cost, so that the splits' loads
+// differ by little.
+__device__ __forceinline__ void build_program(const ModelSmem &M, ProgSmem &P, int splits,
+                                              int tid) {
   const int G = M.hdr.n_genes;
-  if (tid < G) {
-    const PackedGene g = M.genes[tid];
-    DenseGene dg;
-    dg.or_slots = 0u;
-    dg.and_slots = 0u;
-    dg.or_init = __int_as_float(0x7f800000);
-    dg.and_floor = __int_as_float(0xff800000);
-    for (int l = 0; l < g.n_or + g.n_and; ++l) {
-      const PackedLink lk = M.links[g.link_begin + l];
-      const bool is_or = l < g.n_or;
-      if (lk.slot == kConstSlot) {
-        if (is_or) dg.or_init = fminf(dg.or_init, 0.0f);
-        else dg.and_floor = fmaxf(dg.and_floor, 0.0f);
-      } else {
-        if (is_or) dg.or_slots |= 1u << lk.slot;
-        else dg.and_slots |= 1u << lk.slot;
-        D.ab[tid][lk.slot] = make_float2(lk.a, lk.b);
-      }
-    }
-    D.gene[tid] = dg;
+  for (int l = tid; l < M.hdr.n_links; l += blockDim.x) {
+    const PackedLink lk = M.links[l];
+    P.link[l].ab = make_float4(lk.a, lk.a, lk.b, lk.b);
+    P.link[l].slot = lk.slot;
   }
+  if (tid == 0) P.link[M.hdr.n_links].slot = 0;
+  if (tid >= G) return;
+  const PackedGene g = M.genes[tid];
+  const int n = g.n_or + g.n_and;
+  // Rank by cost (links, then index), then the snake deal: round r of the
+  // splits runs backwards in odd full rounds.
+  int rank = 0;
+  for (int q = 0; q < G; ++q) {
+    const int nq = M.genes[q].n_or + M.genes[q].n_and;
+    rank += (nq > n || (nq == n && q < tid)) ? 1 : 0;
+  }
+  const int round = rank / splits, pos = rank - round * splits;
+  const bool back = (round & 1) && (round + 1) * splits <= G;
+  GeneSmem &o = P.gene[round * splits + (back ? splits - 1 - pos : pos)];
+  o.ld = make_float4(g.lim, g.lim, -g.deg, -g.deg);
+  o.dif = f2(g.dif);
+  o.ctl = gene_ctl(tid, g.dif > 0.0f, g.link_begin, g.n_or, n);
 }
 
 // ---- geometry ----------------------------------------------------------
 //
 // A state plane holds the W x H grid as rows of RS = row_floats(W) floats
 // (whole float4 groups, ending in at least one zero cell) plus one zero row
-// above and one below:
-// PS = (H + 2) * RS floats, row y at (y + 1) * RS.  The zero rows make the
+// above and one below, and rows for whole strips (strip_rows):
+// PS = (strip_rows(H) + 2) * RS floats, row y at (y + 1) * RS.  The zero rows
+// make the
 // up/down neighbours of the first and last rows read +0.0, which leaves the
 // reference's neighbour sum unchanged.  Steps write data groups only; when W
 // is not a multiple of 4 the cells past W of a row's last group are written
@@ -490,296 +381,455 @@ __device__ __forceinline__ void build_dense(const ModelSmem &M, DenseSmem &D, in
 // one below (the neighbouring bands' edge rows, pushed into them after every
 // step, or zero at the grid border).
 struct Geom {
-  int W, H, Wg, RS, PS, Q;
-  int y0, Hg;  // first grid row of the band, grid height
+  int W, H, Wg, RS, PS, Q;  // Q: strips of the band
+  int RSb, PSb;             // RS, PS in bytes
+  bool edges;               // chunks do not hold whole rows of groups
+  int y0, Hg;               // first grid row of the band, grid height
+  uint32_t inv_wg;          // ceil(2^32 / Wg): q / Wg by multiplication
 };
 
-// One float4 group a thread owns, with everything a step needs about its
-// position (computed once per launch for fixed items).
-struct Item {
-  int base;           // float offset of the group in a plane
-  float4 tot;         // existing neighbours of each cell (reference `total`)
-  bool valid;         // the group exists (an index past the end is clamped
-                      // onto the last group, computed and not stored)
-  bool v1, v2, v3;    // cells 1..3 of the group exist (cell 0 always does)
-};
-
-__device__ __forceinline__ Item make_item(int y, int gx, bool valid, const Geom &g) {
-  Item it;
-  it.valid = valid;
-  it.base = (y + 1) * g.RS + 4 * gx;
-  const int x0 = 4 * gx;
-  const int yg = y + g.y0;
-  const float tv = (yg > 0 ? 1.0f : 0.0f) + (yg < g.Hg - 1 ? 1.0f : 0.0f);
-  it.tot.x = tv + (x0 > 0 ? 1.0f : 0.0f) + (x0 + 1 < g.W ? 1.0f : 0.0f);
-  it.tot.y = tv + 1.0f + (x0 + 2 < g.W ? 1.0f : 0.0f);
-  it.tot.z = tv + 1.0f + (x0 + 3 < g.W ? 1.0f : 0.0f);
-  it.tot.w = tv + 1.0f + (x0 + 4 < g.W ? 1.0f : 0.0f);
-  it.v1 = x0 + 1 < g.W;
-  it.v2 = x0 + 2 < g.W;
-  it.v3 = x0 + 3 < g.W;
-  return it;
+// Strips of R rows x 4 columns in H rows of Wg groups.
+template <int R>
+__device__ __forceinline__ int strip_count(int H, int Wg) {
+  return ((H + R - 1) / R) * Wg;
 }
 
-__device__ __forceinline__ Item item_at(int q, const Geom &g) {
-  const bool valid = q < g.Q;
-  const int qc = valid ? q : g.Q - 1;
-  const int y = qc / g.Wg;
-  return make_item(y, qc - y * g.Wg, valid, g);
+// The 4 x R cells a thread computes: columns 4gx .. 4gx + 3 of rows y ..
+// y + R - 1.  A strip index past the end is clamped onto the last strip: its
+// values are computed (they are that strip's own) and not stored.  Rows past
+// the grid's last (a plane holds whole strips) are computed from whatever
+// the plane holds there, and neither stored nor part of the max.
+template <int R>
+struct Strip {
+  int base;            // byte offset of the first row's group in a plane
+  int rows;            // rows that exist (1 .. R)
+  bool valid;          // false: nothing is stored
+  bool el, er;         // the left / right neighbour group is not the
+                       // neighbouring lane's
+  bool m1, m2, m3;     // cells 1..3 of the group exist (cell 0 always does)
+  float2 nt[R][2];     // -(existing neighbours) of each cell, as pairs
+};
+
+template <int R>
+__device__ __forceinline__ Strip<R> strip_at(int q, const Geom &g) {
+  Strip<R> s;
+  s.valid = q < g.Q;
+  const int qc = s.valid ? q : g.Q - 1;
+  // Exact while q * Wg < 2^32 (dimensions up to 4096: Wg <= 1024, q < 2^21).
+  const int ys = g.Wg == 1 ? qc : (int)__umulhi((uint32_t)qc, g.inv_wg);
+  const int gx = qc - ys * g.Wg, y = R * ys, x0 = 4 * gx;
+  s.rows = min(R, g.H - y);
+  s.el = gx == 0 || (q & 31) == 0;
+  s.er = gx == g.Wg - 1 || (q & 31) == 31;
+  s.base = 4 * ((y + 1) * g.RS + x0);
+  const int yg = y + g.y0;
+  const float hx = (x0 > 0 ? 1.0f : 0.0f) + (x0 + 1 < g.W ? 1.0f : 0.0f);
+  const float hy = 1.0f + (x0 + 2 < g.W ? 1.0f : 0.0f);
+  const float hz = 1.0f + (x0 + 3 < g.W ? 1.0f : 0.0f);
+  const float hw = 1.0f + (x0 + 4 < g.W ? 1.0f : 0.0f);
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const float tv = (i > 0 || yg > 0 ? 1.0f : 0.0f) + (yg + i + 1 < g.Hg ? 1.0f : 0.0f);
+    s.nt[i][0] = make_float2(-(tv + hx), -(tv + hy));
+    s.nt[i][1] = make_float2(-(tv + hz), -(tv + hw));
+  }
+  s.m1 = x0 + 1 < g.W;
+  s.m2 = x0 + 2 < g.W;
+  s.m3 = x0 + 3 < g.W;
+  return s;
 }
 
 __device__ __forceinline__ int cell_offset(const Geom &g, int y, int x) {
   return (y + 1) * g.RS + x;
 }
 
-// Euler update of one cell (modelsimulator.cpp:224-275).
+// ---- the step ------------------------------------------------------------
+//
+// Work is cut into warp items: a chunk of 32 strips, for every splits-th
+// gene.  A thread evaluates one gene after the other for its 8 cells; the
+// regulators' values are read again, and their lg2 taken again, for every
+// link that reads them.  That is more MUFU work than holding every gene's
+// lg2 in registers (one lg2 per link instead of one per gene), but it needs
+// no register array: no per-gene-count instantiations, no dispatch from a
+// link to a register index (which cost more instructions than the links'
+// arithmetic), a link is a plain loop iteration, and half the registers
+// give twice the warps.  Bound by the MUFU and shared-memory pipes together
+// (each 55-60% busy, issue 60%).  Measured against the register array, same
+// bits (ms): 64 x 64, 4096 models x 2000 steps 203.0 -> 175.2; 100 x 100,
+// 2048 x 500 86.2 -> 77.5; 48 x 48 with 9-16 genes, 600 x 300 18.5 -> 7.5;
+// 256 x 256 with 8 genes, 592 x 100 66.7 -> 57.0; one 32 x 32 model x 500
+// 0.53 -> 0.35.
+
+// Euler update of one cell (modelsimulator.cpp:224-275), the exact path:
 //   r = lim*h - deg*c (+ dif*(s - tot*c) for diffusing genes)
-// exact: the reference's guard on the diffusion term, "a zero rate keeps
-// the value", the minConc clamp and a NaN-ignoring max.
-// fast (minConc 0 and a non-negative finite state, host-checked): the guard
-// only ever skips adding dif*0, a zero rate gives c + dt*0 = c, and the
-// clamp is a max with 0, so these simplify without changing any result.
-template <bool EXACT>
-__device__ __forceinline__ float update_cell(float c, float h, float lim, float deg,
-                                             float dif, bool diffuses, float s, float tot,
-                                             float dt, float min_conc, float &mx) {
-  float r = fmaf(-deg, c, lim * h);
-  if constexpr (EXACT) {
-    if (diffuses && (s > 0.0f || (tot > 0.0f && c > 0.0f))) r = fmaf(dif, fmaf(-tot, c, s), r);
-    float nc = c;
-    if (r != 0.0f) {  // NaN counts as non-zero, like the reference's `if (ratio)`
-      nc = fmaf(dt, r, c);
-      nc = (nc < min_conc) ? 0.0f : nc;
-      const float ar = fabsf(r);
-      mx = (ar > mx) ? ar : mx;  // a NaN rate never raises the max
-    }
-    return nc;
+// with the reference's guard on the diffusion term, "a zero rate keeps the
+// value", the minConc clamp and a NaN-ignoring max.
+__device__ __forceinline__ float update_cell(float c, float h, float lim, float ndeg, float dif,
+                                             bool diffuses, float s, float ntot, float dt,
+                                             float min_conc, float &mx) {
+  float r = fmaf(ndeg, c, lim * h);
+  if (diffuses && (s > 0.0f || (ntot < 0.0f && c > 0.0f))) r = fmaf(dif, fmaf(ntot, c, s), r);
+  float nc = c;
+  if (r != 0.0f) {  // NaN counts as non-zero, like the reference's `if (ratio)`
+    nc = fmaf(dt, r, c);
+    nc = (nc < min_conc) ? 0.0f : nc;
+    const float ar = fabsf(r);
+    mx = (ar > mx) ? ar : mx;  // a NaN rate never raises the max
+  }
+  return nc;
+}
+
+// State accesses of the step: byte offsets from the shared-memory state area
+// (a constant address, so that an offset is all a load needs), or from a
+// global pointer.
+template <int N, bool GL>
+__device__ __forceinline__ const float *state_at(const char *gl, int off) {
+  return chk<N>(reinterpret_cast<const float *>(
+      GL ? gl + off : reinterpret_cast<const char *>(grn_dyn_smem) + kStateOffset + off));
+}
+template <bool GL>
+__device__ __forceinline__ float4 load4(const char *gl, int off) {
+  return *reinterpret_cast<const float4 *>(state_at<4, GL>(gl, off));
+}
+
+// Planes a step reads and writes.  Plane k of the current state is at shared
+// offset sm + k * PSb for k < n_sm, else at gl + k * PSb; its next state at
+// sm_out + k * PSb, or gl_out + k * out_stride.
+struct Planes {
+  int sm, sm_out;
+  const char *gl;
+  char *gl_out;
+  size_t out_stride;
+  int n_sm;
+};
+
+// The terms a*lg2(x) + b of one link for the strip's cells.
+template <int R, bool SPILL>
+__device__ __forceinline__ void link_terms(float4 (&t)[R], const float4 &ab, int slot,
+                                           const Planes &pl, const Strip<R> &st,
+                                           const Geom &g) {
+  float4 x[R];
+  if (SPILL && slot >= pl.n_sm) {
+    const char *q = pl.gl + (size_t)slot * g.PSb;
+#pragma unroll
+    for (int i = 0; i < R; ++i) x[i] = load4<true>(q, st.base + i * g.RSb);
   } else {
-    if (diffuses) r = fmaf(dif, fmaf(-tot, c, s), r);
-    mx = fmaxf(mx, fabsf(r));
-    return fmaxf(fmaf(dt, r, c), 0.0f);
+    const int o = slot * g.PSb + (pl.sm + st.base);
+#pragma unroll
+    for (int i = 0; i < R; ++i) x[i] = load4<false>(nullptr, o + i * g.RSb);
+  }
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const float2 t01 = fma2(lo2(ab), make_float2(lg2_approx(x[i].x), lg2_approx(x[i].y)), hi2(ab));
+    const float2 t23 = fma2(lo2(ab), make_float2(lg2_approx(x[i].z), lg2_approx(x[i].w)), hi2(ab));
+    t[i] = make_float4(t01.x, t01.y, t23.x, t23.y);
   }
 }
 
-// New values of one gene for NI groups; `cur` points at the gene's current
-// plane (shared or global memory).  `mx` takes the max |rate| of the valid
-// groups' real cells.  HPAIR: the fast path adds the horizontal neighbours
-// as FP32 pairs (else as scalar adds; the same roundings).
-template <int NI, int GMAX, bool EXACT, bool RAGGED, bool HPAIR>
-__device__ __forceinline__ void gene_update(const ModelSmem &M, const DenseSmem &D, int p,
-                                            const PackedGene &gn,
-                                            const float4 (&lg)[NI][GMAX], const float *cur,
-                                            const Geom &g, const Item (&it)[NI], float dt,
-                                            float min_conc, float &mx, float4 (&nv)[NI]) {
-  float4 h[NI];
-  if constexpr (EXACT)
-    regulation<NI, GMAX, true>(M, gn, lg, h);
-  else
-    regulation_dense<NI, GMAX>(M, D, p, lg, h);
-  const bool diffuses = gn.dif > 0.0f;  // uniform: the same gene for the whole block
-  if constexpr (!EXACT) {
-    // Fast path (update_cell<false>) on cell pairs: the same roundings,
-    // two cells per FP32 instruction.
+template <int MODE, int R>
+__device__ __forceinline__ void comb_strip(float4 (&v)[R], const float4 (&t)[R]) {
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      const float4 c = *reinterpret_cast<const float4 *>(chk<4>(cur + it[i].base));
-      float2 r01 = fma2(f2(-gn.deg), lo2(c), mul2(f2(gn.lim), lo2(h[i])));
-      float2 r23 = fma2(f2(-gn.deg), hi2(c), mul2(f2(gn.lim), hi2(h[i])));
-      if (diffuses) {
-        const float4 up = *reinterpret_cast<const float4 *>(chk<4>(cur + it[i].base - g.RS));
-        const float4 dn = *reinterpret_cast<const float4 *>(chk<4>(cur + it[i].base + g.RS));
-        // Row borders read the zero cells that end every padded row.
-        const float lft = *chk<1>(cur + it[i].base - 1);
-        const float rgt = *chk<1>(cur + it[i].base + 4);
-        // Reference order: x-1, x+1, y-1, y+1.  Scalar adds suit the step
-        // with two groups per thread and the streaming step (the pairs'
-        // operands straddle the float4's register pairs); paired adds the
-        // steps with one group per thread (measured on the walking step).
-        float2 s01, s23;
-        if constexpr (!HPAIR) {
-          s01 = add2(add2(make_float2(lft + c.y, c.x + c.z), lo2(up)), lo2(dn));
-          s23 = add2(add2(make_float2(c.y + c.w, c.z + rgt), hi2(up)), hi2(dn));
-        } else {
-          s01 = add2(add2(add2(make_float2(lft, c.x), make_float2(c.y, c.z)), lo2(up)), lo2(dn));
-          s23 = add2(add2(add2(make_float2(c.y, c.z), make_float2(c.w, rgt)), hi2(up)), hi2(dn));
-        }
-        r01 = fma2(f2(gn.dif), fma2(make_float2(-it[i].tot.x, -it[i].tot.y), lo2(c), s01), r01);
-        r23 = fma2(f2(gn.dif), fma2(make_float2(-it[i].tot.z, -it[i].tot.w), hi2(c), s23), r23);
-      }
-      const float2 n01 = fma2(f2(dt), r01, lo2(c));
-      const float2 n23 = fma2(f2(dt), r23, hi2(c));
-      nv[i] = make_float4(fmaxf(n01.x, 0.0f), fmaxf(n01.y, 0.0f), fmaxf(n23.x, 0.0f),
-                          fmaxf(n23.y, 0.0f));
-      float m = fabsf(r01.x);
-      float m1 = fabsf(r01.y), m2 = fabsf(r23.x), m3 = fabsf(r23.y);
-      if constexpr (RAGGED) {
-        // Cells past W are padding: kept at 0, never part of the max.
-        if (!it[i].v1) { nv[i].y = 0.0f; m1 = 0.0f; }
-        if (!it[i].v2) { nv[i].z = 0.0f; m2 = 0.0f; }
-        if (!it[i].v3) { nv[i].w = 0.0f; m3 = 0.0f; }
-      }
-      if (it[i].valid) mx = fmaxf(fmaxf(mx, m), fmaxf(fmaxf(m1, m2), m3));
-    }
+  for (int i = 0; i < R; ++i) {
+    v[i].x = comb<MODE>(v[i].x, t[i].x);
+    v[i].y = comb<MODE>(v[i].y, t[i].y);
+    v[i].z = comb<MODE>(v[i].z, t[i].z);
+    v[i].w = comb<MODE>(v[i].w, t[i].w);
+  }
+}
+
+// Regulation 1 / (1 + 2^v) of four cells.
+__device__ __forceinline__ float4 hill4(const float4 &v) {
+  const float2 e01 = add2(f2(1.0f), make_float2(ex2_approx(v.x), ex2_approx(v.y)));
+  const float2 e23 = add2(f2(1.0f), make_float2(ex2_approx(v.z), ex2_approx(v.w)));
+  return make_float4(rcp_approx(e01.x), rcp_approx(e01.y), rcp_approx(e23.x), rcp_approx(e23.y));
+}
+
+// Regulation of one gene (its ctl word) for the strip: the first link's
+// terms start the running exponents, OR links take the min, AND links the
+// max.  exact: the reference's comparison order, where a Hill coefficient
+// of 0 (kConstSlot) gives the constant term 0; in the fast path models have
+// no such link.
+template <int R, bool EXACT, bool SPILL>
+__device__ __forceinline__ void regulation(const ProgSmem &P, int ctl, const Planes &pl,
+                                           const Strip<R> &st, const Geom &g, float4 (&h)[R]) {
+  const int n = ctl >> 21;
+  if (n == 0) {  // OpZero
+#pragma unroll
+    for (int i = 0; i < R; ++i) h[i] = f4(0.0f);
     return;
   }
+  const LinkSmem *L = P.link + ((ctl >> 5) & 255);
+  const int n_or = (ctl >> 13) & 255;
+  float4 v[R], t[R];
+  if constexpr (EXACT) {
 #pragma unroll
-  for (int i = 0; i < NI; ++i) {
-    const float4 c = *reinterpret_cast<const float4 *>(chk<4>(cur + it[i].base));
-    float4 s = f4(0.0f);
-    if (diffuses) {
-      const float4 up = *reinterpret_cast<const float4 *>(chk<4>(cur + it[i].base - g.RS));
-      const float4 dn = *reinterpret_cast<const float4 *>(chk<4>(cur + it[i].base + g.RS));
-      const float lft = *chk<1>(cur + it[i].base - 1);  // zero cells at the row borders
-      const float rgt = *chk<1>(cur + it[i].base + 4);
-      // Reference order: x-1, x+1, y-1, y+1.
-      s.x = ((lft + c.y) + up.x) + dn.x;
-      s.y = ((c.x + c.z) + up.y) + dn.y;
-      s.z = ((c.y + c.w) + up.z) + dn.z;
-      s.w = ((c.z + rgt) + up.w) + dn.w;
+    for (int i = 0; i < R; ++i) v[i] = f4(__int_as_float(0x7fc00000));
+#pragma unroll 1
+    for (int l = 0; l < n; ++l) {
+      const int slot = L[l].slot;
+      if (slot == kConstSlot) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) t[i] = f4(0.0f);
+      } else {
+        link_terms<R, SPILL>(t, L[l].ab, slot, pl, st, g);
+      }
+      if (l < n_or) comb_strip<kOrExact, R>(v, t);
+      else comb_strip<kAndExact, R>(v, t);
     }
-    float m = 0.0f, m1 = 0.0f, m2 = 0.0f, m3 = 0.0f;
-    nv[i].x = update_cell<EXACT>(c.x, h[i].x, gn.lim, gn.deg, gn.dif, diffuses, s.x,
-                                 it[i].tot.x, dt, min_conc, m);
-    nv[i].y = update_cell<EXACT>(c.y, h[i].y, gn.lim, gn.deg, gn.dif, diffuses, s.y,
-                                 it[i].tot.y, dt, min_conc, RAGGED ? m1 : m);
-    nv[i].z = update_cell<EXACT>(c.z, h[i].z, gn.lim, gn.deg, gn.dif, diffuses, s.z,
-                                 it[i].tot.z, dt, min_conc, RAGGED ? m2 : m);
-    nv[i].w = update_cell<EXACT>(c.w, h[i].w, gn.lim, gn.deg, gn.dif, diffuses, s.w,
-                                 it[i].tot.w, dt, min_conc, RAGGED ? m3 : m);
+  } else {
+    link_terms<R, SPILL>(v, L->ab, L->slot, pl, st, g);
+    ++L;
+    int slot = L->slot;  // read one link ahead
+    int left = n_or - 1;
+#pragma unroll 1
+    for (; left > 0; --left) {
+      const float4 ab = L->ab;
+      const int s = slot;
+      ++L;
+      slot = L->slot;
+      link_terms<R, SPILL>(t, ab, s, pl, st, g);
+      comb_strip<kOrFast, R>(v, t);
+    }
+    left = n - max(n_or, 1);
+#pragma unroll 1
+    for (; left > 0; --left) {
+      const float4 ab = L->ab;
+      const int s = slot;
+      ++L;
+      slot = L->slot;
+      link_terms<R, SPILL>(t, ab, s, pl, st, g);
+      comb_strip<kAndFast, R>(v, t);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < R; ++i) h[i] = hill4(v[i]);
+}
+
+// New values of one gene for the strip, from its current plane (at src_gl,
+// or shared offset src) to its next one (dst_gl, dst).  `mx` takes the
+// max |rate| of the strip's real cells.
+// Fast path (minConc 0 and a non-negative finite state, host-checked): the
+// reference's diffusion guard only ever skips adding dif*0, a zero rate
+// gives c + dt*0 = c, and the clamp is a max with 0, so these simplify
+// without changing any result.
+template <int R, bool EXACT, bool RAGGED, bool DIFFUSES, bool SG, bool DG>
+__device__ __forceinline__ void update_strip(const GeneSmem &gn, const float4 (&h)[R],
+                                             const char *src_gl, int src, char *dst_gl, int dst,
+                                             const Strip<R> &st, const Geom &g, float dt,
+                                             float min_conc, float &mx) {
+  const float4 ld = gn.ld;
+  const float2 dif = DIFFUSES ? gn.dif : f2(0.0f);
+  const int o = src + st.base;
+  // Rows -1 .. R of the strip's group (row i at c[i + 1]).
+  float4 c[R + 2];
+  float lft[R], rgt[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) c[i + 1] = load4<SG>(src_gl, o + i * g.RSb);
+  if constexpr (DIFFUSES) {
+    c[0] = load4<SG>(src_gl, o - g.RSb);
+    c[R + 1] = load4<SG>(src_gl, o + R * g.RSb);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const float l = __shfl_up_sync(kFull, c[i + 1].w, 1);
+      const float r = __shfl_down_sync(kFull, c[i + 1].x, 1);
+      lft[i] = st.el ? 0.0f : l;
+      rgt[i] = st.er ? 0.0f : r;
+    }
+    if (g.edges) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        if (st.el) lft[i] = *state_at<1, SG>(src_gl, o + i * g.RSb - 4);
+        if (st.er) rgt[i] = *state_at<1, SG>(src_gl, o + i * g.RSb + 16);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const float4 ci = c[i + 1];
+    float2 s01 = f2(0.0f), s23 = f2(0.0f);
+    if constexpr (DIFFUSES) {
+      // Reference order: x-1, x+1, y-1, y+1.
+      s01 = make_float2(lft[i] + ci.y, ci.x + ci.z);
+      s23 = make_float2(ci.y + ci.w, ci.z + rgt[i]);
+      s01 = add2(add2(s01, lo2(c[i])), lo2(c[i + 2]));
+      s23 = add2(add2(s23, hi2(c[i])), hi2(c[i + 2]));
+    }
+    float4 nv;
+    float m, m1, m2, m3;
+    if constexpr (!EXACT) {
+      float2 r01 = fma2(hi2(ld), lo2(ci), mul2(lo2(ld), lo2(h[i])));
+      float2 r23 = fma2(hi2(ld), hi2(ci), mul2(lo2(ld), hi2(h[i])));
+      if constexpr (DIFFUSES) {
+        r01 = fma2(dif, fma2(st.nt[i][0], lo2(ci), s01), r01);
+        r23 = fma2(dif, fma2(st.nt[i][1], hi2(ci), s23), r23);
+      }
+      const float2 n01 = fma2(f2(dt), r01, lo2(ci));
+      const float2 n23 = fma2(f2(dt), r23, hi2(ci));
+      nv = make_float4(fmaxf(n01.x, 0.0f), fmaxf(n01.y, 0.0f), fmaxf(n23.x, 0.0f),
+                       fmaxf(n23.y, 0.0f));
+      m = fabsf(r01.x);
+      m1 = fabsf(r01.y);
+      m2 = fabsf(r23.x);
+      m3 = fabsf(r23.y);
+    } else {
+      m = m1 = m2 = m3 = 0.0f;
+      nv.x = update_cell(ci.x, h[i].x, ld.x, ld.z, dif.x, DIFFUSES, s01.x, st.nt[i][0].x, dt,
+                         min_conc, m);
+      nv.y = update_cell(ci.y, h[i].y, ld.x, ld.z, dif.x, DIFFUSES, s01.y, st.nt[i][0].y, dt,
+                         min_conc, m1);
+      nv.z = update_cell(ci.z, h[i].z, ld.x, ld.z, dif.x, DIFFUSES, s23.x, st.nt[i][1].x, dt,
+                         min_conc, m2);
+      nv.w = update_cell(ci.w, h[i].w, ld.x, ld.z, dif.x, DIFFUSES, s23.y, st.nt[i][1].y, dt,
+                         min_conc, m3);
+    }
     if constexpr (RAGGED) {
       // Cells past W are padding: kept at 0, never part of the max.
-      if (!it[i].v1) { nv[i].y = 0.0f; m1 = 0.0f; }
-      if (!it[i].v2) { nv[i].z = 0.0f; m2 = 0.0f; }
-      if (!it[i].v3) { nv[i].w = 0.0f; m3 = 0.0f; }
-      m = fmaxf(fmaxf(m, m1), fmaxf(m2, m3));
+      if (!st.m1) { nv.y = 0.0f; m1 = 0.0f; }
+      if (!st.m2) { nv.z = 0.0f; m2 = 0.0f; }
+      if (!st.m3) { nv.w = 0.0f; m3 = 0.0f; }
     }
-    if (it[i].valid) mx = fmaxf(mx, m);
+    if (st.valid && (i == 0 || i < st.rows)) {
+      mx = fmaxf(fmaxf(mx, m), fmaxf(fmaxf(m1, m2), m3));
+        *reinterpret_cast<float4 *>(const_cast<float *>(
+            state_at<4, DG>(dst_gl, dst + st.base + i * g.RSb))) = nv;
+    }
   }
+}
+
+// One gene (entry k of the program) for the strip.  SPILL: genes n_sm and on
+// live in the global slot.  BAND: the source planes are a staged band in
+// shared memory, the destination is global.
+template <int R, bool EXACT, bool RAGGED, bool SPILL, bool BAND>
+__device__ __forceinline__ void gene_step(const ProgSmem &P, int k, const Planes &pl,
+                                          const Strip<R> &st, const Geom &g, float dt,
+                                          float min_conc, float &mx) {
+  const GeneSmem &gn = P.gene[k];
+  const int ctl = uniform(gn.ctl);
+  const int p = ctl & 15;
+  float4 h[R];
+  regulation<R, EXACT, SPILL>(P, ctl, pl, st, g, h);
+  const auto update = [&](auto diffuses) {
+    constexpr bool D = decltype(diffuses)::value;
+    char *const out = pl.gl_out + p * pl.out_stride;
+    if (SPILL && p >= pl.n_sm)
+      update_strip<R, EXACT, RAGGED, D, true, true>(gn, h, pl.gl + (size_t)p * g.PSb, 0, out, 0,
+                                                    st, g, dt, min_conc, mx);
+    else
+      update_strip<R, EXACT, RAGGED, D, false, BAND>(gn, h, nullptr, pl.sm + p * g.PSb, out,
+                                                     BAND ? 0 : pl.sm_out + p * g.PSb, st, g, dt,
+                                                     min_conc, mx);
+  };
+  if (ctl & 16) update(True{});
+  else update(False{});
 }
 
 // Block-wide max of a non-negative, non-NaN float (bit order == value
-// order).  `parity` alternates two buffers so that one barrier per step
-// suffices.
-template <int NT>
-__device__ __forceinline__ float block_max(float v, float *red, int parity, int lane,
-                                           int warp) {
+// order): each warp publishes its max, a barrier follows, and any thread
+// can read the block's.  `parity` alternates two buffers so that one barrier
+// per step suffices.
+__device__ __forceinline__ void publish_max(float v, float *red, int parity, int lane, int warp) {
   const unsigned bits = __reduce_max_sync(kFull, __float_as_uint(v));
-  float *r = red + parity * 32;
-  if (lane == 0) r[warp] = __uint_as_float(bits);
-  __syncthreads();
+  if (lane == 0) red[parity * 32 + warp] = __uint_as_float(bits);
+}
+__device__ __forceinline__ float published_max(const float *red, int parity, int lane,
+                                               int n_warps) {
   // One warp value per lane, then a warp max (redux) in every warp.
-  const unsigned mine = lane < NT / 32 ? __float_as_uint(r[lane]) : 0u;
+  const unsigned mine = lane < n_warps ? __float_as_uint(red[parity * 32 + lane]) : 0u;
   return __uint_as_float(__reduce_max_sync(kFull, mine));
 }
+__device__ __forceinline__ float block_max(float v, float *red, int parity, int lane, int warp,
+                                           int n_warps) {
+  publish_max(v, red, parity, lane, warp);
+  __syncthreads();
+  return published_max(red, parity, lane, n_warps);
+}
 
-// Block-wide FP64 sum; every thread gets the same value (fixed order).
-template <int NT>
-__device__ __forceinline__ double block_sum(double v, double *dred, int lane, int warp) {
+// The experiment's fitness sum over the block's cells (simstate.cpp:135-158)
+// in FP64.  Cell i belongs to lane i % 32 of virtual warp (i / 32) %
+// kSumWarps, whatever the block size, and the virtual warps' sums are added
+// in order, so every schedule and block size gives the same bits.  Every
+// thread gets the sum.
+constexpr int kSumWarps = 16;
+
+template <typename F>
+__device__ __forceinline__ double cell_sum(int cells, F term, double *dred, int lane, int warp,
+                                           int n_warps) {
+  for (int vw = warp; vw < kSumWarps; vw += n_warps) {
+    double v = 0.0;
+    for (int i = vw * 32 + lane; i < cells; i += kSumWarps * 32) v = term(i, v);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFull, v, o);
-  if (lane == 0) dred[warp] = v;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFull, v, o);
+    if (lane == 0) dred[vw] = v;
+  }
   __syncthreads();
   double s = 0.0;
 #pragma unroll
-  for (int w = 0; w < NT / 32; ++w) s += dred[w];
+  for (int w = 0; w < kSumWarps; ++w) s += dred[w];
   return s;
 }
 
 // Where a model's state lives during one step: genes p < n_sm are double
 // buffered in shared-memory planes p and p + n_sm; the others in the
-// block's global slot, planes p and p + GMAX.  `par` selects the buffer
+// block's global slot, planes p and p + gmax.  `par` selects the buffer
 // holding the current values.
 struct StatePtrs {
   float *sm;   // shared-memory planes
   float *gl;   // global-memory slot
   int n_sm;    // genes held in shared memory
+  int gmax;    // genes a global slot holds
 };
 
-template <int GMAX>
 __device__ __forceinline__ float *plane_of(const StatePtrs &sp, const Geom &g, int p, int par) {
   return p < sp.n_sm ? sp.sm + (p + (par ? sp.n_sm : 0)) * g.PS
-                     : sp.gl + (p + (par ? GMAX : 0)) * g.PS;
+                     : sp.gl + (p + (par ? sp.gmax : 0)) * g.PS;
 }
 
-// New values of all genes of NI groups: shared-memory genes first, then
-// global-memory genes (two loops so that each uses its own load path).
-// GMAX is the launch's gene capacity (the global slot layout); GS >= the
-// model's gene count bounds the regulator slots the step evaluates (the
-// unrolled slot loops cost GS steps per gene whatever the links).
-template <int NI, int GMAX, int GS, bool EXACT, bool RAGGED>
-__device__ __forceinline__ void group_step(const ModelSmem &M, const DenseSmem &D,
-                                           const StatePtrs &sp,
-                                           const Geom &g, const Item (&it)[NI], int par,
-                                           float dt, float min_conc, float &mx) {
-  const int G = M.hdr.n_genes;
-  const uint32_t lg_mask = M.hdr.lg_mask;
-  const float *sm_cur = sp.sm + (par ? sp.n_sm : 0) * g.PS;
-  float *sm_nxt = sp.sm + (par ? 0 : sp.n_sm) * g.PS;
-  const float *gl_cur = sp.gl + (par ? GMAX : 0) * g.PS;
-  float *gl_nxt = sp.gl + (par ? 0 : GMAX) * g.PS;
-  // lg2 of the genes' current values.  The fast path takes it for every
-  // gene of the model (a uniform bound, no per-slot test; its dense slot
-  // masks read only the regulators) and zeroes the slots past the model's
-  // genes; the exact path takes it for the regulators only (lg_mask) and
-  // keeps the other slots 0 for its slot switch.
-  float4 lg[NI][GS];
-#pragma unroll
-  for (int k = 0; k < GS; ++k) {
-    if (EXACT || k >= G) {
-#pragma unroll
-      for (int i = 0; i < NI; ++i) lg[i][k] = f4(0.0f);
-    }
-    if (k < G && (!EXACT || ((lg_mask >> k) & 1u))) {
-      const float *pl = (k < sp.n_sm ? sm_cur : gl_cur) + k * g.PS;
-#pragma unroll
-      for (int i = 0; i < NI; ++i) {
-        const float4 c = *reinterpret_cast<const float4 *>(chk<4>(pl + it[i].base));
-        lg[i][k].x = lg2_approx(c.x);
-        lg[i][k].y = lg2_approx(c.y);
-        lg[i][k].z = lg2_approx(c.z);
-        lg[i][k].w = lg2_approx(c.w);
-      }
-    }
-  }
-  for (int p = 0; p < sp.n_sm; ++p) {
-    const PackedGene gn = M.genes[p];
-    float4 nv[NI];
-    gene_update<NI, GS, EXACT, RAGGED, (NI == 1)>(M, D, p, gn, lg, sm_cur + p * g.PS, g, it, dt,
-                                                  min_conc, mx, nv);
-#pragma unroll
-    for (int i = 0; i < NI; ++i)
-      if (it[i].valid) *reinterpret_cast<float4 *>(chk<4>(sm_nxt + p * g.PS + it[i].base)) = nv[i];
-  }
-  for (int p = sp.n_sm; p < G; ++p) {
-    const PackedGene gn = M.genes[p];
-    float4 nv[NI];
-    gene_update<NI, GS, EXACT, RAGGED, (NI == 1)>(M, D, p, gn, lg, gl_cur + p * g.PS, g, it, dt,
-                                                  min_conc, mx, nv);
-#pragma unroll
-    for (int i = 0; i < NI; ++i)
-      if (it[i].valid) *reinterpret_cast<float4 *>(chk<4>(gl_nxt + p * g.PS + it[i].base)) = nv[i];
-  }
+// Genes first, first + splits, .. of the program for one strip.
+template <int R, bool EXACT, bool RAGGED, bool SPILL>
+__device__ __forceinline__ void strip_step(const ProgSmem &P, const StatePtrs &sp, int G,
+                                           const Geom &g, const Strip<R> &st, int first,
+                                           int splits, int par, float dt, float min_conc,
+                                           float &mx) {
+  const int half = sp.n_sm * g.PSb;
+  const size_t gl_half = (size_t)sp.gmax * g.PSb;
+  char *gl = reinterpret_cast<char *>(sp.gl);
+  const Planes pl{opaque(par ? half : 0), opaque(par ? 0 : half), gl + (par ? gl_half : 0),
+                  gl + (par ? 0 : gl_half), (size_t)g.PSb,  sp.n_sm};
+#pragma unroll 1
+  for (int k = first; k < G; k += splits)
+    gene_step<R, EXACT, RAGGED, SPILL, false>(P, k, pl, st, g, dt, min_conc, mx);
 }
 
-// The fast path of one step, with the slot bound fitted to the model's gene
-// count (a uniform branch per model).
-template <int NI, int GMAX, bool RAGGED>
-__device__ __forceinline__ void group_step_fast(const ModelSmem &M, const DenseSmem &D,
-                                                const StatePtrs &sp, const Geom &g,
-                                                const Item (&it)[NI], int par, float dt,
-                                                float min_conc, float &mx) {
-  const int G = M.hdr.n_genes;
-  if (GMAX > 2 && G <= 2)
-    group_step<NI, GMAX, (GMAX < 2 ? GMAX : 2), false, RAGGED>(M, D, sp, g, it, par, dt,
-                                                               min_conc, mx);
-  else if (GMAX > 4 && G <= 4)
-    group_step<NI, GMAX, (GMAX < 4 ? GMAX : 4), false, RAGGED>(M, D, sp, g, it, par, dt,
-                                                               min_conc, mx);
-  else if (GMAX > 6 && G <= 6)
-    group_step<NI, GMAX, (GMAX < 6 ? GMAX : 6), false, RAGGED>(M, D, sp, g, it, par, dt,
-                                                               min_conc, mx);
+// The same by the model's class: all planes in shared memory or some in the
+// global slot; the exact path always takes the general form.
+template <int R, bool RAGGED>
+__device__ __forceinline__ void strip_step_any(bool exact, const ProgSmem &P, const StatePtrs &sp,
+                                               int G, const Geom &g, const Strip<R> &st, int first,
+                                               int splits, int par, float dt, float min_conc,
+                                               float &mx) {
+  if (exact)
+    strip_step<R, true, RAGGED, true>(P, sp, G, g, st, first, splits, par, dt, min_conc, mx);
+  else if (sp.n_sm < G)
+    strip_step<R, false, RAGGED, true>(P, sp, G, g, st, first, splits, par, dt, min_conc, mx);
   else
-    group_step<NI, GMAX, GMAX, false, RAGGED>(M, D, sp, g, it, par, dt, min_conc, mx);
+    strip_step<R, false, RAGGED, false>(P, sp, G, g, st, first, splits, par, dt, min_conc, mx);
+}
+
+// Warps that share a chunk's genes when `chunks` chunks are walked by
+// n_warps warps: the power of two (at most 4) with the shortest longest
+// warp, counted in gene evaluations (an item costs about a quarter of one).
+__device__ __forceinline__ int choose_splits(int chunks, int n_warps, int G) {
+  int best = 1, cost = 0x7fffffff;
+  for (int s = 1; s <= 4; s *= 2) {
+    if (s > G) break;
+    const int rounds = (chunks * s + n_warps - 1) / n_warps;
+    const int c = rounds * (4 * ((G + s - 1) / s) + 1);
+    if (c < cost) {
+      cost = c;
+      best = s;
+    }
+  }
+  return best;
 }
 
 // ---- streaming schedule -------------------------------------------------
@@ -790,69 +840,40 @@ __device__ __forceinline__ void group_step_fast(const ModelSmem &M, const DenseS
 // shared-memory stage by bulk copies (the TMA engine's cp.async.bulk, one
 // per gene, completing on the stage's mbarrier) while the previous band is
 // computed from the other stage; new values go straight to the global slot.
-// The step's arithmetic is the other schedules' (gene_update), so states
-// are bit-identical.
+// The step's arithmetic is the other schedules' (regulation and
+// update_strip), so states are bit-identical.
 
-// New values of all genes of NI groups of one band (stage planes of
-// gb.PS floats), written to the global next-state planes.
-// `out` addresses the band's cells as a plane does: cell (x, local row y)
-// of gene p at out + p * gps + (y + 1) * RS + x.
-template <int NI, int GS, bool EXACT, bool RAGGED>
-__device__ __forceinline__ void band_group_step(const ModelSmem &M, const DenseSmem &D,
-                                                const float *stage, int G, const Geom &gb,
-                                                const Item (&it)[NI], float *out, size_t gps,
-                                                float dt, float min_conc, float &mx) {
-  const uint32_t lg_mask = M.hdr.lg_mask;
-  float4 lg[NI][GS];
-#pragma unroll
-  for (int k = 0; k < GS; ++k) {
-    if (EXACT || k >= G) {
-#pragma unroll
-      for (int i = 0; i < NI; ++i) lg[i][k] = f4(0.0f);
-    }
-    if (k < G && (!EXACT || ((lg_mask >> k) & 1u))) {
-      const float *pl = stage + k * gb.PS;
-#pragma unroll
-      for (int i = 0; i < NI; ++i) {
-        const float4 c = *reinterpret_cast<const float4 *>(chk<4>(pl + it[i].base));
-        lg[i][k].x = lg2_approx(c.x);
-        lg[i][k].y = lg2_approx(c.y);
-        lg[i][k].z = lg2_approx(c.z);
-        lg[i][k].w = lg2_approx(c.w);
-      }
-    }
-  }
-  for (int p = 0; p < G; ++p) {
-    float4 nv[NI];
-    gene_update<NI, GS, EXACT, RAGGED, false>(M, D, p, M.genes[p], lg, stage + p * gb.PS, gb, it,
-                                              dt, min_conc, mx, nv);
-#pragma unroll
-    for (int i = 0; i < NI; ++i)
-      if (it[i].valid) *reinterpret_cast<float4 *>(chk<4>(out + p * gps + it[i].base)) = nv[i];
+// New values of all genes of one band from its stage planes (of gb.PS
+// floats), written to the global next-state planes: the warps walk the
+// band's items.  `out` addresses the band's cells as a plane does: cell (x,
+// local row y) of gene p at out + p * gps + (y + 1) * RS + x.
+template <int R, bool EXACT, bool RAGGED>
+__device__ __forceinline__ void band_step(const ProgSmem &P, const float *stage, int G,
+                                          const Geom &gb, float *out, size_t gps, int splits,
+                                          float dt, float min_conc, float &mx) {
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+  const int items = ((gb.Q + 31) / 32) * splits;
+  const int shift = 31 - __clz(splits);
+  const Planes pl{(int)(reinterpret_cast<const unsigned char *>(stage) - grn_dyn_smem) -
+                      (int)kStateOffset,
+                  0, nullptr, reinterpret_cast<char *>(out), gps * sizeof(float), G};
+#pragma unroll 1
+  for (int i = warp; i < items; i += n_warps) {
+    const Strip<R> st = strip_at<R>((i >> shift) * 32 + lane, gb);
+#pragma unroll 1
+    for (int k = i & (splits - 1); k < G; k += splits)
+      gene_step<R, EXACT, RAGGED, false, true>(P, k, pl, st, gb, dt, min_conc, mx);
   }
 }
 
-template <int NI, int GMAX, bool RAGGED>
-__device__ __forceinline__ void band_group_step_any(bool exact, const ModelSmem &M,
-                                                    const DenseSmem &D, const float *stage, int G,
-                                                    const Geom &gb, const Item (&it)[NI],
-                                                    float *out, size_t gps, float dt,
-                                                    float min_conc, float &mx) {
+template <int R, bool RAGGED>
+__device__ __forceinline__ void band_step_any(bool exact, const ProgSmem &P, const float *stage,
+                                              int G, const Geom &gb, float *out, size_t gps,
+                                              int splits, float dt, float min_conc, float &mx) {
   if (exact)
-    band_group_step<NI, GMAX, true, RAGGED>(M, D, stage, G, gb, it, out, gps, dt, min_conc,
-                                            mx);
-  else if (GMAX > 2 && G <= 2)
-    band_group_step<NI, (GMAX < 2 ? GMAX : 2), false, RAGGED>(M, D, stage, G, gb, it, out,
-                                                              gps, dt, min_conc, mx);
-  else if (GMAX > 4 && G <= 4)
-    band_group_step<NI, (GMAX < 4 ? GMAX : 4), false, RAGGED>(M, D, stage, G, gb, it, out,
-                                                              gps, dt, min_conc, mx);
-  else if (GMAX > 6 && G <= 6)
-    band_group_step<NI, (GMAX < 6 ? GMAX : 6), false, RAGGED>(M, D, stage, G, gb, it, out,
-                                                              gps, dt, min_conc, mx);
+    band_step<R, true, RAGGED>(P, stage, G, gb, out, gps, splits, dt, min_conc, mx);
   else
-    band_group_step<NI, GMAX, false, RAGGED>(M, D, stage, G, gb, it, out, gps, dt, min_conc,
-                                             mx);
+    band_step<R, false, RAGGED>(P, stage, G, gb, out, gps, splits, dt, min_conc, mx);
 }
 
 // One Euler step of the streaming schedule.  Stages alternate by band; the
@@ -864,19 +885,19 @@ __device__ __forceinline__ void band_group_step_any(bool exact, const ModelSmem 
 // whatever the stage holds; the band's one barrier then makes the decision
 // block-wide (the model's results are discarded on that path).  *fail is 0
 // on entry and is never cleared: the kernel returns after a failure.
-template <int NT, int GMAX, bool RAGGED>
-__device__ bool stream_step(const SimArgs &A, const ModelSmem &M, const DenseSmem &D,
-                            const StatePtrs &sp, const Geom &g, int G, int par, bool exact,
+template <bool RAGGED>
+__device__ bool stream_step(const SimArgs &A, const ProgSmem &P, const StatePtrs &sp,
+                            const Geom &g, int G, int splits, int par, bool exact,
                             float dt, float min_conc, float &mx, uint64_t *bars,
                             uint32_t &mphase, volatile int *fail, int R) {
   const int nb = (g.H + R - 1) / R;
   const int SPS = (R + 2) * g.RS;
   float *stage0 = sp.sm;
   const size_t gps = (size_t)g.PS;
-  const float *gl_cur = sp.gl + (par ? GMAX : 0) * gps;
-  float *gl_nxt = sp.gl + (par ? 0 : GMAX) * gps;
+  const float *gl_cur = sp.gl + (par ? sp.gmax : 0) * gps;
+  float *gl_nxt = sp.gl + (par ? 0 : sp.gmax) * gps;
   auto issue = [&](int b) {
-    float *st = stage0 + (b & 1) * GMAX * SPS;
+    float *st = stage0 + (b & 1) * sp.gmax * SPS;
     const int rows = min(R + 2, g.H + 2 - b * R);  // plane rows b*R .. b*R + rows - 1
     const uint32_t bytes = (uint32_t)rows * g.RS * 4u;
     fence_proxy_async_shared();
@@ -902,15 +923,10 @@ __device__ bool stream_step(const SimArgs &A, const ModelSmem &M, const DenseSme
     gb.y0 = b * R;
     gb.H = min(R, g.H - b * R);
     gb.PS = SPS;
-    gb.Q = gb.H * g.Wg;
-    const float *st = stage0 + s * GMAX * SPS;
-    const int n_it = (gb.Q + NT - 1) / NT;
-    for (int i = 0; i < n_it; ++i) {  // the same count in every thread (barriers follow)
-      const Item it[1] = {item_at(threadIdx.x + i * NT, gb)};
-      band_group_step_any<1, GMAX, RAGGED>(exact, M, D, st, G, gb, it,
-                                            gl_nxt + (size_t)gb.y0 * g.RS, gps, dt, min_conc,
-                                            mx);
-    }
+    gb.PSb = 4 * SPS;
+    gb.Q = strip_count<kStripRows>(gb.H, g.Wg);
+    band_step_any<kStripRows, RAGGED>(exact, P, stage0 + s * sp.gmax * SPS, G, gb,
+                          gl_nxt + (size_t)gb.y0 * g.RS, gps, splits, dt, min_conc, mx);
     __syncthreads();  // stage s is free again; *fail is the same for every thread
     if (*fail) {
       // Bounded second waits for copies that may still be in flight: the
@@ -938,19 +954,19 @@ __device__ bool stream_step(const SimArgs &A, const ModelSmem &M, const DenseSme
 // computes the band from the intermediate and writes it to the global
 // next-state planes.  The copy of band b + 1 is issued once step one of band
 // b has read the stage, so it overlaps step two.  Both steps run
-// band_group_step, the one-step schedules' arithmetic, so states are
+// band_step, the one-step schedules' arithmetic, so states are
 // bit-identical to them.  Shared memory: G * (R + 4) stage rows and
 // G * (R + 2) intermediate rows (R = A.band_rows); the same space holds the
-// one-step schedule's two stages of R + 1 + 2 rows, which the kernel uses
+// one-step schedule's two stages of R + 2 rows, which the kernel uses
 // for a single step (an odd last step, or a first step after which the
 // simulation stops).
 //
 // mx1 / mx2 receive the threads' max |rate| of the first / second step.
 // Returns false (the same in every thread) if a copy did not complete in
 // time, after a bounded wait for the copy still in flight.
-template <int NT, int GMAX, bool RAGGED>
-__device__ bool stream_step2(const SimArgs &A, const ModelSmem &M, const DenseSmem &D,
-                             const StatePtrs &sp, const Geom &g, int G, int par, bool exact,
+template <bool RAGGED>
+__device__ bool stream_step2(const SimArgs &A, const ProgSmem &P, const StatePtrs &sp,
+                             const Geom &g, int G, int splits, int par, bool exact,
                              float dt, float min_conc, float &mx1, float &mx2, uint64_t *bars,
                              uint32_t &mphase, volatile int *fail) {
   const int R = A.band_rows;
@@ -958,10 +974,10 @@ __device__ bool stream_step2(const SimArgs &A, const ModelSmem &M, const DenseSm
   const int SPS = (R + 4) * g.RS;   // stage plane stride: plane rows bR-1 .. bR+R+2
   const int IPS = (R + 2) * g.RS;   // intermediate plane stride: grid rows bR-1 .. bR+R
   float *stage = sp.sm;
-  float *inter = sp.sm + (size_t)GMAX * SPS;
+  float *inter = sp.sm + (size_t)sp.gmax * SPS;
   const size_t gps = (size_t)g.PS;
-  const float *gl_cur = sp.gl + (par ? GMAX : 0) * gps;
-  float *gl_nxt = sp.gl + (par ? 0 : GMAX) * gps;
+  const float *gl_cur = sp.gl + (par ? sp.gmax : 0) * gps;
+  float *gl_nxt = sp.gl + (par ? 0 : sp.gmax) * gps;
   auto issue = [&](int b) {
     const int p0 = max(b * R - 1, 0);               // first plane row copied
     const int p1 = min(b * R + R + 3, g.H + 2);     // one past the last
@@ -987,20 +1003,16 @@ __device__ bool stream_step2(const SimArgs &A, const ModelSmem &M, const DenseSm
     g1.y0 = y1;
     g1.H = h1;
     g1.PS = SPS;
-    g1.Q = h1 * g.Wg;
+    g1.PSb = 4 * SPS;
+    g1.Q = strip_count<kStripRows>(h1, g.Wg);
     // Stage row of grid row y is y - bR + 2; g1's row 0 is grid row y1 - 1.
     const float *st1 = stage + (y1 - b * R + 1) * g.RS;
     float *out1 = inter + (y1 - b * R) * g.RS;  // cell rows land at y - (bR - 1)
-    const int n1 = (g1.Q + NT - 1) / NT;
-    for (int i = 0; i < n1; ++i) {
-      const Item it[1] = {item_at(threadIdx.x + i * NT, g1)};
-      band_group_step_any<1, GMAX, RAGGED>(exact, M, D, st1, G, g1, it, out1, (size_t)IPS, dt,
-                                            min_conc, mx1);
-    }
+    band_step_any<kStripRows, RAGGED>(exact, P, st1, G, g1, out1, (size_t)IPS, splits, dt, min_conc, mx1);
     // Intermediate rows outside the grid are the planes' zero rows.
     const int zlo = (b == 0) ? 0 : -1;                            // grid row -1
     const int zhi = (b * R + R >= g.H) ? g.H - (b * R - 1) : -1;  // grid row H
-    for (int i = threadIdx.x; i < 2 * G * g.RS; i += NT) {
+    for (int i = threadIdx.x; i < 2 * G * g.RS; i += blockDim.x) {
       const int z = i / (G * g.RS), r = i - z * G * g.RS;
       const int row = z == 0 ? zlo : zhi;
       if (row < 0) continue;
@@ -1018,14 +1030,10 @@ __device__ bool stream_step2(const SimArgs &A, const ModelSmem &M, const DenseSm
     g2.y0 = b * R;
     g2.H = min(R, g.H - b * R);
     g2.PS = IPS;
-    g2.Q = g2.H * g.Wg;
-    const int n2 = (g2.Q + NT - 1) / NT;
-    for (int i = 0; i < n2; ++i) {
-      const Item it[1] = {item_at(threadIdx.x + i * NT, g2)};
-      band_group_step_any<1, GMAX, RAGGED>(exact, M, D, inter, G, g2, it,
-                                            gl_nxt + (size_t)g2.y0 * g.RS, gps, dt, min_conc,
-                                            mx2);
-    }
+    g2.PSb = 4 * IPS;
+    g2.Q = strip_count<kStripRows>(g2.H, g.Wg);
+    band_step_any<kStripRows, RAGGED>(exact, P, inter, G, g2, gl_nxt + (size_t)g2.y0 * g.RS, gps, splits, dt,
+                          min_conc, mx2);
     __syncthreads();  // the intermediate is free again
   }
   fence_proxy_async_global();  // this pass's writes before the next pass's copies
@@ -1037,17 +1045,16 @@ __device__ bool stream_step2(const SimArgs &A, const ModelSmem &M, const DenseSm
 // Hb + 1), the last row to the band below (its row 0).  Shared-memory planes
 // are reached through the cluster's distributed shared memory, global slots
 // directly (a cluster's CTAs are consecutive blocks).
-template <int NT, int GMAX>
 __device__ __forceinline__ void push_halos(const SimArgs &A, const StatePtrs &sp, const Geom &g,
                                            int G, int nxt, int rank, int C, int Hb) {
   cg::cluster_group cl = cg::this_cluster();
   const int n4 = g.RS / 4;
-  for (int i = threadIdx.x; i < G * 2 * n4; i += NT) {
+  for (int i = threadIdx.x; i < G * 2 * n4; i += blockDim.x) {
     const int p = i / (2 * n4), rem = i - p * 2 * n4;
     const int dir = rem / n4, c = rem - dir * n4;
     const int dst = dir == 0 ? rank - 1 : rank + 1;
     if (dst < 0 || dst >= C) continue;
-    float *pl = plane_of<GMAX>(sp, g, p, nxt);
+    float *pl = plane_of(sp, g, p, nxt);
     const float4 v =
         *reinterpret_cast<const float4 *>(chk<4>(pl + (dir == 0 ? 1 : g.H) * g.RS + 4 * c));
     const int off = (dir == 0 ? Hb + 1 : 0) * g.RS + 4 * c;
@@ -1061,15 +1068,14 @@ __device__ __forceinline__ void push_halos(const SimArgs &A, const StatePtrs &sp
 
 // Copies the first min(G, A.state_planes) genes' current values of the
 // block's rows into dst ([plane][H][W], unpadded).
-template <int NT, int GMAX>
 __device__ __forceinline__ void write_planes(const SimArgs &A, const StatePtrs &sp, const Geom &g,
                                           int G, int par, float *dst) {
   const int planes_out = min(G, A.state_planes);
-  for (int i = threadIdx.x; i < planes_out * g.W * g.H; i += NT) {
+  for (int i = threadIdx.x; i < planes_out * g.W * g.H; i += blockDim.x) {
     const int kk = i / (g.W * g.H), r = i - kk * g.W * g.H;
     const int y = r / g.W, x = r - y * g.W;
     dst[((size_t)kk * g.Hg + g.y0 + y) * g.W + x] =
-        *chk<1>(plane_of<GMAX>(sp, g, kk, par) + cell_offset(g, y, x));
+        *chk<1>(plane_of(sp, g, kk, par) + cell_offset(g, y, x));
   }
 }
 
@@ -1083,13 +1089,12 @@ __device__ __forceinline__ void cluster_share(T *slots, T v, int rank, int C) {
   cl.sync();
 }
 
-// The simulation kernel.
-//   NT      threads per block
-//   GMAX    most genes (products in use) per model
-//   ITEMS   float4 groups each thread owns when LOOP is false (geometry
-//           computed once per launch)
-//   LOOP    grids with more groups than NT * ITEMS: each thread walks its
-//           groups with incrementally updated geometry
+// The simulation kernel.  A.threads threads per block (whole warps).
+//   NTMAX   most threads per block (the register budget: 65536 / NTMAX)
+//   LOOP    false: one chunk of strips per warp, geometry computed once per
+//           launch; warp w owns chunk w % chunks and takes its part of the
+//           genes, w / chunks of (warps / chunks) parts.  true: the warps walk
+//           (chunk, gene part) items, any grid size
 //   RAGGED  W is not a multiple of 4
 //   TRACE   writes trace frames (trace_out) during the step loop; only the
 //           variants compiled for it carry that code
@@ -1101,18 +1106,19 @@ __device__ __forceinline__ void cluster_share(T *slots, T v, int rank, int C) {
 //           and passes the same cluster barriers: the model index, the step
 //           max and the fitness sum are shared values, identical bits in
 //           every CTA.
-template <int NT, int GMAX, int ITEMS, bool LOOP, bool RAGGED, bool CL, bool TRACE, int ST>
-__global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) sim_kernel(const SimArgs A) {
+template <int NTMAX, bool LOOP, bool RAGGED, bool CL, bool TRACE, int ST>
+__global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
   extern __shared__ __align__(128) unsigned char smem[];
   ModelSmem &M = *reinterpret_cast<ModelSmem *>(smem);
-  DenseSmem &D = *reinterpret_cast<DenseSmem *>(smem + kDenseOffset);
+  ProgSmem &P = *reinterpret_cast<ProgSmem *>(smem + kProgOffset);
   float *s_red = reinterpret_cast<float *>(smem + kRedOffset);
   double *s_dred = reinterpret_cast<double *>(smem + kDredOffset);
   int *s_work = reinterpret_cast<int *>(smem + kWorkOffset);
   float *s_cmax = reinterpret_cast<float *>(smem + kCmaxOffset);
   double *s_csum = reinterpret_cast<double *>(smem + kCsumOffset);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int NT = blockDim.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = uniform(tid >> 5), n_warps = NT >> 5;
   int rank = 0, C = 1;
   if constexpr (CL) {
     rank = (int)cg::this_cluster().block_rank();
@@ -1125,15 +1131,20 @@ __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) sim_kernel(const SimA
   g.y0 = rank * Hb;
   g.H = min(A.H - g.y0, Hb);
   g.Wg = A.Wg;
-  g.RS = row_floats(A.W);
-  g.PS = (Hb + 2) * g.RS;
-  g.Q = g.H * A.Wg;
+  g.RS = A.row_floats;
+  g.PS = A.plane_floats;
+  g.RSb = A.row_bytes;
+  g.edges = 32 % g.Wg != 0;
+  g.PSb = A.plane_bytes;
+  g.Q = strip_count<kStripRows>(g.H, A.Wg);
+  g.inv_wg = A.inv_wg;
   const float dt = A.dt, min_conc = A.min_conc;
   uint4 *Mw = reinterpret_cast<uint4 *>(smem);
 
   StatePtrs sp;
   sp.sm = reinterpret_cast<float *>(smem + kStateOffset);
   sp.gl = A.gstate ? A.gstate + (size_t)blockIdx.x * (size_t)A.slot_floats : nullptr;
+  sp.gmax = A.gmax;
 
 #if GRN_BOUNDS_CHECK
   if (tid == 0) {
@@ -1162,18 +1173,17 @@ __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) sim_kernel(const SimA
     __syncthreads();
   }
 
+  // Chunks of a full band: the same in every CTA of a cluster.
+  const int chunks = (strip_count<kStripRows>(ST ? min(Hb, A.band_rows) : Hb, g.Wg) + 31) / 32;
   // Fixed items: geometry once per launch.
-  Item items[LOOP ? 1 : ITEMS];
+  Strip<kStripRows> fixed;
+  int fixed_part = 0;
+  const int fixed_splits = LOOP ? 1 : max(1, n_warps / chunks);
   if constexpr (!LOOP) {
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) items[i] = item_at(tid + i * NT, g);
+    fixed = strip_at<kStripRows>((warp % chunks) * 32 + lane, g);
+    fixed_part = warp / chunks;
+    if (fixed_part >= fixed_splits) fixed_part = GRN_MAX_GENES;  // no work
   }
-  // Walking items: per-iteration stride (ITEMS * NT groups) in (row, group
-  // column).
-  const int dy = (ITEMS * NT) / g.Wg, dgx = ITEMS * NT - dy * g.Wg;
-  const int n_iter = (g.Q + ITEMS * NT - 1) / (ITEMS * NT);
-  // Items per thread of a full band: the same in every CTA of a cluster.
-  const int n_iter_band = (Hb * g.Wg + NT - 1) / NT;
 
   for (int iter = 0;; ++iter) {
     int m;
@@ -1216,9 +1226,9 @@ __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) sim_kernel(const SimA
     sp.n_sm = min(G, A.planes / 2);
     const bool exact = !(A.fast_ok && (M.hdr.flags & kFlagFast) &&
                          G <= GRN_MAX_GENES);
-    const bool bad = G < 1 || G > GMAX || M.hdr.n_links < 0 ||
+    const bool bad = G < 1 || G > GRN_MAX_GENES || M.hdr.n_links < 0 ||
                      M.hdr.n_links > GRN_MAX_LINKS || (sp.n_sm < G && sp.gl == nullptr) ||
-                     (!LOOP && n_iter_band > ITEMS) ||
+                     ((sp.n_sm < G || ST) && G > A.gmax) || (!LOOP && chunks > n_warps) ||
                      (ST && (A.band_rows < 1 || sp.gl == nullptr || A.planes != 0));
     if (bad) {
       if (tid == 0 && rank == 0) {
@@ -1231,10 +1241,9 @@ __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) sim_kernel(const SimA
       continue;
     }
 
-    if (!exact) {
-      build_dense(M, D, tid);
-      __syncthreads();
-    }
+    const int splits = LOOP ? choose_splits(chunks, n_warps, G) : fixed_splits;
+    build_program(M, P, splits, tid);
+    __syncthreads();
 
     double error = 0.0, change_sum = 0.0;
     int steps_total = 0;
@@ -1254,7 +1263,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) sim_kernel(const SimA
         float v = 0.0f;
         if (kk < A.n_in && y >= 0 && y < g.Hg && x < g.W)
           v = init[((size_t)kk * g.Hg + y) * g.W + x];
-        float *pl = plane_of<GMAX>(sp, g, kk, kb < G ? 0 : 1);
+        float *pl = plane_of(sp, g, kk, kb < G ? 0 : 1);
         *chk<1>(pl + r) = v;
       }
       if constexpr (ST == 2) {
@@ -1262,8 +1271,9 @@ __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) sim_kernel(const SimA
         // cells are never written by a step, so they start at 0 here (the
         // one-step pass's stage copies that may land there carry the
         // planes' zero cells in the same columns).
-        float *inter = sp.sm + (size_t)GMAX * (A.band_rows + 4) * g.RS;
-        for (int i = tid; i < GMAX * (A.band_rows + 2) * g.RS; i += NT) *chk<1>(inter + i) = 0.0f;
+        float *inter = sp.sm + (size_t)sp.gmax * (A.band_rows + 4) * g.RS;
+        for (int i = tid; i < sp.gmax * (A.band_rows + 2) * g.RS; i += NT)
+          *chk<1>(inter + i) = 0.0f;
       }
       if constexpr (ST) fence_proxy_async_global();  // before the first bulk copies
       if constexpr (CL) cg::this_cluster().sync();
@@ -1276,41 +1286,35 @@ __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) sim_kernel(const SimA
       if constexpr (TRACE) {
         trace = A.trace_out + ((size_t)orig * A.n_exp + e) * A.trace_frames * A.state_planes *
                                   g.W * g.Hg;
-        write_planes<NT, GMAX>(A, sp, g, G, 0, trace);
+        write_planes(A, sp, g, G, 0, trace);
       }
 
-      double change = 1.0;
+      float change = 1.0f;
       int step = 0;
       int par = 0;  // buffer holding the current values
-      while (step < A.n_steps && change > A.min_conc_change) {
+      while (step < A.n_steps && change > A.change_bound) {
         float mx = 0.0f;
         int adv = 1;  // Euler steps this iteration advanced
-        if constexpr (ST == 2) {
-          // Two steps per pass while two remain.  If the first step's change
-          // already ends the simulation, that step is run alone again (the
-          // one-step pass, R + 1 rows per band in the same shared memory),
-          // so the state is the one after exactly one step.
-          bool ok;
-          if (step + 2 <= A.n_steps) {
+        if constexpr (ST) {
+          // ST == 2: two steps per pass while two remain.  If the first
+          // step's change already ends the simulation, that step is run alone
+          // again (the one-step pass, in the same shared memory), so the
+          // state is the one after exactly one step.
+          bool ok = true, single = true;
+          if (ST == 2 && step + 2 <= A.n_steps) {
             float mx2 = 0.0f;
-            ok = stream_step2<NT, GMAX, RAGGED>(A, M, D, sp, g, G, par, exact, dt, min_conc, mx,
-                                                mx2, bars, mphase, s_stream_fail);
+            ok = stream_step2<RAGGED>(A, P, sp, g, G, splits, par, exact, dt, min_conc, mx, mx2,
+                                          bars, mphase, s_stream_fail);
             if (ok) {
-              const float b1 = block_max<NT>(mx, s_red, par ^ 1, lane, warp);
-              if ((double)b1 > A.min_conc_change) {
-                mx = mx2;
-                adv = 2;
-              } else {
-                mx = 0.0f;
-                ok = stream_step<NT, GMAX, RAGGED>(A, M, D, sp, g, G, par, exact, dt, min_conc,
-                                                   mx, bars, mphase, s_stream_fail,
-                                                   A.band_rows + 1);
-              }
+              const float b1 = block_max(mx, s_red, par ^ 1, lane, warp, n_warps);
+              single = !(b1 > A.change_bound);
+              mx = single ? 0.0f : mx2;
+              adv = single ? 1 : 2;
             }
-          } else {
-            ok = stream_step<NT, GMAX, RAGGED>(A, M, D, sp, g, G, par, exact, dt, min_conc, mx,
-                                               bars, mphase, s_stream_fail, A.band_rows + 1);
           }
+          if (ok && single)
+            ok = stream_step<RAGGED>(A, P, sp, g, G, splits, par, exact, dt, min_conc, mx, bars,
+                                         mphase, s_stream_fail, A.band_rows);
           if (!ok) {
             if (tid == 0) {
               atomicExch(A.error_flag, 2);
@@ -1318,86 +1322,45 @@ __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) sim_kernel(const SimA
             }
             return;  // every thread of the block: the decision is block-uniform
           }
-        } else if constexpr (ST) {
-          if (!stream_step<NT, GMAX, RAGGED>(A, M, D, sp, g, G, par, exact, dt, min_conc, mx,
-                                              bars, mphase, s_stream_fail, A.band_rows)) {
-            if (tid == 0) {
-              atomicExch(A.error_flag, 2);
-              A.raw_error[orig] = __longlong_as_double(0x7ff8000000000000ll);
-            }
-            return;  // every thread of the block: the decision is block-uniform
-          }
         } else if constexpr (!LOOP) {
-          // All ITEMS groups of the thread at once (items past the grid are
-          // clamped duplicates and store nothing).
-          if (exact)
-            group_step<ITEMS, GMAX, GMAX, true, RAGGED>(M, D, sp, g, items, par, dt, min_conc,
-                                                        mx);
-          else
-            group_step_fast<ITEMS, GMAX, RAGGED>(M, D, sp, g, items, par, dt, min_conc, mx);
+          strip_step_any<kStripRows, RAGGED>(exact, P, sp, G, g, fixed, fixed_part, splits, par, dt,
+                                     min_conc, mx);
         } else {
-          // ITEMS groups per iteration (more loads in flight), each
-          // advanced by ITEMS * NT groups.
-          int y[ITEMS], gx[ITEMS];
-#pragma unroll
-          for (int j = 0; j < ITEMS; ++j) {
-            y[j] = (tid + j * NT) / g.Wg;
-            gx[j] = (tid + j * NT) - y[j] * g.Wg;
-          }
-          for (int i = 0; i < n_iter; ++i) {
-            Item it[ITEMS];
-#pragma unroll
-            for (int j = 0; j < ITEMS; ++j) {
-              const int q = tid + (i * ITEMS + j) * NT;
-              it[j] = q < g.Q ? make_item(y[j], gx[j], true, g) : item_at(q, g);
-            }
-            if (exact)
-              group_step<ITEMS, GMAX, GMAX, true, RAGGED>(M, D, sp, g, it, par, dt, min_conc,
-                                                          mx);
-            else
-              group_step_fast<ITEMS, GMAX, RAGGED>(M, D, sp, g, it, par, dt, min_conc, mx);
-#pragma unroll
-            for (int j = 0; j < ITEMS; ++j) {
-              y[j] += dy;
-              gx[j] += dgx;
-              if (gx[j] >= g.Wg) {
-                gx[j] -= g.Wg;
-                ++y[j];
-              }
-            }
+          const int shift = 31 - __clz(splits), items = chunks * splits;
+          for (int i = warp; i < items; i += n_warps) {
+            const Strip<kStripRows> st = strip_at<kStripRows>((i >> shift) * 32 + lane, g);
+            strip_step_any<kStripRows, RAGGED>(exact, P, sp, G, g, st, i & (splits - 1), splits, par, dt,
+                                       min_conc, mx);
           }
         }
-        float bm = block_max<NT>(mx, s_red, par, lane, warp);
+        change = block_max(mx, s_red, par, lane, warp, n_warps);
         if constexpr (CL) {
-          push_halos<NT, GMAX>(A, sp, g, G, par ^ 1, rank, C, Hb);
-          cluster_share(s_cmax + par * kMaxCluster, bm, rank, C);
-          bm = 0.0f;
-          for (int r = 0; r < C; ++r) bm = fmaxf(bm, s_cmax[par * kMaxCluster + r]);
+          push_halos(A, sp, g, G, par ^ 1, rank, C, Hb);
+          cluster_share(s_cmax + par * kMaxCluster, change, rank, C);
+          change = 0.0f;
+          for (int r = 0; r < C; ++r) change = fmaxf(change, s_cmax[par * kMaxCluster + r]);
         }
-        change = (double)bm;
         par ^= 1;
         step += adv;
         if constexpr (TRACE) {
           if (step % A.trace_every == 0 && step / A.trace_every < A.trace_frames)
-            write_planes<NT, GMAX>(A, sp, g, G, par,
-                                   trace + (size_t)(step / A.trace_every) * A.state_planes *
-                                               g.W * g.Hg);
+            write_planes(A, sp, g, G, par,
+                         trace + (size_t)(step / A.trace_every) * A.state_planes * g.W * g.Hg);
         }
       }
       steps_total += step;
-      change_sum += change;
+      change_sum += (double)change;
       if (A.state_out)  // final state of this experiment, unpadded [gene][y][x]
-        write_planes<NT, GMAX>(A, sp, g, G, par,
+        write_planes(A, sp, g, G, par,
                                A.state_out + ((size_t)orig * A.n_exp + e) * A.state_planes *
                                                  g.W * g.Hg);
 
       // Fitness of the experiment (simstate.cpp:135-158), FP64 sums.
       const float *tgt = A.target + (size_t)e * A.n_target * A.W * A.H;
-      double acc = 0.0;
-      for (int i = tid; i < g.W * g.H; i += NT) {
+      const auto term = [&](int i, double acc) {
         const int y = i / g.W, x = i - y * g.W;
         for (int kk = 0; kk < A.n_target; ++kk) {
-          const double a = *chk<1>(plane_of<GMAX>(sp, g, A.n_in + kk, par) + cell_offset(g, y, x));
+          const double a = *chk<1>(plane_of(sp, g, A.n_in + kk, par) + cell_offset(g, y, x));
           const double b = tgt[((size_t)kk * g.Hg + g.y0 + y) * g.W + x];
           if (A.fitness_kind == GRN_FITNESS_MSE) {
             acc += (a - b) * (a - b);
@@ -1406,8 +1369,9 @@ __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) sim_kernel(const SimA
             if (sub > 0) acc += log(1.0 + sub);
           }
         }
-      }
-      double dist = block_sum<NT>(acc, s_dred, lane, warp);
+        return acc;
+      };
+      double dist = cell_sum(g.W * g.H, term, s_dred, lane, warp, n_warps);
       if constexpr (CL) {
         cluster_share(s_csum, dist, rank, C);
         dist = 0.0;
@@ -1439,40 +1403,29 @@ struct VariantEntry {
   KernelFn fn;
 };
 
-#define GRN_VARIANT_X(NT, GMAX, ITEMS, LOOP, CL, TR, ST)                                   \
-  {{NT, GMAX, ITEMS, LOOP, false, CL, TR, ST},                                            \
-   &sim_kernel<NT, GMAX, ITEMS, LOOP, false, CL, TR, ST>},                                \
-  {{NT, GMAX, ITEMS, LOOP, true, CL, TR, ST}, &sim_kernel<NT, GMAX, ITEMS, LOOP, true, CL, TR, ST>}
-#define GRN_VARIANT_T(NT, GMAX, ITEMS, LOOP, CL, TR) \
-  GRN_VARIANT_X(NT, GMAX, ITEMS, LOOP, CL, TR, 0)
-#define GRN_VARIANT(NT, GMAX, ITEMS, LOOP, CL) GRN_VARIANT_T(NT, GMAX, ITEMS, LOOP, CL, false)
+#define GRN_VARIANT(NT, LOOP, CL, TR, ST)                                     \
+  {{NT, LOOP, false, CL, TR, ST}, &sim_kernel<NT, LOOP, false, CL, TR, ST>}, \
+  {{NT, LOOP, true, CL, TR, ST}, &sim_kernel<NT, LOOP, true, CL, TR, ST>}
 
 const VariantEntry kVariants[] = {
-    GRN_VARIANT(256, 4, 1, false, false),  GRN_VARIANT(256, 8, 1, false, false),
-    GRN_VARIANT(256, 16, 1, false, false), GRN_VARIANT(512, 4, 2, false, false),
-    GRN_VARIANT(512, 8, 2, false, false),
-    GRN_VARIANT(512, 8, 1, true, false),   GRN_VARIANT(512, 16, 1, true, false),
-    GRN_VARIANT(256, 4, 1, true, false),
+    GRN_VARIANT(512, false, false, false, 0), GRN_VARIANT(512, true, false, false, 0),
+    GRN_VARIANT(1024, false, false, false, 0), GRN_VARIANT(1024, true, false, false, 0),
     // cluster-split
-    GRN_VARIANT(512, 8, 1, false, true),
-    GRN_VARIANT(512, 8, 1, true, true),    GRN_VARIANT(512, 16, 1, true, true),
+    GRN_VARIANT(512, true, true, false, 0),
     // trace frames (one model at a time: any grid, any gene count)
-    GRN_VARIANT_T(256, 16, 1, true, false, true),
+    GRN_VARIANT(512, true, false, true, 0),
     // streaming (bands staged by bulk copies)
-    GRN_VARIANT_X(512, 8, 1, true, false, false, 1),
-    GRN_VARIANT_X(512, 16, 1, true, false, false, 1),
+    GRN_VARIANT(512, true, false, false, 1), GRN_VARIANT(1024, true, false, false, 1),
     // streaming with temporal blocking: two Euler steps per pass
-    GRN_VARIANT_X(512, 8, 1, true, false, false, 2),
-    GRN_VARIANT_X(512, 16, 1, true, false, false, 2),
+    GRN_VARIANT(512, true, false, false, 2),
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
 const VariantEntry *find_variant(const KernelVariant &v) {
   for (int i = 0; i < kNumVariants; ++i) {
     const KernelVariant &k = kVariants[i].v;
-    if (k.threads == v.threads && k.gmax == v.gmax && k.items == v.items &&
-        k.loop == v.loop && k.ragged == v.ragged && k.cluster == v.cluster &&
-        k.trace == v.trace && k.stream == v.stream)
+    if (k.max_threads == v.max_threads && k.loop == v.loop && k.ragged == v.ragged &&
+        k.cluster == v.cluster && k.trace == v.trace && k.stream == v.stream)
       return &kVariants[i];
   }
   return nullptr;
@@ -1486,7 +1439,8 @@ int sim_variant_count() { return kNumVariants; }
 
 KernelVariant sim_variant(int i) { return kVariants[i].v; }
 
-cudaError_t sim_occupancy(const KernelVariant &v, size_t smem_bytes, int *blocks_per_sm) {
+cudaError_t sim_occupancy(const KernelVariant &v, int threads, size_t smem_bytes,
+                          int *blocks_per_sm) {
   const VariantEntry *e = find_variant(v);
   if (!e) return cudaErrorInvalidValue;
   cudaError_t err =
@@ -1496,12 +1450,12 @@ cudaError_t sim_occupancy(const KernelVariant &v, size_t smem_bytes, int *blocks
     cudaGetLastError();
     return cudaSuccess;
   }
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, e->fn, v.threads,
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, e->fn, threads,
                                                        smem_bytes);
 }
 
-cudaError_t sim_cluster_occupancy(const KernelVariant &v, size_t smem_bytes, int cluster,
-                                  int *clusters) {
+cudaError_t sim_cluster_occupancy(const KernelVariant &v, int threads, size_t smem_bytes,
+                                  int cluster, int *clusters) {
   *clusters = 0;
   const VariantEntry *e = find_variant(v);
   if (!e || !v.cluster || cluster < 2 || cluster > kMaxCluster) return cudaErrorInvalidValue;
@@ -1514,7 +1468,7 @@ cudaError_t sim_cluster_occupancy(const KernelVariant &v, size_t smem_bytes, int
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cluster, 1, 1);
-  cfg.blockDim = dim3(v.threads, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem_bytes;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1533,7 +1487,9 @@ cudaError_t sim_cluster_occupancy(const KernelVariant &v, size_t smem_bytes, int
 cudaError_t sim_launch(const LaunchPlan &plan, const SimArgs &args, cudaStream_t stream) {
   const VariantEntry *e = find_variant(plan.v);
   if (!e) return cudaErrorInvalidValue;
-  if (plan.v.cluster != (plan.cluster > 1)) return cudaErrorInvalidValue;
+  if (plan.v.cluster != (plan.cluster > 1) || plan.threads < 32 || plan.threads % 32 != 0 ||
+      plan.threads > plan.v.max_threads)
+    return cudaErrorInvalidValue;
   cudaError_t err = cudaFuncSetAttribute(e->fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)plan.smem_bytes);
   if (err != cudaSuccess) return err;
@@ -1547,7 +1503,7 @@ cudaError_t sim_launch(const LaunchPlan &plan, const SimArgs &args, cudaStream_t
     if (err != cudaSuccess) return err;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(plan.blocks, 1, 1);
-    cfg.blockDim = dim3(plan.v.threads, 1, 1);
+    cfg.blockDim = dim3(plan.threads, 1, 1);
     cfg.dynamicSmemBytes = plan.smem_bytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -1559,7 +1515,7 @@ cudaError_t sim_launch(const LaunchPlan &plan, const SimArgs &args, cudaStream_t
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, e->fn, args);
   }
-  e->fn<<<plan.blocks, plan.v.threads, plan.smem_bytes, stream>>>(args);
+  e->fn<<<plan.blocks, plan.threads, plan.smem_bytes, stream>>>(args);
   return cudaGetLastError();
 }
 

@@ -90,8 +90,7 @@ struct grn_ctx {
   bool autotune = true;
   struct Tuned {
     grn::KernelVariant v;
-    int cluster, planes;
-    double ms;
+    int schedule, threads, cluster;
   };
   std::map<std::array<int, 7>, Tuned> tuned;
   std::string last_tuning;  // the last autotuning's candidates and times
@@ -224,54 +223,45 @@ int host_threads(const grn_ctx *ctx) {
   return n ? (int)n : 1;
 }
 
-// Autotuner, first stage: every compiled kernel variant that can run the
-// batch is scored by its resident useful threads per SM (occupancy x
-// threads that own a group), fixed items preferred over walking ones and
-// all-shared-memory state over state spilling to global slots.
-// Every feasible launch plan for a batch, with the heuristic throughput
-// score of each.
 // Rows per staged band of the streaming schedule: two stages of
-// gmax x (rows + 2) padded rows must fit the shared memory left over, one
-// stage's bytes must stay below the mbarrier transaction limit (2^20), and
-// a multiple of NT / Wg rows keeps every thread busy when Wg divides NT.
-int stream_rows(int W, int H, int gmax, size_t room, int threads) {
-  const int Wg = (W + 3) / 4;
+// genes x (rows + 2) padded rows, and one row that the last strip of an odd
+// band may read, must fit the shared memory left over, and one stage's bytes
+// must stay below the mbarrier transaction limit (2^20); an even count, since
+// a thread computes two rows.
+int stream_rows(int W, int H, int genes, size_t room) {
   const size_t row_bytes = (size_t)grn::row_floats(W) * sizeof(float);
-  long r = (long)(room / (2 * gmax * row_bytes)) - 2;
+  long r = (long)((room - std::min(room, row_bytes)) / (2 * genes * row_bytes)) - 2;
   r = std::min<long>(r, H);
-  while (r > 1 && (size_t)gmax * (r + 2) * row_bytes >= (size_t)1 << 20) --r;
+  while (r > 1 && (size_t)genes * (r + 2) * row_bytes >= (size_t)1 << 20) --r;
   if (r < 1) return 0;
-  if (threads % Wg == 0 && r >= threads / Wg) r -= r % (threads / Wg);
+  if (r > 1 && r < H) r &= ~1L;
   return (int)r;
 }
 
 // Output rows per band of the two-steps-per-pass streaming variant: its
 // stage holds R + 4 rows of every gene and its intermediate R + 2, i.e.
-// gmax * (2R + 6) rows (the one-step pass it falls back to uses the same
-// space as two stages of R + 3 rows).  Rows of a pass's step one are a
-// multiple of the block's threads where that is possible.
-int stream2_rows(int W, int H, int gmax, size_t room, int threads) {
-  const int Wg = (W + 3) / 4;
+// genes * (2R + 6) rows and the row past an odd band (the one-step pass it
+// falls back to uses the same space).
+int stream2_rows(int W, int H, int genes, size_t room) {
   const size_t row_bytes = (size_t)grn::row_floats(W) * sizeof(float);
-  long r = ((long)(room / (gmax * row_bytes)) - 6) / 2;
+  long r = ((long)((room - std::min(room, row_bytes)) / (genes * row_bytes)) - 6) / 2;
   r = std::min<long>(r, H);
   // One pass's copies complete on one mbarrier (transaction count < 2^20).
-  while (r > 1 && (size_t)gmax * (r + 4) * row_bytes >= (size_t)1 << 20) --r;
+  while (r > 1 && (size_t)genes * (r + 4) * row_bytes >= (size_t)1 << 20) --r;
   if (r < 1) return 0;
-  if (threads % Wg == 0) {
-    const long per = threads / Wg;  // rows per full pass of the block's threads
-    if (r + 2 >= per && (r + 2) % per != 0) r -= (r + 2) % per;
-  }
-  return r >= 1 ? (int)r : 0;
+  if (r > 1 && r < H) r &= ~1L;
+  return (int)r;
 }
 
+// Every feasible launch plan for a batch, best heuristic score first.
 grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace,
                            std::vector<std::pair<double, LaunchPlan>> *out) {
   const int W = ctx->p.dim_x, H = ctx->p.dim_y;
-  const int Wg = (W + 3) / 4;
   const bool ragged = (W % 4) != 0;
+  max_genes = std::max(1, max_genes);
   const size_t fixed = grn::sim_fixed_smem_bytes();
   const size_t optin = (size_t)ctx->smem_optin;
+  const size_t row_bytes = (size_t)grn::row_floats(W) * sizeof(float);
   // A trace runs on the trace variants whatever schedule is forced.
   const int sched = trace ? GRN_SCHEDULE_WALK_ITEMS : ctx->forced_schedule;
   static const int kClusterSizes[] = {2, 4, 8, 16};
@@ -279,40 +269,40 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
   const int nv = grn::sim_variant_count();
   for (int i = 0; i < nv; ++i) {
     const grn::KernelVariant v = grn::sim_variant(i);
-    if (v.gmax < max_genes || v.ragged != ragged || v.trace != trace) continue;
-    if (ctx->forced_threads && !trace && v.threads != ctx->forced_threads) continue;
+    if (max_genes > GRN_MAX_GENES || v.ragged != ragged || v.trace != trace) continue;
     if (v.stream) {
       // Streaming: only where the planes do not all fit shared memory.
       const int own = v.stream == 2 ? GRN_SCHEDULE_STREAM2 : GRN_SCHEDULE_STREAM;
       if (sched != GRN_SCHEDULE_AUTO && sched != own) continue;
+      if (ctx->forced_threads && ctx->forced_threads != v.max_threads) continue;
       const size_t plane_bytes = (size_t)grn::plane_floats(W, H) * sizeof(float);
       const int fit = optin > fixed ? (int)((optin - fixed) / plane_bytes) & ~1 : 0;
       if (sched == GRN_SCHEDULE_AUTO && fit / 2 >= max_genes) continue;
       const size_t room = optin > fixed ? optin - fixed : 0;
-      const int R = v.stream == 2 ? stream2_rows(W, H, v.gmax, room, v.threads)
-                                  : stream_rows(W, H, v.gmax, room, v.threads);
+      const int R = v.stream == 2 ? stream2_rows(W, H, max_genes, room)
+                                  : stream_rows(W, H, max_genes, room);
       if (R < 1) continue;
-      const size_t rows = v.stream == 2 ? (size_t)v.gmax * (2 * R + 6)
-                                        : (size_t)2 * v.gmax * (R + 2);
-      const size_t smem = fixed + rows * grn::row_floats(W) * sizeof(float);
+      const size_t rows = v.stream == 2 ? (size_t)max_genes * (2 * R + 6)
+                                        : (size_t)2 * max_genes * (R + 2);
+      const size_t smem = fixed + (rows + 1) * row_bytes;
       int per_sm = 0;
-      GRN_CUDA(ctx, grn::sim_occupancy(v, smem, &per_sm));
+      GRN_CUDA(ctx, grn::sim_occupancy(v, v.max_threads, smem, &per_sm));
       const int ctas = per_sm * ctx->n_sm;
       if (ctas < 1) continue;
       LaunchPlan plan{};
       plan.v = v;
       plan.schedule = own;
+      plan.threads = v.max_threads;
+      plan.gmax = max_genes;
       plan.planes = 0;
       plan.smem_bytes = smem;
       plan.blocks_per_sm = per_sm;
-      plan.slot_floats = 2LL * v.gmax * grn::plane_floats(W, H);
+      plan.slot_floats = 2LL * max_genes * grn::plane_floats(W, H);
       plan.cluster = 1;
       plan.band_rows = R;
       plan.blocks = std::max(1, std::min(n_models, ctas));
-      const double busy = (double)std::min(ctas, n_models) * std::min(v.threads, R * Wg);
-      // Heuristic rank below the walking / all-global plans (faster only where the
-      // slots' traffic leaves L2); the autotuner measures it against them.
-      out->push_back({busy * 0.6 - 1e-3 * v.gmax, plan});
+      const double warps = (double)std::min(ctas, n_models) * v.max_threads / 32;
+      out->push_back({warps * (v.stream == 2 ? 0.4 : 0.6), plan});
       continue;
     }
     if (sched == GRN_SCHEDULE_STREAM || sched == GRN_SCHEDULE_STREAM2) continue;
@@ -325,8 +315,7 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
       if (v.cluster && ctx->forced_cluster && C != ctx->forced_cluster) continue;
       const int Hb = (H + C - 1) / C;
       if (C > 1 && (C - 1) * Hb >= H) continue;  // every band non-empty
-      const int Qb = Hb * Wg;
-      if (!v.loop && Qb > v.threads * v.items) continue;
+      const int chunks = grn::strip_chunks(W, Hb);
       const size_t plane_bytes = (size_t)grn::plane_floats(W, H, C) * sizeof(float);
       int fit = optin > fixed ? (int)((optin - fixed) / plane_bytes) : 0;
       fit &= ~1;
@@ -335,49 +324,71 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
       const int smem_planes = std::min(fit, 2 * max_genes);
       const bool offer_global = sched == GRN_SCHEDULE_AUTO && v.loop && C == 1 &&
                                 smem_planes / 2 < max_genes && smem_planes > 0;
-      for (int gv = 0; gv < (offer_global ? 2 : 1); ++gv) {
-        const int planes = (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? 0 : smem_planes;
-        const bool spills = planes / 2 < max_genes;
-        const size_t smem = fixed + planes * plane_bytes;
-        int ctas = 0, per_sm = 0;  // resident CTAs on the device
-        if (C == 1) {
-          GRN_CUDA(ctx, grn::sim_occupancy(v, smem, &per_sm));
-          ctas = per_sm * ctx->n_sm;
-        } else {
-          int clusters = 0;
-          GRN_CUDA(ctx, grn::sim_cluster_occupancy(v, smem, C, &clusters));
-          ctas = clusters * C;
-          per_sm = 1;
-        }
-        if (ctas < 1) continue;
-        // Throughput model: busy threads (no more CTAs than models need),
-        // fixed items ahead of walking ones, and a penalty for genes kept in
-        // global memory -- mild while every resident CTA's slot fits in L2.
-        const double busy = (double)std::min(ctas, n_models * C) * std::min(v.threads, Qb);
-        const double spill_frac = spills ? 1.0 - (double)(planes / 2) / max_genes : 0.0;
-        const double slot_bytes = spills ? 2.0 * v.gmax * plane_bytes : 0.0;
-        const bool l2 = slot_bytes * ctas <= 80e6;
-        double score = busy * (v.loop ? 1.0 : 1.25) * (1.0 - (l2 ? 0.3 : 0.7) * spill_frac);
-        // One cluster barrier per step costs about as much as a step of a
-        // small band (measured): clusters only as a last resort unmeasured.
-        if (C > 1) score *= 0.3 - 0.01 * C;
-        if (gv == 1) score *= 0.9;
-        score -= 1e-3 * v.gmax;  // prefer the tighter register footprint
-        LaunchPlan plan{};
-        plan.v = v;
-        plan.schedule = C > 1                                      ? GRN_SCHEDULE_CLUSTER
-                        : (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? GRN_SCHEDULE_GLOBAL
-                        : v.loop                                    ? GRN_SCHEDULE_WALK_ITEMS
-                                                                    : GRN_SCHEDULE_FIXED_ITEMS;
-        plan.planes = planes;
-        plan.smem_bytes = smem;
-        plan.blocks_per_sm = per_sm;
-        plan.slot_floats = spills ? 2LL * v.gmax * grn::plane_floats(W, H, C) : 0;
-        plan.cluster = C;
-        plan.blocks = C > 1 ? C * std::max(1, std::min(n_models, ctas / C))
-                            : std::max(1, std::min(n_models, ctas));
-        out->push_back({score, plan});
+      // Block sizes: walking blocks are the variant's largest; fixed ones hold
+      // every chunk once, or up to 4 times (a part of the genes each).  A
+      // forced size is taken where the variant can run it.
+      std::vector<int> sizes;
+      const int ft = trace ? 0 : ctx->forced_threads;
+      if (ft) {
+        if (ft % 32 == 0 && ft <= v.max_threads && (v.max_threads == 512 || ft > 512) &&
+            (v.loop || chunks * 32 <= ft))
+          sizes.push_back(ft);
+      } else if (v.loop) {
+        sizes.push_back(v.max_threads);
+      } else {
+        for (int parts = 1; parts <= 4 && parts <= std::max(1, max_genes); ++parts)
+          if (chunks * parts * 32 <= v.max_threads &&
+              (v.max_threads == 512 || chunks * parts * 32 > 512))
+            sizes.push_back(chunks * parts * 32);
       }
+      for (const int threads : sizes)
+        for (int gv = 0; gv < (offer_global ? 2 : 1); ++gv) {
+          const int planes = (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? 0 : smem_planes;
+          const bool spills = planes / 2 < max_genes;
+          const size_t smem = fixed + planes * plane_bytes;
+          int ctas = 0, per_sm = 0;  // resident CTAs on the device
+          if (C == 1) {
+            GRN_CUDA(ctx, grn::sim_occupancy(v, threads, smem, &per_sm));
+            ctas = per_sm * ctx->n_sm;
+          } else {
+            int clusters = 0;
+            GRN_CUDA(ctx, grn::sim_cluster_occupancy(v, threads, smem, C, &clusters));
+            ctas = clusters * C;
+            per_sm = 1;
+          }
+          if (ctas < 1) continue;
+          // Throughput model: resident warps that have work (no more CTAs
+          // than models need), fixed items ahead of walking ones, and a
+          // penalty for genes kept in global memory -- mild while every
+          // resident CTA's slot fits in L2.
+          const int warps = threads / 32;
+          const double busy =
+              (double)std::min(ctas, n_models * C) * std::min(warps, chunks * std::min(4, max_genes));
+          const double spill_frac = spills ? 1.0 - (double)(planes / 2) / max_genes : 0.0;
+          const double slot_bytes = spills ? 2.0 * max_genes * plane_bytes : 0.0;
+          const bool l2 = slot_bytes * ctas <= 80e6;
+          double score = busy * (v.loop ? 1.0 : 1.25) * (1.0 - (l2 ? 0.3 : 0.7) * spill_frac);
+          // One cluster barrier per step costs about as much as a step of a
+          // small band (measured): clusters only as a last resort unmeasured.
+          if (C > 1) score *= 0.3 - 0.01 * C;
+          if (gv == 1) score *= 0.9;
+          LaunchPlan plan{};
+          plan.v = v;
+          plan.schedule = C > 1                                      ? GRN_SCHEDULE_CLUSTER
+                          : (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? GRN_SCHEDULE_GLOBAL
+                          : v.loop                                    ? GRN_SCHEDULE_WALK_ITEMS
+                                                                      : GRN_SCHEDULE_FIXED_ITEMS;
+          plan.threads = threads;
+          plan.gmax = max_genes;
+          plan.planes = planes;
+          plan.smem_bytes = smem;
+          plan.blocks_per_sm = per_sm;
+          plan.slot_floats = spills ? 2LL * max_genes * grn::plane_floats(W, H, C) : 0;
+          plan.cluster = C;
+          plan.blocks = C > 1 ? C * std::max(1, std::min(n_models, ctas / C))
+                              : std::max(1, std::min(n_models, ctas));
+          out->push_back({score, plan});
+        }
     }
   }
   if (out->empty())
@@ -397,11 +408,10 @@ grn_status choose_plan(grn_ctx *ctx, int max_genes, int n_models, LaunchPlan *ou
   return GRN_OK;
 }
 
-bool same_plan(const LaunchPlan &a, const grn::KernelVariant &v, int cluster, int planes) {
-  return a.v.threads == v.threads && a.v.gmax == v.gmax && a.v.items == v.items &&
-         a.v.loop == v.loop && a.v.ragged == v.ragged && a.v.cluster == v.cluster &&
-         a.v.stream == v.stream &&
-         a.cluster == cluster && a.planes == planes;
+bool same_plan(const LaunchPlan &a, const grn_ctx::Tuned &t) {
+  return a.v.max_threads == t.v.max_threads && a.v.loop == t.v.loop &&
+         a.v.ragged == t.v.ragged && a.v.cluster == t.v.cluster && a.v.stream == t.v.stream &&
+         a.threads == t.threads && a.schedule == t.schedule && a.cluster == t.cluster;
 }
 
 // Launches the simulation of `n_models` packed records already on the
@@ -409,7 +419,9 @@ bool same_plan(const LaunchPlan &a, const grn::KernelVariant &v, int cluster, in
 // Sets the plan's state planes and global state slots in `a` (allocating
 // the slots if they grew).
 grn_status bind_state(grn_ctx *ctx, const LaunchPlan &plan, grn::SimArgs *a) {
+  grn::set_geometry(a, a->W, a->H, plan.cluster);
   a->planes = plan.planes;
+  a->gmax = plan.gmax;
   a->band_rows = plan.band_rows;
   a->gstate = nullptr;
   a->slot_floats = 0;
@@ -454,7 +466,7 @@ grn_status launch_plan(grn_ctx *ctx, const LaunchPlan &plan, grn::SimArgs a, cud
 // per SM.  The exact gene and link counts are left out: a search's batches
 // vary in them from one generation to the next (its population grows), and
 // each new key costs a tuning run.  A kept plan is reused only where it is
-// among the batch's own candidates (same variant, cluster and planes),
+// among the batch's own candidates (same variant, schedule, block and cluster),
 // else the batch is tuned again.
 std::array<int, 7> tune_key(const grn_ctx *ctx, int n_models, int max_genes, int max_links) {
   const int genes_class = max_genes <= 4 ? 4 : max_genes <= 8 ? 8 : 16;
@@ -470,7 +482,7 @@ bool cached_plan(const grn_ctx *ctx, const std::vector<std::pair<double, LaunchP
   const auto it = ctx->tuned.find(key);
   if (it == ctx->tuned.end()) return false;
   for (const auto &c : plans)
-    if (same_plan(c.second, it->second.v, it->second.cluster, it->second.planes)) {
+    if (same_plan(c.second, it->second)) {
       *out = c.second;
       return true;
     }
@@ -560,9 +572,9 @@ grn_status autotune_plan(grn_ctx *ctx, const std::vector<std::pair<double, Launc
     const LaunchPlan &p = cand[i];
     char line[200];
     std::snprintf(line, sizeof line,
-                  "%s schedule %d threads %d gmax %d items %d cluster %d planes %d band %d "
+                  "%s schedule %d threads %d (of %d) genes %d cluster %d planes %d band %d "
                   "blocks %d ms %.4f\n",
-                  i == best ? "*" : " ", p.schedule, p.v.threads, p.v.gmax, p.v.items,
+                  i == best ? "*" : " ", p.schedule, p.threads, p.v.max_threads, p.gmax,
                   std::max(1, p.cluster), p.planes, p.band_rows, p.blocks, best_ms[i]);
     rep += line;
   }
@@ -598,7 +610,7 @@ grn_status prepare_packed(grn_ctx *ctx, const uint4 *d_words, const int32_t *d_o
   grn_status s = enumerate_plans(ctx, max_genes, n_models, trace, &plans);
   if (s != GRN_OK) return s;
   LaunchPlan plan = plans[0].second;
-  const int W = ctx->p.dim_x, H = ctx->p.dim_y, Wg = (W + 3) / 4;
+  const int W = ctx->p.dim_x, H = ctx->p.dim_y;
   grn::SimArgs a{};
   a.packed = d_words;
   a.offsets = d_offsets;
@@ -608,13 +620,13 @@ grn_status prepare_packed(grn_ctx *ctx, const uint4 *d_words, const int32_t *d_o
   a.n_target = ctx->p.n_target_morphogens;
   a.W = W;
   a.H = H;
-  a.Wg = Wg;
   a.n_steps = ctx->p.num_sim_steps;
   a.fitness_kind = ctx->p.fitness_kind;
   a.planes = plan.planes;
   a.dt = (float)ctx->p.dt;
   a.min_conc = (float)ctx->p.min_conc;
   a.min_conc_change = ctx->p.min_conc_change;
+  a.change_bound = grn::float_below(a.min_conc_change);
   a.dist_threshold = ctx->p.dist_error_threshold;
   a.initial = static_cast<const float *>(ctx->d_initial.p);
   a.target = static_cast<const float *>(ctx->d_target.p);
@@ -651,7 +663,7 @@ grn_status prepare_packed(grn_ctx *ctx, const uint4 *d_words, const int32_t *d_o
       ctx->last_tuning = kl + ctx->last_tuning;
       ctx->tuning_ms +=
           std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-      ctx->tuned[key] = grn_ctx::Tuned{plan.v, plan.cluster, plan.planes, 0.0};
+      ctx->tuned[key] = grn_ctx::Tuned{plan.v, plan.schedule, plan.threads, plan.cluster};
     }
   }
   s = bind_state(ctx, plan, &a);
@@ -701,7 +713,7 @@ void fill_launch_stats(grn_eval_stats *stats, int n, std::chrono::steady_clock::
   stats->h2d_bytes = (int64_t)h2d;
   stats->d2h_bytes = (int64_t)d2h;
   stats->schedule = plan.schedule;
-  stats->threads_per_block = plan.v.threads;
+  stats->threads_per_block = plan.threads;
   stats->blocks = plan.blocks;
   stats->cluster_size = std::max(1, plan.cluster);
 }

@@ -127,6 +127,7 @@ grn_status pack_model(const grn_product *products, int n_products,
         if (!(kn > 0) || !(kn <= 1e300) || n > 32) hdr.flags &= ~kFlagFast;
       }
       if (n == 0) {
+        hdr.flags &= ~kFlagFast;  // a constant term: only the exact path has it
         pl.slot = kConstSlot;  // pow(x, 0) = pow(K, 0) = 1: Hill value 1/2
         pl.a = 0.0f;
         pl.b = 0.0f;
@@ -163,23 +164,6 @@ grn_status pack_model(const grn_product *products, int n_products,
     }
     if (g.n_or + g.n_and > 0) ++c.reg_genes;
   }
-  // The kernel's dense regulation holds one link per (regulated, regulator)
-  // pair; a model with a repeated pair takes the exact path.
-  for (size_t i = 0; i < plinks.size() && (hdr.flags & kFlagFast); ++i)
-    for (size_t j = i + 1; j < plinks.size(); ++j)
-      if (plinks[i].slot == plinks[j].slot && plinks[i].slot != kConstSlot) {
-        // same slot twice within one gene's link range?
-        int gi = -1, gj = -1;
-        for (int q = 0; q < G; ++q) {
-          const int b = genes[q].link_begin, e = b + genes[q].n_or + genes[q].n_and;
-          if ((int)i >= b && (int)i < e) gi = q;
-          if ((int)j >= b && (int)j < e) gj = q;
-        }
-        if (gi == gj) {
-          hdr.flags &= ~kFlagFast;
-          break;
-        }
-      }
   hdr.n_links = (int16_t)plinks.size();
   c.links = (int)plinks.size();
   c.lg_genes = __builtin_popcount(hdr.lg_mask);

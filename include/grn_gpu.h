@@ -200,8 +200,9 @@ const char *grn_status_str(grn_status status);
 int grn_abi_version(void);
 
 /* Forces a schedule instead of the autotuner's choice (GRN_SCHEDULE_AUTO to
- * restore).  Returns GRN_ERR_CAPACITY later, at launch, if the forced
- * schedule cannot hold the batch. */
+ * restore), and its threads per block (0: any; else a multiple of 32).
+ * Returns GRN_ERR_CAPACITY later, at launch, if the forced schedule cannot
+ * hold the batch or has no kernel for that block size. */
 grn_status grn_set_schedule(grn_ctx *ctx, int schedule, int threads_per_block);
 
 /* CTAs per cluster for GRN_SCHEDULE_CLUSTER (2, 4, 8 or 16; 0: the
@@ -222,9 +223,9 @@ grn_status grn_set_autotune(grn_ctx *ctx, int enable);
 
 /* The autotuning on this context: a first line starting with '#' that
  * counts the runs so far and their host time, then the last run, one line
- * per timed plan ("*" marks the one kept): schedule, threads, gene
- * capacity, items per thread, cluster size, shared-memory planes, streaming
- * band rows and the fastest sample launch in ms.  GRN_ERR_CAPACITY if it
+ * per timed plan ("*" marks the one kept): schedule, threads (of the kernel's
+ * most), genes, cluster size, shared-memory planes, streaming band rows,
+ * blocks and the fastest sample launch in ms.  GRN_ERR_CAPACITY if it
  * was truncated to buf_len. */
 grn_status grn_autotune_report(const grn_ctx *ctx, char *buf, int buf_len);
 
