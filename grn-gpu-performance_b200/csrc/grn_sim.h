@@ -25,6 +25,8 @@ struct SimArgs {
   int32_t W, H;              // grid width (x) and height (y)
   int32_t Wg;                // float4 groups per row = ceil(W / 4)
   uint32_t inv_wg;           // ceil(2^32 / Wg) (unused when Wg is 1)
+  uint32_t inv_w;            // ceil(2^32 / W): a cell's row by multiplication, or 0
+                             // where that is not exact
   int32_t row_floats, row_bytes;      // one padded state row
   int32_t plane_floats, plane_bytes;  // one state plane (of a CTA's band)
   int32_t gmax;              // genes a global state slot (or a streaming
@@ -140,7 +142,11 @@ inline void set_geometry(SimArgs *a, int W, int H, int cluster) {
   a->W = W;
   a->H = H;
   a->Wg = (W + 3) / 4;
-  a->inv_wg = a->Wg > 1 ? (uint32_t)((((uint64_t)1 << 32) + a->Wg - 1) / a->Wg) : 0u;
+  const auto inverse = [](int d) {
+    return d > 1 ? (uint32_t)((((uint64_t)1 << 32) + d - 1) / d) : 0u;
+  };
+  a->inv_wg = inverse(a->Wg);
+  a->inv_w = (int64_t)W * H * W < (int64_t)1 << 32 ? inverse(W) : 0u;
   a->row_floats = row_floats(W);
   a->row_bytes = 4 * a->row_floats;
   a->plane_floats = (int32_t)plane_floats(W, H, cluster);

@@ -192,6 +192,8 @@ struct LinkSmem {
 struct ProgSmem {
   GeneSmem gene[GRN_MAX_GENES];      // in the order the splits take them
   LinkSmem link[GRN_MAX_LINKS + 1];  // the slot after the last is read ahead
+  int start[33];  // walked items: each warp's first (chunk * 16 + gene entry)
+  int pad[3];
 };
 static_assert(sizeof(GeneSmem) == 32 && sizeof(LinkSmem) == 32, "program words");
 
@@ -211,10 +213,10 @@ constexpr size_t kProgOffset = sizeof(ModelSmem);
 constexpr size_t kRedOffset = kProgOffset + sizeof(ProgSmem);  // float [2][32]
 constexpr size_t kDredOffset = kRedOffset + 2 * 32 * 4;  // double [32]
 constexpr size_t kWorkOffset = kDredOffset + 32 * 8;     // int [2]
-// Cluster exchange slots: per-CTA step maxima float [2][kMaxCluster] (by
-// step parity) and per-CTA fitness sums double [kMaxCluster].
+// Cluster exchange slots: step maxima float [2][kMaxCluster][32] (by step
+// parity, CTA and warp) and per-CTA fitness sums double [kMaxCluster].
 constexpr size_t kCmaxOffset = kWorkOffset + 16;
-constexpr size_t kCsumOffset = kCmaxOffset + 2 * kMaxCluster * 4;
+constexpr size_t kCsumOffset = kCmaxOffset + 2 * kMaxCluster * 32 * 4;
 // Two mbarriers of the streaming schedule's copy stages, then its copy
 // time-out flag (int).
 constexpr size_t kMbarOffset = (kCsumOffset + kMaxCluster * 8 + 15) & ~size_t(15);
@@ -332,12 +334,23 @@ __device__ __forceinline__ float comb(float run, float t) {
   else return comb_and(run, t);
 }
 
+// Relative cost of one gene of a strip, in instructions per cell.
+__device__ __forceinline__ int gene_cost(const PackedGene &g) {
+  const int n = g.n_or + g.n_and;
+  return 13 + (n > 0 ? 5 + 5 * n : 0);
+}
+
 // Builds the program of the model in M (all threads; a barrier follows).
-// `splits` is the number of warps that share a chunk's genes: the genes are
-// dealt to them in snake order of their cost, so that the splits' loads
-// differ by little.
+// Owned chunks: `splits` is the number of warps that share a chunk's genes,
+// which are dealt to them in snake order of their cost, so that the splits'
+// loads differ by little.
+// Walked chunks (splits 0): the genes keep their order, and the items
+// (chunk, gene), chunk by chunk, are cut into one range per warp of nearly
+// equal cost, so that a warp changes its strips at most once per G items.
+// Measured on 100 x 100 (G cell-updates/s): 142; warps taking whole chunks
+// in turn, 1, 2 or 4 warps to a chunk, 127.
 __device__ __forceinline__ void build_program(const ModelSmem &M, ProgSmem &P, int splits,
-                                              int tid) {
+                                              int chunks, int n_warps, int tid) {
   const int G = M.hdr.n_genes;
   for (int l = tid; l < M.hdr.n_links; l += blockDim.x) {
     const PackedLink lk = M.links[l];
@@ -345,22 +358,46 @@ __device__ __forceinline__ void build_program(const ModelSmem &M, ProgSmem &P, i
     P.link[l].slot = lk.slot;
   }
   if (tid == 0) P.link[M.hdr.n_links].slot = 0;
+  if (splits == 0 && tid <= n_warps) {
+    int total = 0;
+    for (int q = 0; q < G; ++q) total += gene_cost(M.genes[q]);
+    // The first item whose middle lies at or past tid / n_warps of the cost.
+    const int64_t goal2 = 2 * (int64_t)total * chunks * tid;
+    int64_t chunk = goal2 / (2 * (int64_t)total * n_warps);
+    int64_t at = chunk * total;
+    int k = 0;
+    while (k < G) {
+      const int c = gene_cost(M.genes[k]);
+      if ((2 * at + c) * n_warps >= goal2) break;
+      at += c;
+      ++k;
+    }
+    if (k == G) {
+      k = 0;
+      ++chunk;
+    }
+    P.start[tid] = (int)chunk * 16 + k;
+  }
   if (tid >= G) return;
   const PackedGene g = M.genes[tid];
-  const int n = g.n_or + g.n_and;
-  // Rank by cost (links, then index), then the snake deal: round r of the
-  // splits runs backwards in odd full rounds.
-  int rank = 0;
-  for (int q = 0; q < G; ++q) {
-    const int nq = M.genes[q].n_or + M.genes[q].n_and;
-    rank += (nq > n || (nq == n && q < tid)) ? 1 : 0;
+  int place = tid;
+  if (splits > 0) {
+    // Rank by cost (then index), then the snake deal: round r of the splits
+    // runs backwards in odd full rounds.
+    const int cost = gene_cost(g);
+    int rank = 0;
+    for (int q = 0; q < G; ++q) {
+      const int cq = gene_cost(M.genes[q]);
+      rank += (cq > cost || (cq == cost && q < tid)) ? 1 : 0;
+    }
+    const int round = rank / splits, pos = rank - round * splits;
+    const bool back = (round & 1) && (round + 1) * splits <= G;
+    place = round * splits + (back ? splits - 1 - pos : pos);
   }
-  const int round = rank / splits, pos = rank - round * splits;
-  const bool back = (round & 1) && (round + 1) * splits <= G;
-  GeneSmem &o = P.gene[round * splits + (back ? splits - 1 - pos : pos)];
+  GeneSmem &o = P.gene[place];
   o.ld = make_float4(g.lim, g.lim, -g.deg, -g.deg);
   o.dif = f2(g.dif);
-  o.ctl = gene_ctl(tid, g.dif > 0.0f, g.link_begin, g.n_or, n);
+  o.ctl = gene_ctl(tid, g.dif > 0.0f, g.link_begin, g.n_or, g.n_or + g.n_and);
 }
 
 // ---- geometry ----------------------------------------------------------
@@ -407,6 +444,8 @@ struct Strip {
   bool el, er;         // the left / right neighbour group is not the
                        // neighbouring lane's
   bool m1, m2, m3;     // cells 1..3 of the group exist (cell 0 always does)
+  bool first, last;    // holds the band's first row / its last one, and a
+                       // neighbouring CTA has that row as a halo row
   float2 nt[R][2];     // -(existing neighbours) of each cell, as pairs
 };
 
@@ -422,6 +461,8 @@ __device__ __forceinline__ Strip<R> strip_at(int q, const Geom &g) {
   s.el = gx == 0 || (q & 31) == 0;
   s.er = gx == g.Wg - 1 || (q & 31) == 31;
   s.base = 4 * ((y + 1) * g.RS + x0);
+  s.first = s.valid && y == 0 && g.y0 > 0;
+  s.last = s.valid && y + R >= g.H && g.y0 + g.H < g.Hg;
   const int yg = y + g.y0;
   const float hx = (x0 > 0 ? 1.0f : 0.0f) + (x0 + 1 < g.W ? 1.0f : 0.0f);
   const float hy = 1.0f + (x0 + 2 < g.W ? 1.0f : 0.0f);
@@ -445,8 +486,9 @@ __device__ __forceinline__ int cell_offset(const Geom &g, int y, int x) {
 
 // ---- the step ------------------------------------------------------------
 //
-// Work is cut into warp items: a chunk of 32 strips, for every splits-th
-// gene.  A thread evaluates one gene after the other for its 8 cells; the
+// Work is cut into warp items: one gene of a chunk of 32 strips.  A warp owns
+// a chunk and its part of the genes, or walks a range of (chunk, gene) items
+// (build_program).  A thread evaluates one gene after the other for its 8 cells; the
 // regulators' values are read again, and their lg2 taken again, for every
 // link that reads them.  That is more MUFU work than holding every gene's
 // lg2 in registers (one lg2 per link instead of one per gene), but it needs
@@ -502,6 +544,34 @@ struct Planes {
   size_t out_stride;
   int n_sm;
 };
+
+// Where a band's edge rows also go: the halo rows of the neighbouring CTAs'
+// planes, `rows` bytes further down (up) than the row's own place, in their
+// shared memory (cluster addresses of their state areas) or their global
+// slots (slot_bytes before and after this CTA's).
+struct Halo {
+  uint32_t up, down;
+  int rows;
+  int64_t slot_bytes;
+};
+
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+  return a;
+}
+
+template <bool GL>
+__device__ __forceinline__ void halo_store(uint32_t remote, char *gl, int off, const float4 &v) {
+  if constexpr (GL) {
+    *reinterpret_cast<float4 *>(chk<4>(reinterpret_cast<float *>(gl + off))) = v;
+  } else {
+    (void)state_at<4, false>(nullptr, off);  // the same offset in this CTA, checked
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote + off),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+  }
+}
 
 // The terms a*lg2(x) + b of one link for the strip's cells.
 template <int R, bool SPILL>
@@ -612,11 +682,12 @@ __device__ __forceinline__ void regulation(const ProgSmem &P, int ctl, const Pla
 // reference's diffusion guard only ever skips adding dif*0, a zero rate
 // gives c + dt*0 = c, and the clamp is a max with 0, so these simplify
 // without changing any result.
-template <int R, bool EXACT, bool RAGGED, bool DIFFUSES, bool SG, bool DG>
+template <int R, bool EXACT, bool RAGGED, bool DIFFUSES, bool SG, bool DG, bool CL>
 __device__ __forceinline__ void update_strip(const GeneSmem &gn, const float4 (&h)[R],
                                              const char *src_gl, int src, char *dst_gl, int dst,
-                                             const Strip<R> &st, const Geom &g, float dt,
-                                             float min_conc, float &mx) {
+                                             const Strip<R> &st, const Geom &g,
+                                             const Halo &halo, float dt, float min_conc,
+                                             float &mx) {
   const float4 ld = gn.ld;
   const float2 dif = DIFFUSES ? gn.dif : f2(0.0f);
   const int o = src + st.base;
@@ -688,10 +759,16 @@ __device__ __forceinline__ void update_strip(const GeneSmem &gn, const float4 (&
       if (!st.m2) { nv.z = 0.0f; m2 = 0.0f; }
       if (!st.m3) { nv.w = 0.0f; m3 = 0.0f; }
     }
+    const int row = dst + st.base + i * g.RSb;
     if (st.valid && (i == 0 || i < st.rows)) {
       mx = fmaxf(fmaxf(mx, m), fmaxf(fmaxf(m1, m2), m3));
-        *reinterpret_cast<float4 *>(const_cast<float *>(
-            state_at<4, DG>(dst_gl, dst + st.base + i * g.RSb))) = nv;
+      *reinterpret_cast<float4 *>(const_cast<float *>(state_at<4, DG>(dst_gl, row))) = nv;
+    }
+    if constexpr (CL) {
+      if (i == 0 && st.first)
+        halo_store<DG>(halo.up, dst_gl - halo.slot_bytes, row + halo.rows, nv);
+      if (i == st.rows - 1 && st.last)
+        halo_store<DG>(halo.down, dst_gl + halo.slot_bytes, row - halo.rows, nv);
     }
   }
 }
@@ -699,10 +776,10 @@ __device__ __forceinline__ void update_strip(const GeneSmem &gn, const float4 (&
 // One gene (entry k of the program) for the strip.  SPILL: genes n_sm and on
 // live in the global slot.  BAND: the source planes are a staged band in
 // shared memory, the destination is global.
-template <int R, bool EXACT, bool RAGGED, bool SPILL, bool BAND>
+template <int R, bool EXACT, bool RAGGED, bool SPILL, bool BAND, bool CL>
 __device__ __forceinline__ void gene_step(const ProgSmem &P, int k, const Planes &pl,
-                                          const Strip<R> &st, const Geom &g, float dt,
-                                          float min_conc, float &mx) {
+                                          const Strip<R> &st, const Geom &g, const Halo &halo,
+                                          float dt, float min_conc, float &mx) {
   const GeneSmem &gn = P.gene[k];
   const int ctl = uniform(gn.ctl);
   const int p = ctl & 15;
@@ -712,12 +789,12 @@ __device__ __forceinline__ void gene_step(const ProgSmem &P, int k, const Planes
     constexpr bool D = decltype(diffuses)::value;
     char *const out = pl.gl_out + p * pl.out_stride;
     if (SPILL && p >= pl.n_sm)
-      update_strip<R, EXACT, RAGGED, D, true, true>(gn, h, pl.gl + (size_t)p * g.PSb, 0, out, 0,
-                                                    st, g, dt, min_conc, mx);
+      update_strip<R, EXACT, RAGGED, D, true, true, CL>(
+          gn, h, pl.gl + (size_t)p * g.PSb, 0, out, 0, st, g, halo, dt, min_conc, mx);
     else
-      update_strip<R, EXACT, RAGGED, D, false, BAND>(gn, h, nullptr, pl.sm + p * g.PSb, out,
-                                                     BAND ? 0 : pl.sm_out + p * g.PSb, st, g, dt,
-                                                     min_conc, mx);
+      update_strip<R, EXACT, RAGGED, D, false, BAND, CL>(
+          gn, h, nullptr, pl.sm + p * g.PSb, out, BAND ? 0 : pl.sm_out + p * g.PSb, st, g, halo, dt,
+          min_conc, mx);
   };
   if (ctl & 16) update(True{});
   else update(False{});
@@ -784,52 +861,66 @@ __device__ __forceinline__ float *plane_of(const StatePtrs &sp, const Geom &g, i
                      : sp.gl + (p + (par ? sp.gmax : 0)) * g.PS;
 }
 
-// Genes first, first + splits, .. of the program for one strip.
-template <int R, bool EXACT, bool RAGGED, bool SPILL>
-__device__ __forceinline__ void strip_step(const ProgSmem &P, const StatePtrs &sp, int G,
-                                           const Geom &g, const Strip<R> &st, int first,
-                                           int splits, int par, float dt, float min_conc,
-                                           float &mx) {
+// The planes of a step from buffer `par` to the other one.
+__device__ __forceinline__ Planes planes_of(const StatePtrs &sp, const Geom &g, int par) {
   const int half = sp.n_sm * g.PSb;
   const size_t gl_half = (size_t)sp.gmax * g.PSb;
   char *gl = reinterpret_cast<char *>(sp.gl);
-  const Planes pl{opaque(par ? half : 0), opaque(par ? 0 : half), gl + (par ? gl_half : 0),
-                  gl + (par ? 0 : gl_half), (size_t)g.PSb,  sp.n_sm};
+  return Planes{opaque(par ? half : 0),   opaque(par ? 0 : half), gl + (par ? gl_half : 0),
+                gl + (par ? 0 : gl_half), (size_t)g.PSb,          sp.n_sm};
+}
+
+// Genes first, first + splits, .. of the program for one strip.
+template <int R, bool EXACT, bool RAGGED, bool SPILL, bool CL>
+__device__ __forceinline__ void strip_step(const ProgSmem &P, const Planes &pl, int G,
+                                           const Geom &g, const Strip<R> &st, const Halo &halo,
+                                           int first, int splits, float dt, float min_conc,
+                                           float &mx) {
 #pragma unroll 1
   for (int k = first; k < G; k += splits)
-    gene_step<R, EXACT, RAGGED, SPILL, false>(P, k, pl, st, g, dt, min_conc, mx);
+    gene_step<R, EXACT, RAGGED, SPILL, false, CL>(P, k, pl, st, g, halo, dt, min_conc, mx);
 }
 
-// The same by the model's class: all planes in shared memory or some in the
-// global slot; the exact path always takes the general form.
-template <int R, bool RAGGED>
-__device__ __forceinline__ void strip_step_any(bool exact, const ProgSmem &P, const StatePtrs &sp,
-                                               int G, const Geom &g, const Strip<R> &st, int first,
-                                               int splits, int par, float dt, float min_conc,
-                                               float &mx) {
-  if (exact)
-    strip_step<R, true, RAGGED, true>(P, sp, G, g, st, first, splits, par, dt, min_conc, mx);
-  else if (sp.n_sm < G)
-    strip_step<R, false, RAGGED, true>(P, sp, G, g, st, first, splits, par, dt, min_conc, mx);
-  else
-    strip_step<R, false, RAGGED, false>(P, sp, G, g, st, first, splits, par, dt, min_conc, mx);
-}
-
-// Warps that share a chunk's genes when `chunks` chunks are walked by
-// n_warps warps: the power of two (at most 4) with the shortest longest
-// warp, counted in gene evaluations (an item costs about a quarter of one).
-__device__ __forceinline__ int choose_splits(int chunks, int n_warps, int G) {
-  int best = 1, cost = 0x7fffffff;
-  for (int s = 1; s <= 4; s *= 2) {
-    if (s > G) break;
-    const int rounds = (chunks * s + n_warps - 1) / n_warps;
-    const int c = rounds * (4 * ((G + s - 1) / s) + 1);
-    if (c < cost) {
-      cost = c;
-      best = s;
-    }
+// A warp's range of walked items, of the first `chunks` chunks.
+template <int R, bool EXACT, bool RAGGED, bool SPILL, bool BAND, bool CL>
+__device__ __forceinline__ void walk_step(const ProgSmem &P, const Planes &pl, int G,
+                                          const Geom &g, const Halo &halo, int chunks, int warp,
+                                          int lane, float dt, float min_conc, float &mx) {
+  const int end = uniform(P.start[warp + 1]);
+  int at = uniform(P.start[warp]);
+#pragma unroll 1
+  while (at < end && (at >> 4) < chunks) {
+    const int chunk = at >> 4;
+    const Strip<R> st = strip_at<R>(chunk * 32 + lane, g);
+    const int stop = (end >> 4) == chunk ? end & 15 : G;
+#pragma unroll 1
+    for (int k = at & 15; k < stop; ++k)
+      gene_step<R, EXACT, RAGGED, SPILL, BAND, CL>(P, k, pl, st, g, halo, dt, min_conc, mx);
+    at = (chunk + 1) << 4;
   }
-  return best;
+}
+
+// One step of the whole block by the model's class: all planes in shared
+// memory or some in the global slot; the exact path always takes the general
+// form.
+template <int R, bool LOOP, bool RAGGED, bool CL>
+__device__ __forceinline__ void block_step(bool exact, const ProgSmem &P, const StatePtrs &sp,
+                                           int G, const Geom &g, const Strip<R> &st,
+                                           const Halo &halo, int first, int splits, int chunks,
+                                           int warp, int lane, int par, float dt, float min_conc,
+                                           float &mx) {
+  const Planes pl = planes_of(sp, g, par);
+  const auto run = [&](auto e, auto spill) {
+    constexpr bool E = decltype(e)::value, S = decltype(spill)::value;
+    if constexpr (LOOP)
+      walk_step<R, E, RAGGED, S, false, CL>(P, pl, G, g, halo, chunks, warp, lane, dt, min_conc,
+                                            mx);
+    else
+      strip_step<R, E, RAGGED, S, CL>(P, pl, G, g, st, halo, first, splits, dt, min_conc, mx);
+  };
+  if (exact) run(True{}, True{});
+  else if (sp.n_sm < G) run(False{}, True{});
+  else run(False{}, False{});
 }
 
 // ---- streaming schedule -------------------------------------------------
@@ -847,33 +938,21 @@ __device__ __forceinline__ int choose_splits(int chunks, int n_warps, int G) {
 // floats), written to the global next-state planes: the warps walk the
 // band's items.  `out` addresses the band's cells as a plane does: cell (x,
 // local row y) of gene p at out + p * gps + (y + 1) * RS + x.
-template <int R, bool EXACT, bool RAGGED>
-__device__ __forceinline__ void band_step(const ProgSmem &P, const float *stage, int G,
-                                          const Geom &gb, float *out, size_t gps, int splits,
+template <int R, bool RAGGED>
+__device__ __forceinline__ void band_step(bool exact, const ProgSmem &P, const float *stage,
+                                          int G, const Geom &gb, float *out, size_t gps,
                                           float dt, float min_conc, float &mx) {
-  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
-  const int items = ((gb.Q + 31) / 32) * splits;
-  const int shift = 31 - __clz(splits);
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const Planes pl{(int)(reinterpret_cast<const unsigned char *>(stage) - grn_dyn_smem) -
                       (int)kStateOffset,
                   0, nullptr, reinterpret_cast<char *>(out), gps * sizeof(float), G};
-#pragma unroll 1
-  for (int i = warp; i < items; i += n_warps) {
-    const Strip<R> st = strip_at<R>((i >> shift) * 32 + lane, gb);
-#pragma unroll 1
-    for (int k = i & (splits - 1); k < G; k += splits)
-      gene_step<R, EXACT, RAGGED, false, true>(P, k, pl, st, gb, dt, min_conc, mx);
-  }
-}
-
-template <int R, bool RAGGED>
-__device__ __forceinline__ void band_step_any(bool exact, const ProgSmem &P, const float *stage,
-                                              int G, const Geom &gb, float *out, size_t gps,
-                                              int splits, float dt, float min_conc, float &mx) {
+  const int chunks = (gb.Q + 31) / 32;
   if (exact)
-    band_step<R, true, RAGGED>(P, stage, G, gb, out, gps, splits, dt, min_conc, mx);
+    walk_step<R, true, RAGGED, false, true, false>(P, pl, G, gb, Halo{}, chunks, warp, lane, dt,
+                                                   min_conc, mx);
   else
-    band_step<R, false, RAGGED>(P, stage, G, gb, out, gps, splits, dt, min_conc, mx);
+    walk_step<R, false, RAGGED, false, true, false>(P, pl, G, gb, Halo{}, chunks, warp, lane, dt,
+                                                    min_conc, mx);
 }
 
 // One Euler step of the streaming schedule.  Stages alternate by band; the
@@ -887,7 +966,7 @@ __device__ __forceinline__ void band_step_any(bool exact, const ProgSmem &P, con
 // on entry and is never cleared: the kernel returns after a failure.
 template <bool RAGGED>
 __device__ bool stream_step(const SimArgs &A, const ProgSmem &P, const StatePtrs &sp,
-                            const Geom &g, int G, int splits, int par, bool exact,
+                            const Geom &g, int G, int par, bool exact,
                             float dt, float min_conc, float &mx, uint64_t *bars,
                             uint32_t &mphase, volatile int *fail, int R) {
   const int nb = (g.H + R - 1) / R;
@@ -925,8 +1004,8 @@ __device__ bool stream_step(const SimArgs &A, const ProgSmem &P, const StatePtrs
     gb.PS = SPS;
     gb.PSb = 4 * SPS;
     gb.Q = strip_count<kStripRows>(gb.H, g.Wg);
-    band_step_any<kStripRows, RAGGED>(exact, P, stage0 + s * sp.gmax * SPS, G, gb,
-                          gl_nxt + (size_t)gb.y0 * g.RS, gps, splits, dt, min_conc, mx);
+    band_step<kStripRows, RAGGED>(exact, P, stage0 + s * sp.gmax * SPS, G, gb,
+                          gl_nxt + (size_t)gb.y0 * g.RS, gps, dt, min_conc, mx);
     __syncthreads();  // stage s is free again; *fail is the same for every thread
     if (*fail) {
       // Bounded second waits for copies that may still be in flight: the
@@ -966,7 +1045,7 @@ __device__ bool stream_step(const SimArgs &A, const ProgSmem &P, const StatePtrs
 // time, after a bounded wait for the copy still in flight.
 template <bool RAGGED>
 __device__ bool stream_step2(const SimArgs &A, const ProgSmem &P, const StatePtrs &sp,
-                             const Geom &g, int G, int splits, int par, bool exact,
+                             const Geom &g, int G, int par, bool exact,
                              float dt, float min_conc, float &mx1, float &mx2, uint64_t *bars,
                              uint32_t &mphase, volatile int *fail) {
   const int R = A.band_rows;
@@ -1008,7 +1087,7 @@ __device__ bool stream_step2(const SimArgs &A, const ProgSmem &P, const StatePtr
     // Stage row of grid row y is y - bR + 2; g1's row 0 is grid row y1 - 1.
     const float *st1 = stage + (y1 - b * R + 1) * g.RS;
     float *out1 = inter + (y1 - b * R) * g.RS;  // cell rows land at y - (bR - 1)
-    band_step_any<kStripRows, RAGGED>(exact, P, st1, G, g1, out1, (size_t)IPS, splits, dt, min_conc, mx1);
+    band_step<kStripRows, RAGGED>(exact, P, st1, G, g1, out1, (size_t)IPS, dt, min_conc, mx1);
     // Intermediate rows outside the grid are the planes' zero rows.
     const int zlo = (b == 0) ? 0 : -1;                            // grid row -1
     const int zhi = (b * R + R >= g.H) ? g.H - (b * R - 1) : -1;  // grid row H
@@ -1032,7 +1111,7 @@ __device__ bool stream_step2(const SimArgs &A, const ProgSmem &P, const StatePtr
     g2.PS = IPS;
     g2.PSb = 4 * IPS;
     g2.Q = strip_count<kStripRows>(g2.H, g.Wg);
-    band_step_any<kStripRows, RAGGED>(exact, P, inter, G, g2, gl_nxt + (size_t)g2.y0 * g.RS, gps, splits, dt,
+    band_step<kStripRows, RAGGED>(exact, P, inter, G, g2, gl_nxt + (size_t)g2.y0 * g.RS, gps, dt,
                           min_conc, mx2);
     __syncthreads();  // the intermediate is free again
   }
@@ -1040,30 +1119,10 @@ __device__ bool stream_step2(const SimArgs &A, const ProgSmem &P, const StatePtr
   return true;
 }
 
-// Pushes the edge rows of the new buffer (`nxt`) of every gene into the
-// neighbouring bands' halo rows: the first row to the band above (its row
-// Hb + 1), the last row to the band below (its row 0).  Shared-memory planes
-// are reached through the cluster's distributed shared memory, global slots
-// directly (a cluster's CTAs are consecutive blocks).
-__device__ __forceinline__ void push_halos(const SimArgs &A, const StatePtrs &sp, const Geom &g,
-                                           int G, int nxt, int rank, int C, int Hb) {
-  cg::cluster_group cl = cg::this_cluster();
-  const int n4 = g.RS / 4;
-  for (int i = threadIdx.x; i < G * 2 * n4; i += blockDim.x) {
-    const int p = i / (2 * n4), rem = i - p * 2 * n4;
-    const int dir = rem / n4, c = rem - dir * n4;
-    const int dst = dir == 0 ? rank - 1 : rank + 1;
-    if (dst < 0 || dst >= C) continue;
-    float *pl = plane_of(sp, g, p, nxt);
-    const float4 v =
-        *reinterpret_cast<const float4 *>(chk<4>(pl + (dir == 0 ? 1 : g.H) * g.RS + 4 * c));
-    const int off = (dir == 0 ? Hb + 1 : 0) * g.RS + 4 * c;
-    float *dpl = p < sp.n_sm
-                     ? cl.map_shared_rank(chk<4>(pl + off), (unsigned)dst)  // checked locally
-                     : chk<4>(A.gstate + (size_t)(blockIdx.x - rank + dst) * (size_t)A.slot_floats +
-                              (pl - sp.gl) + off);
-    *reinterpret_cast<float4 *>(dpl) = v;
-  }
+// Sets n floats (whole float4 words) to 0, all threads of the block.
+__device__ __forceinline__ void zero_floats(float *p, int n) {
+  for (int i = threadIdx.x; i < n / 4; i += blockDim.x)
+    *reinterpret_cast<float4 *>(chk<4>(p + 4 * (size_t)i)) = f4(0.0f);
 }
 
 // Copies the first min(G, A.state_planes) genes' current values of the
@@ -1080,13 +1139,30 @@ __device__ __forceinline__ void write_planes(const SimArgs &A, const StatePtrs &
 }
 
 // Cluster-wide combine of one value per CTA: CTA `rank` stores v into slot
-// `rank` of every CTA's array, then the cluster barrier (which also orders
-// the halo rows pushed before it).  Every CTA then reads the same C slots.
+// `rank` of every CTA's array, then the cluster barrier.  Every CTA then
+// reads the same C slots.
 template <typename T>
 __device__ __forceinline__ void cluster_share(T *slots, T v, int rank, int C) {
   cg::cluster_group cl = cg::this_cluster();
   if ((int)threadIdx.x < C) *cl.map_shared_rank(slots + rank, threadIdx.x) = v;
   cl.sync();
+}
+
+// Max of a non-negative, non-NaN float over the cluster's CTAs with one
+// cluster barrier: every warp stores its max into slot [rank][warp] of every
+// CTA's array.  The barrier also orders the step's halo rows.
+__device__ __forceinline__ float cluster_max(float v, float *slots, int rank, int C, int lane,
+                                             int warp, int n_warps) {
+  const unsigned bits = __reduce_max_sync(kFull, __float_as_uint(v));
+  if (lane < C) {
+    const uint32_t a = cluster_addr(smem_addr(slots + rank * 32 + warp), lane);
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(bits) : "memory");
+  }
+  cg::this_cluster().sync();
+  unsigned mine = 0u;
+  if (lane < n_warps)
+    for (int r = 0; r < C; ++r) mine = max(mine, __float_as_uint(slots[r * 32 + lane]));
+  return __uint_as_float(__reduce_max_sync(kFull, mine));
 }
 
 // The simulation kernel.  A.threads threads per block (whole warps).
@@ -1173,16 +1249,28 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
     __syncthreads();
   }
 
+  Halo halo{};
+  if constexpr (CL) {
+    const uint32_t state = smem_addr(smem + kStateOffset);
+    if (rank > 0) halo.up = cluster_addr(state, rank - 1);
+    if (rank < C - 1) halo.down = cluster_addr(state, rank + 1);
+    halo.rows = Hb * g.RSb;
+    halo.slot_bytes = A.slot_floats * (int64_t)sizeof(float);
+  }
+
   // Chunks of a full band: the same in every CTA of a cluster.
-  const int chunks = (strip_count<kStripRows>(ST ? min(Hb, A.band_rows) : Hb, g.Wg) + 31) / 32;
+  // (Streaming: of a full band; of a two-step pass's first step, whose last
+  // chunks the second step does not have.)
+  const int rows = ST ? min(Hb, A.band_rows + (ST == 2 ? 2 : 0)) : Hb;
+  const int chunks = (strip_count<kStripRows>(rows, g.Wg) + 31) / 32;
   // Fixed items: geometry once per launch.
   Strip<kStripRows> fixed;
   int fixed_part = 0;
-  const int fixed_splits = LOOP ? 1 : max(1, n_warps / chunks);
+  const int splits = LOOP ? 0 : max(1, n_warps / chunks);
   if constexpr (!LOOP) {
     fixed = strip_at<kStripRows>((warp % chunks) * 32 + lane, g);
     fixed_part = warp / chunks;
-    if (fixed_part >= fixed_splits) fixed_part = GRN_MAX_GENES;  // no work
+    if (fixed_part >= splits) fixed_part = GRN_MAX_GENES;  // no work
   }
 
   for (int iter = 0;; ++iter) {
@@ -1241,8 +1329,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
       continue;
     }
 
-    const int splits = LOOP ? choose_splits(chunks, n_warps, G) : fixed_splits;
-    build_program(M, P, splits, tid);
+    build_program(M, P, splits, chunks, n_warps, tid);
     __syncthreads();
 
     double error = 0.0, change_sum = 0.0;
@@ -1250,21 +1337,29 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
     const double max_err = A.max_error[orig];
 
     for (int e = 0; e < A.n_exp && error <= max_err; ++e) {
-      // Initial state, both buffers of every gene: input morphogen planes
-      // from the experiment, the other products 0 (simstate.cpp:64-90);
-      // zero rows and padding cells 0.
-      // A band's halo rows start as the neighbouring grid rows.
+      // Initial state: every plane of both buffers 0, then buffer 0 of the
+      // input morphogens from the experiment (simstate.cpp:64-90); the other
+      // buffer's cells are all written by the first step.  A band's halo rows
+      // start as the neighbouring grid rows.
       const float *init = A.initial + (size_t)e * A.n_in * A.W * A.H;
-      for (int i = tid; i < 2 * G * g.PS; i += NT) {
-        const int kb = i / g.PS, r = i - kb * g.PS;
-        const int kk = kb < G ? kb : kb - G;  // gene of this plane
-        const int rr = r / g.RS, x = r - rr * g.RS;
-        const int y = g.y0 - 1 + rr;  // grid row
-        float v = 0.0f;
-        if (kk < A.n_in && y >= 0 && y < g.Hg && x < g.W)
-          v = init[((size_t)kk * g.Hg + y) * g.W + x];
-        float *pl = plane_of(sp, g, kk, kb < G ? 0 : 1);
-        *chk<1>(pl + r) = v;
+      zero_floats(sp.sm, 2 * sp.n_sm * g.PS);
+      if (sp.n_sm < G) {
+        zero_floats(sp.gl + (size_t)sp.n_sm * g.PS, (G - sp.n_sm) * g.PS);
+        zero_floats(sp.gl + (size_t)(sp.gmax + sp.n_sm) * g.PS, (G - sp.n_sm) * g.PS);
+      }
+      __syncthreads();
+      for (int kk = 0; kk < min(A.n_in, G); ++kk) {
+        float *pl = plane_of(sp, g, kk, 0);
+        for (int i = tid; i < (g.H + 2) * g.Wg; i += NT) {
+          const int rr = g.Wg == 1 ? i : (int)__umulhi((uint32_t)i, g.inv_wg);
+          const int x0 = 4 * (i - rr * g.Wg), y = g.y0 - 1 + rr;  // grid row
+          if (y < 0 || y >= g.Hg) continue;
+          const float *src = init + ((size_t)kk * g.Hg + y) * g.W + x0;
+          float *dst = chk<4>(pl + rr * g.RS + x0);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (x0 + j < g.W) dst[j] = src[j];
+        }
       }
       if constexpr (ST == 2) {
         // The two-step pass's intermediate buffer: its rows' trailing zero
@@ -1303,7 +1398,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
           bool ok = true, single = true;
           if (ST == 2 && step + 2 <= A.n_steps) {
             float mx2 = 0.0f;
-            ok = stream_step2<RAGGED>(A, P, sp, g, G, splits, par, exact, dt, min_conc, mx, mx2,
+            ok = stream_step2<RAGGED>(A, P, sp, g, G, par, exact, dt, min_conc, mx, mx2,
                                           bars, mphase, s_stream_fail);
             if (ok) {
               const float b1 = block_max(mx, s_red, par ^ 1, lane, warp, n_warps);
@@ -1313,7 +1408,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
             }
           }
           if (ok && single)
-            ok = stream_step<RAGGED>(A, P, sp, g, G, splits, par, exact, dt, min_conc, mx, bars,
+            ok = stream_step<RAGGED>(A, P, sp, g, G, par, exact, dt, min_conc, mx, bars,
                                          mphase, s_stream_fail, A.band_rows);
           if (!ok) {
             if (tid == 0) {
@@ -1322,24 +1417,15 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
             }
             return;  // every thread of the block: the decision is block-uniform
           }
-        } else if constexpr (!LOOP) {
-          strip_step_any<kStripRows, RAGGED>(exact, P, sp, G, g, fixed, fixed_part, splits, par, dt,
-                                     min_conc, mx);
         } else {
-          const int shift = 31 - __clz(splits), items = chunks * splits;
-          for (int i = warp; i < items; i += n_warps) {
-            const Strip<kStripRows> st = strip_at<kStripRows>((i >> shift) * 32 + lane, g);
-            strip_step_any<kStripRows, RAGGED>(exact, P, sp, G, g, st, i & (splits - 1), splits, par, dt,
-                                       min_conc, mx);
-          }
+          block_step<kStripRows, LOOP, RAGGED, CL>(exact, P, sp, G, g, fixed, halo, fixed_part,
+                                                   splits, chunks, warp, lane, par, dt, min_conc,
+                                                   mx);
         }
-        change = block_max(mx, s_red, par, lane, warp, n_warps);
-        if constexpr (CL) {
-          push_halos(A, sp, g, G, par ^ 1, rank, C, Hb);
-          cluster_share(s_cmax + par * kMaxCluster, change, rank, C);
-          change = 0.0f;
-          for (int r = 0; r < C; ++r) change = fmaxf(change, s_cmax[par * kMaxCluster + r]);
-        }
+        if constexpr (CL)  // also orders the halo rows stored by this step
+          change = cluster_max(mx, s_cmax + par * kMaxCluster * 32, rank, C, lane, warp, n_warps);
+        else
+          change = block_max(mx, s_red, par, lane, warp, n_warps);
         par ^= 1;
         step += adv;
         if constexpr (TRACE) {
@@ -1358,7 +1444,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
       // Fitness of the experiment (simstate.cpp:135-158), FP64 sums.
       const float *tgt = A.target + (size_t)e * A.n_target * A.W * A.H;
       const auto term = [&](int i, double acc) {
-        const int y = i / g.W, x = i - y * g.W;
+        const int y = A.inv_w ? (int)__umulhi((uint32_t)i, A.inv_w) : i / g.W, x = i - y * g.W;
         for (int kk = 0; kk < A.n_target; ++kk) {
           const double a = *chk<1>(plane_of(sp, g, A.n_in + kk, par) + cell_offset(g, y, x));
           const double b = tgt[((size_t)kk * g.Hg + g.y0 + y) * g.W + x];
@@ -1411,11 +1497,11 @@ const VariantEntry kVariants[] = {
     GRN_VARIANT(512, false, false, false, 0), GRN_VARIANT(512, true, false, false, 0),
     GRN_VARIANT(1024, false, false, false, 0), GRN_VARIANT(1024, true, false, false, 0),
     // cluster-split
-    GRN_VARIANT(512, true, true, false, 0),
+    GRN_VARIANT(1024, false, true, false, 0), GRN_VARIANT(1024, true, true, false, 0),
     // trace frames (one model at a time: any grid, any gene count)
     GRN_VARIANT(512, true, false, true, 0),
     // streaming (bands staged by bulk copies)
-    GRN_VARIANT(512, true, false, false, 1), GRN_VARIANT(1024, true, false, false, 1),
+    GRN_VARIANT(512, true, false, false, 1),
     // streaming with temporal blocking: two Euler steps per pass
     GRN_VARIANT(512, true, false, false, 2),
 };

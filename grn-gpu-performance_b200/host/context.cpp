@@ -228,14 +228,29 @@ int host_threads(const grn_ctx *ctx) {
 // band may read, must fit the shared memory left over, and one stage's bytes
 // must stay below the mbarrier transaction limit (2^20); an even count, since
 // a thread computes two rows.
-int stream_rows(int W, int H, int genes, size_t room) {
+int stream_rows(int W, int H, int genes, size_t room, int threads) {
   const size_t row_bytes = (size_t)grn::row_floats(W) * sizeof(float);
   long r = (long)((room - std::min(room, row_bytes)) / (2 * genes * row_bytes)) - 2;
   r = std::min<long>(r, H);
   while (r > 1 && (size_t)genes * (r + 2) * row_bytes >= (size_t)1 << 20) --r;
   if (r < 1) return 0;
   if (r > 1 && r < H) r &= ~1L;
-  return (int)r;
+  // Of the counts that fit, the one whose items (chunks x genes) leave the
+  // least of the block's warps idle in the last round; a band also costs a
+  // barrier and two halo rows, about half a row's work.
+  const int warps = threads / 32;
+  long best = r;
+  double best_eff = 0;
+  for (long q = r; q >= 1; q -= q > 2 ? 2 - (q & 1) : 1) {
+    const int chunks = grn::strip_chunks(W, (int)q);
+    const int rounds = (chunks * genes + warps - 1) / warps;
+    const double eff = (double)q / rounds * q / (q + 0.5);
+    if (eff > 1.001 * best_eff) {
+      best_eff = eff;
+      best = q;
+    }
+  }
+  return (int)best;
 }
 
 // Output rows per band of the two-steps-per-pass streaming variant: its
@@ -253,7 +268,45 @@ int stream2_rows(int W, int H, int genes, size_t room) {
   return (int)r;
 }
 
-// Every feasible launch plan for a batch, best heuristic score first.
+// Expected cycles of the batch's steps on a plan, per model step and relative
+// to other plans of the batch: the order in which plans are tried.  Fitted to
+// measurements on B200 (G cell-updates/s at 4 genes and 8 links on average
+// unless noted):
+//   - a gene of a chunk takes about 98 cycles of an SM whose planes are in
+//     shared memory and which holds 28 warps or more; 12 warps take 1.12x, 8
+//     warps 1.46x, 4 warps 1.86x that (32 x 32 grids);
+//   - walked items 1.12x owned chunks, a cluster's chunks 1.15x;
+//   - genes in global slots 1.35x while what the CTAs touch of them stays in
+//     L2 (100 x 100, walked, 2 of 4 genes spilled: 142 against 194), 1.8x
+//     past that (116 x 206: 111); staged bands 1.35x and two steps per pass
+//     1.7x (256 x 256, 8 genes, 24 links: staged 63, walked 43);
+//   - a step's barrier 300 cycles, a cluster's 1200 (2 CTAs) to 6100 (16).
+double plan_cost(const grn_ctx *ctx, const LaunchPlan &p, int max_genes, int n_models,
+                 double slot_bytes) {
+  const int C = std::max(1, p.cluster);
+  const int Hb = (ctx->p.dim_y + C - 1) / C;
+  const int chunks = grn::strip_chunks(ctx->p.dim_x, Hb);
+  const double genes = std::max(1.0, 0.5 * max_genes);  // of an average model
+  const int resident = p.blocks / C;                    // models at a time
+  const double per_sm = std::max(1.0, (double)p.blocks / ctx->n_sm);
+  const double warps = per_sm * std::min<double>(p.threads / 32, chunks * genes);
+  double f = warps >= 12 ? 1.0 + std::max(0.0, 28 - warps) * 0.0075 : 1.12 + (12 - warps) * 0.09;
+  if (p.v.stream) {
+    f *= p.v.stream == 2 ? 1.7 : 1.35;
+  } else {
+    const double spilled = std::max(0.0, 1.0 - p.planes / 2 / genes);
+    const double spilled_max = std::max(0.0, 1.0 - (double)(p.planes / 2) / max_genes);
+    const bool l2 = slot_bytes * genes / max_genes * p.blocks <= 8e7;
+    f *= 1.0 + (l2 ? 0.35 : 0.8) * 0.5 * (spilled + spilled_max);
+    if (C > 1) f *= 1.15;
+    else if (p.v.loop) f *= 1.12;
+  }
+  const double sync = C == 1 ? 300 : 500 + 350 * C;
+  const double step = per_sm * chunks * genes * 98 * f + sync;
+  return step * std::max(1.0, (double)n_models / resident);
+}
+
+// Every feasible launch plan for a batch, lowest expected cost first.
 grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace,
                            std::vector<std::pair<double, LaunchPlan>> *out) {
   const int W = ctx->p.dim_x, H = ctx->p.dim_y;
@@ -264,45 +317,41 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
   const size_t row_bytes = (size_t)grn::row_floats(W) * sizeof(float);
   // A trace runs on the trace variants whatever schedule is forced.
   const int sched = trace ? GRN_SCHEDULE_WALK_ITEMS : ctx->forced_schedule;
+  const int ft = trace ? 0 : ctx->forced_threads;
   static const int kClusterSizes[] = {2, 4, 8, 16};
   out->clear();
   const int nv = grn::sim_variant_count();
   for (int i = 0; i < nv; ++i) {
     const grn::KernelVariant v = grn::sim_variant(i);
     if (max_genes > GRN_MAX_GENES || v.ragged != ragged || v.trace != trace) continue;
+    LaunchPlan plan{};
+    plan.v = v;
+    plan.gmax = max_genes;
     if (v.stream) {
       // Streaming: only where the planes do not all fit shared memory.
       const int own = v.stream == 2 ? GRN_SCHEDULE_STREAM2 : GRN_SCHEDULE_STREAM;
       if (sched != GRN_SCHEDULE_AUTO && sched != own) continue;
-      if (ctx->forced_threads && ctx->forced_threads != v.max_threads) continue;
+      if (ft && ft != v.max_threads) continue;
       const size_t plane_bytes = (size_t)grn::plane_floats(W, H) * sizeof(float);
       const int fit = optin > fixed ? (int)((optin - fixed) / plane_bytes) & ~1 : 0;
       if (sched == GRN_SCHEDULE_AUTO && fit / 2 >= max_genes) continue;
       const size_t room = optin > fixed ? optin - fixed : 0;
       const int R = v.stream == 2 ? stream2_rows(W, H, max_genes, room)
-                                  : stream_rows(W, H, max_genes, room);
+                                  : stream_rows(W, H, max_genes, room, v.max_threads);
       if (R < 1) continue;
       const size_t rows = v.stream == 2 ? (size_t)max_genes * (2 * R + 6)
                                         : (size_t)2 * max_genes * (R + 2);
-      const size_t smem = fixed + (rows + 1) * row_bytes;
-      int per_sm = 0;
-      GRN_CUDA(ctx, grn::sim_occupancy(v, v.max_threads, smem, &per_sm));
-      const int ctas = per_sm * ctx->n_sm;
+      plan.smem_bytes = fixed + (rows + 1) * row_bytes;
+      GRN_CUDA(ctx, grn::sim_occupancy(v, v.max_threads, plan.smem_bytes, &plan.blocks_per_sm));
+      const int ctas = plan.blocks_per_sm * ctx->n_sm;
       if (ctas < 1) continue;
-      LaunchPlan plan{};
-      plan.v = v;
       plan.schedule = own;
       plan.threads = v.max_threads;
-      plan.gmax = max_genes;
-      plan.planes = 0;
-      plan.smem_bytes = smem;
-      plan.blocks_per_sm = per_sm;
       plan.slot_floats = 2LL * max_genes * grn::plane_floats(W, H);
       plan.cluster = 1;
       plan.band_rows = R;
       plan.blocks = std::max(1, std::min(n_models, ctas));
-      const double warps = (double)std::min(ctas, n_models) * v.max_threads / 32;
-      out->push_back({warps * (v.stream == 2 ? 0.4 : 0.6), plan});
+      out->push_back({plan_cost(ctx, plan, max_genes, n_models, 0), plan});
       continue;
     }
     if (sched == GRN_SCHEDULE_STREAM || sched == GRN_SCHEDULE_STREAM2) continue;
@@ -319,75 +368,66 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
       const size_t plane_bytes = (size_t)grn::plane_floats(W, H, C) * sizeof(float);
       int fit = optin > fixed ? (int)((optin - fixed) / plane_bytes) : 0;
       fit &= ~1;
+      const int smem_planes = std::min(fit, 2 * max_genes);
+      if (C > 1 && sched == GRN_SCHEDULE_AUTO) {
+        // A cluster pays where it keeps more genes on chip, or where models
+        // are fewer than SMs.
+        const int fit1 =
+            optin > fixed
+                ? (int)((optin - fixed) / ((size_t)grn::plane_floats(W, H) * sizeof(float))) & ~1
+                : 0;
+        if (fit1 >= 2 * max_genes && 2 * n_models > ctx->n_sm) continue;
+        if (C > 4 && C * n_models > ctx->n_sm) continue;
+      }
       // Under AUTO a walking variant whose genes spill is also offered with
       // every plane in global memory (the L1 then caches more of them).
-      const int smem_planes = std::min(fit, 2 * max_genes);
       const bool offer_global = sched == GRN_SCHEDULE_AUTO && v.loop && C == 1 &&
                                 smem_planes / 2 < max_genes && smem_planes > 0;
       // Block sizes: walking blocks are the variant's largest; fixed ones hold
       // every chunk once, or up to 4 times (a part of the genes each).  A
       // forced size is taken where the variant can run it.
       std::vector<int> sizes;
-      const int ft = trace ? 0 : ctx->forced_threads;
       if (ft) {
-        if (ft % 32 == 0 && ft <= v.max_threads && (v.max_threads == 512 || ft > 512) &&
+        if (ft % 32 == 0 && ft <= v.max_threads && (v.max_threads == 512 || v.cluster || ft > 512) &&
             (v.loop || chunks * 32 <= ft))
           sizes.push_back(ft);
       } else if (v.loop) {
         sizes.push_back(v.max_threads);
       } else {
-        for (int parts = 1; parts <= 4 && parts <= std::max(1, max_genes); ++parts)
-          if (chunks * parts * 32 <= v.max_threads &&
-              (v.max_threads == 512 || chunks * parts * 32 > 512))
-            sizes.push_back(chunks * parts * 32);
+        for (int parts = 1; parts <= 4 && parts <= max_genes; ++parts) {
+          const int threads = chunks * parts * 32;
+          if (threads <= v.max_threads && (v.max_threads == 512 || v.cluster || threads > 512))
+            sizes.push_back(threads);
+        }
       }
       for (const int threads : sizes)
         for (int gv = 0; gv < (offer_global ? 2 : 1); ++gv) {
-          const int planes = (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? 0 : smem_planes;
-          const bool spills = planes / 2 < max_genes;
-          const size_t smem = fixed + planes * plane_bytes;
-          int ctas = 0, per_sm = 0;  // resident CTAs on the device
+          plan.planes = (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? 0 : smem_planes;
+          const bool spills = plan.planes / 2 < max_genes;
+          plan.smem_bytes = fixed + plan.planes * plane_bytes;
+          int ctas = 0;  // resident CTAs on the device
           if (C == 1) {
-            GRN_CUDA(ctx, grn::sim_occupancy(v, threads, smem, &per_sm));
-            ctas = per_sm * ctx->n_sm;
+            GRN_CUDA(ctx, grn::sim_occupancy(v, threads, plan.smem_bytes, &plan.blocks_per_sm));
+            ctas = plan.blocks_per_sm * ctx->n_sm;
           } else {
             int clusters = 0;
-            GRN_CUDA(ctx, grn::sim_cluster_occupancy(v, threads, smem, C, &clusters));
+            GRN_CUDA(ctx, grn::sim_cluster_occupancy(v, threads, plan.smem_bytes, C, &clusters));
             ctas = clusters * C;
-            per_sm = 1;
+            plan.blocks_per_sm = 1;
           }
           if (ctas < 1) continue;
-          // Throughput model: resident warps that have work (no more CTAs
-          // than models need), fixed items ahead of walking ones, and a
-          // penalty for genes kept in global memory -- mild while every
-          // resident CTA's slot fits in L2.
-          const int warps = threads / 32;
-          const double busy =
-              (double)std::min(ctas, n_models * C) * std::min(warps, chunks * std::min(4, max_genes));
-          const double spill_frac = spills ? 1.0 - (double)(planes / 2) / max_genes : 0.0;
-          const double slot_bytes = spills ? 2.0 * max_genes * plane_bytes : 0.0;
-          const bool l2 = slot_bytes * ctas <= 80e6;
-          double score = busy * (v.loop ? 1.0 : 1.25) * (1.0 - (l2 ? 0.3 : 0.7) * spill_frac);
-          // One cluster barrier per step costs about as much as a step of a
-          // small band (measured): clusters only as a last resort unmeasured.
-          if (C > 1) score *= 0.3 - 0.01 * C;
-          if (gv == 1) score *= 0.9;
-          LaunchPlan plan{};
-          plan.v = v;
           plan.schedule = C > 1                                      ? GRN_SCHEDULE_CLUSTER
                           : (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? GRN_SCHEDULE_GLOBAL
                           : v.loop                                    ? GRN_SCHEDULE_WALK_ITEMS
                                                                       : GRN_SCHEDULE_FIXED_ITEMS;
           plan.threads = threads;
-          plan.gmax = max_genes;
-          plan.planes = planes;
-          plan.smem_bytes = smem;
-          plan.blocks_per_sm = per_sm;
           plan.slot_floats = spills ? 2LL * max_genes * grn::plane_floats(W, H, C) : 0;
           plan.cluster = C;
           plan.blocks = C > 1 ? C * std::max(1, std::min(n_models, ctas / C))
                               : std::max(1, std::min(n_models, ctas));
-          out->push_back({score, plan});
+          out->push_back({plan_cost(ctx, plan, max_genes, n_models,
+                                    spills ? 2.0 * max_genes * plane_bytes : 0.0),
+                          plan});
         }
     }
   }
@@ -396,7 +436,7 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
                                            " genes on this grid with this schedule");
   std::stable_sort(out->begin(), out->end(),
                    [](const std::pair<double, LaunchPlan> &a,
-                      const std::pair<double, LaunchPlan> &b) { return a.first > b.first; });
+                      const std::pair<double, LaunchPlan> &b) { return a.first < b.first; });
   return GRN_OK;
 }
 
@@ -450,8 +490,8 @@ grn_status launch_plan(grn_ctx *ctx, const LaunchPlan &plan, grn::SimArgs a, cud
   return enqueue_plan(ctx, plan, a, stream);
 }
 
-// Measured autotuning: times the feasible plans (best heuristic scores
-// first, at most 8) on the batch's first models -- the most expensive ones,
+// Measured autotuning: times the feasible plans (lowest expected cost
+// first, at most 6) on the batch's first models -- the most expensive ones,
 // the host orders records by cost -- with the step count capped.  Every
 // candidate is launched once untimed (first-launch costs, and the GPU's
 // clock ramp before any timing), then timed in three interleaved rounds,
@@ -520,7 +560,11 @@ grn_status autotune_plan(grn_ctx *ctx, const std::vector<std::pair<double, Launc
   }
   t.state_out = nullptr;
   t.state_planes = 0;
-  const int n_try = std::min<int>((int)plans.size(), 8);
+  // The plans expected to take at most 1.7x the first one's time, 6 of them.
+  int n_try = 1;
+  while (n_try < std::min<int>((int)plans.size(), 6) &&
+         plans[n_try].first <= 1.7 * plans[0].first)
+    ++n_try;
   std::vector<LaunchPlan> cand;
   for (int i = 0; i < n_try; ++i) {
     LaunchPlan ps = plans[i].second;

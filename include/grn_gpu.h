@@ -211,7 +211,7 @@ grn_status grn_set_cluster_size(grn_ctx *ctx, int cluster_size);
 
 /* GRN_SCHEDULE_AUTO's plan choice.  enable = 1 (default): measured -- on the
  * first batch of each shape (W, H, most genes, most links, experiments,
- * fast path, batch size below 2 x SMs) up to 8 feasible plans are timed on
+ * fast path, batch size below 2 x SMs) up to 6 feasible plans are timed on
  * a sample of the batch (2 to 8 models per SM, spread evenly over its cost
  * order; about 2^29 cell-updates per sample launch, at least 128 steps),
  * in three interleaved rounds after an untimed launch of each; the
