@@ -154,15 +154,17 @@ __global__ void output_forward_kernel(int B, int K, const __nv_bfloat16 *h, cons
   if (lane == 0) y[warp] = s + b0[0];
 }
 
-// Loss 1/B sum (y - t)^2, dy = 2 (y - t) / B and db = sum dy; one block of
-// kLossThreads, tree sums in a fixed order.  The operands do not alias, so
-// a thread's loads are all issued before its first store.
+// dL/dy of a row whose error is d.
+__device__ __forceinline__ float output_grad(float d, int B) { return 2.0f * d / (float)B; }
+
+// Loss 1/B sum (y - t)^2 and db = sum dy, dy = 2 (y - t) / B; one block of
+// kLossThreads, tree sums in a fixed order.
 constexpr int kLossThreads = 1024;
 
 __global__ void __launch_bounds__(kLossThreads)
     loss_kernel(int B, const float *__restrict__ y, const float *__restrict__ t,
-                float *__restrict__ dy, double *__restrict__ loss, float *__restrict__ db,
-                int *__restrict__ adam_step) {
+                double *__restrict__ loss, float *__restrict__ db, int *__restrict__ adam_step,
+                int *__restrict__ row) {
   __shared__ double part[kLossThreads];
   __shared__ float dpart[kLossThreads];
   double s = 0.0;
@@ -170,9 +172,7 @@ __global__ void __launch_bounds__(kLossThreads)
 #pragma unroll 4
   for (int i = threadIdx.x; i < B; i += kLossThreads) {
     const float d = y[i] - t[i];
-    const float g = 2.0f * d / (float)B;
-    dy[i] = g;
-    sd += g;
+    sd += output_grad(d, B);
     s += (double)d * d;
   }
   part[threadIdx.x] = s;
@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(kLossThreads)
     loss[1] += l;
     db[0] = dpart[0];
     if (adam_step) *adam_step += 1;  // the Adam step this minibatch takes
+    if (row) *row += B;
   }
 }
 
@@ -199,39 +200,71 @@ __global__ void __launch_bounds__(kLossThreads)
 // that the row-major and the transposed stores are both coalesced.
 constexpr int kTile = 32;
 
-// Gradient of the last hidden layer's pre-activation: dz[b][k] =
-// h[b][k] > 0 ? dy[b] w[k] : 0 (BF16), and dzT[k][b].
-__global__ void output_backward_kernel(int B, int K, const __nv_bfloat16 *h, const float *w,
-                                       const float *dy, __nv_bfloat16 *dz, __nv_bfloat16 *dzT,
-                                       int64_t ldt) {
+// The output layer of a training step and its gradient (mlp_output_step).  A
+// block takes 32 rows and a 32-column tile of dz: its 8 warps each sum 4
+// rows (output_forward_kernel's order; every column tile's block sums the
+// same rows again, which takes less time than a second launch), then the
+// tile is written row-wise and, through shared memory, column-wise.  One
+// launch instead of output, loss and gradient one after the other: the
+// gradient needs only its own row's output.
+__global__ void __launch_bounds__(256)
+    output_step_kernel(int B, int K, const __nv_bfloat16 *h, const float *w, const float *b0,
+                       const float *t, float *y, float *dy, __nv_bfloat16 *dz, __nv_bfloat16 *dzT,
+                       int64_t ldt) {
   __shared__ __nv_bfloat16 tile[kTile][kTile + 2];
-  const int b0 = blockIdx.x * kTile, k0 = blockIdx.y * kTile;
+  __shared__ float g[kTile];
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const int k = k0 + tx;
-  const float wk = k < K ? w[k] : 0.0f;
+  const int r0 = blockIdx.x * kTile, k0 = blockIdx.y * kTile, k = k0 + tx;
+  pdl_trigger();
+  const float bias = b0[0], wk = w[k];
+  pdl_wait();
+  float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  for (int c = tx; c < K; c += 32) {
+    const float wc = w[c];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int b = r0 + ty + 8 * i;
+      if (b < B) s[i] += __bfloat162float(h[(int64_t)b * K + c]) * wc;
+    }
+  }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int r = ty + 8 * i, b = b0 + r;
-    __nv_bfloat16 v = __float2bfloat16(0.0f);
-    if (b < B && k < K) {
-      const float hv = __bfloat162float(h[(int64_t)b * K + k]);
-      v = __float2bfloat16(hv > 0.0f ? dy[b] * wk : 0.0f);
-      dz[(int64_t)b * K + k] = v;
+    const int r = ty + 8 * i, b = r0 + r;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[i] += __shfl_down_sync(0xffffffffu, s[i], o);
+    if (tx == 0 && b < B) {
+      const float yv = s[i] + bias;
+      const float gv = output_grad(yv - t[b], B);
+      g[r] = gv;
+      if (k0 == 0) {
+        y[b] = yv;
+        dy[b] = gv;
+      }
     }
-    tile[r][tx] = v;
   }
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int c = ty + 8 * i, b = b0 + tx;
-    if (k0 + c < K && b < B) dzT[(int64_t)(k0 + c) * ldt + b] = tile[tx][c];
+    const int r = ty + 8 * i, b = r0 + r;
+    if (b < B) {
+      const float hv = __bfloat162float(h[(int64_t)b * K + k]);
+      const __nv_bfloat16 v = __float2bfloat16(hv > 0.0f ? g[r] * wk : 0.0f);
+      dz[(int64_t)b * K + k] = v;
+      tile[r][tx] = v;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int c = ty + 8 * i, b = r0 + tx;
+    if (b < B) dzT[(int64_t)(k0 + c) * ldt + b] = tile[tx][c];
   }
 }
 
-// Rows to BF16: row r is row idx[r] of the BF16 matrix src_b (a gather), or
-// row r of the FP32 matrix src_f; tdst[r] = tsrc[idx[r]] when gathering.
-// dstT (optional) receives the transpose.
-__global__ void rows_to_bf16_kernel(int rows, int width, const int32_t *idx,
+// Rows to BF16: row r is row idx[*first + r] of the BF16 matrix src_b (a
+// gather), or row r of the FP32 matrix src_f; tdst[r] = tsrc[idx[*first + r]]
+// when gathering.  dstT (optional) receives the transpose.
+__global__ void rows_to_bf16_kernel(int rows, int width, const int32_t *idx, const int *first,
                                     const __nv_bfloat16 *src_b, const float *src_f,
                                     const float *tsrc, __nv_bfloat16 *dst, float *tdst,
                                     __nv_bfloat16 *dstT, int64_t ldt) {
@@ -239,6 +272,8 @@ __global__ void rows_to_bf16_kernel(int rows, int width, const int32_t *idx,
   const int r0 = blockIdx.x * kTile, c0 = blockIdx.y * kTile;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int c = c0 + tx;
+  pdl_trigger();
+  if (idx) idx += *first;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int r = ty + 8 * i, row = r0 + r;
@@ -336,14 +371,29 @@ __global__ void __launch_bounds__(256) row_sums_kernel(const RowSumJobs jobs, in
 // Adam on FP32 master weights, step t = *adam_step (device memory, so that
 // a captured training step replays as is); refreshes the BF16 copy and the
 // transposed BF16 copies of the square matrices listed in tr.
-__global__ void adam_kernel(int n, float *w, const float *g, float *m, float *v, float lr,
-                            float b1, float b2, float eps, const int *adam_step,
-                            __nv_bfloat16 *wb, const MlpTransposed tr) {
+// Gradients left as split-K partial tiles are added here, in range order (the
+// order of the separate addition kernel that other callers of the split GEMM
+// use), which saves three launches and one pass over the gradients.
+__global__ void adam_kernel(int n, float *w, const float *g, const MlpPartials part, float *m,
+                            float *v, float lr, float b1, float b2, float eps,
+                            const int *adam_step, __nv_bfloat16 *wb, const MlpTransposed tr) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float t = (float)*adam_step;
   const float c1 = 1.0f - powf(b1, t), c2 = 1.0f - powf(b2, t);
-  const float gi = g[i];
+  float gi = 0.0f;
+  bool own = true;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int64_t o = i - part.offset[j];
+    if (part.split[j] > 1 && o >= 0 && o < part.n[j]) {
+      const float *q = part.work[j] + o;
+#pragma unroll 4
+      for (int z = 0; z < part.split[j]; ++z) gi += q[(int64_t)z * part.n[j]];
+      own = false;
+    }
+  }
+  if (own) gi = g[i];
   const float mi = b1 * m[i] + (1.0f - b1) * gi;
   const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
   m[i] = mi;
@@ -391,19 +441,18 @@ cudaError_t mlp_output_forward(int B, int K, const __nv_bfloat16 *h, const float
   return cudaGetLastError();
 }
 
-cudaError_t mlp_loss(int B, const float *y, const float *t, float *dy, double *loss, float *db,
-                     int *adam_step, cudaStream_t st) {
-  loss_kernel<<<1, kLossThreads, 0, st>>>(B, y, t, dy, loss, db, adam_step);
+cudaError_t mlp_loss(int B, const float *y, const float *t, double *loss, float *db,
+                     int *adam_step, int *row, cudaStream_t st) {
+  loss_kernel<<<1, kLossThreads, 0, st>>>(B, y, t, loss, db, adam_step, row);
   return cudaGetLastError();
 }
 
-cudaError_t mlp_output_backward(int B, int K, const __nv_bfloat16 *h, const float *w,
-                                const float *dy, __nv_bfloat16 *dz, __nv_bfloat16 *dzT,
-                                int64_t ldt, cudaStream_t st) {
-  if (B < 1 || K < 1) return cudaSuccess;
-  output_backward_kernel<<<tile_grid(B, K), dim3(kTile, 8), 0, st>>>(B, K, h, w, dy, dz, dzT,
-                                                                     ldt);
-  return cudaGetLastError();
+cudaError_t mlp_output_step(int B, int K, const __nv_bfloat16 *h, const float *w, const float *b0,
+                            const float *t, float *y, float *dy, __nv_bfloat16 *dz,
+                            __nv_bfloat16 *dzT, int64_t ldt, cudaStream_t st) {
+  if (B < 1 || K < kTile || K % kTile != 0) return cudaErrorInvalidValue;
+  return launch_chained(output_step_kernel, tile_grid(B, K), dim3(kTile, 8), 0, st, B, K, h, w, b0,
+                        t, y, dy, dz, dzT, ldt);
 }
 
 cudaError_t mlp_row_sums(int n_jobs, const MlpRowSum *jobs, int rows, int cols, int64_t ldx,
@@ -415,11 +464,11 @@ cudaError_t mlp_row_sums(int n_jobs, const MlpRowSum *jobs, int rows, int cols, 
   return cudaGetLastError();
 }
 
-cudaError_t mlp_adam(int n, float *w, const float *g, float *m, float *v, float lr, float b1,
-                     float b2, float eps, const int *adam_step, __nv_bfloat16 *wb,
-                     const MlpTransposed &tr, cudaStream_t st) {
-  adam_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, w, g, m, v, lr, b1, b2, eps, adam_step, wb,
-                                               tr);
+cudaError_t mlp_adam(int n, float *w, const float *g, const MlpPartials &part, float *m, float *v,
+                     float lr, float b1, float b2, float eps, const int *adam_step,
+                     __nv_bfloat16 *wb, const MlpTransposed &tr, cudaStream_t st) {
+  adam_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, w, g, part, m, v, lr, b1, b2, eps, adam_step,
+                                               wb, tr);
   return cudaGetLastError();
 }
 
@@ -436,12 +485,12 @@ cudaError_t mlp_transpose(int rows, int cols, const __nv_bfloat16 *src, int64_t 
   return cudaGetLastError();
 }
 
-cudaError_t mlp_gather_rows(int rows, int width, const int32_t *idx, const __nv_bfloat16 *src,
-                            const float *tsrc, __nv_bfloat16 *dst, float *tdst,
+cudaError_t mlp_gather_rows(int rows, int width, const int32_t *idx, const int *first,
+                            const __nv_bfloat16 *src, const float *tsrc, __nv_bfloat16 *dst, float *tdst,
                             __nv_bfloat16 *dstT, int64_t ldt, cudaStream_t st) {
   if (rows < 1) return cudaSuccess;
   rows_to_bf16_kernel<<<tile_grid(rows, width), dim3(kTile, 8), 0, st>>>(
-      rows, width, idx, src, nullptr, tsrc, dst, tdst, dstT, ldt);
+      rows, width, idx, first, src, nullptr, tsrc, dst, tdst, dstT, ldt);
   return cudaGetLastError();
 }
 
@@ -449,7 +498,7 @@ cudaError_t mlp_convert_rows(int rows, int width, const float *src, __nv_bfloat1
                              __nv_bfloat16 *dstT, int64_t ldt, cudaStream_t st) {
   if (rows < 1) return cudaSuccess;
   rows_to_bf16_kernel<<<tile_grid(rows, width), dim3(kTile, 8), 0, st>>>(
-      rows, width, nullptr, nullptr, src, nullptr, dst, nullptr, dstT, ldt);
+      rows, width, nullptr, nullptr, nullptr, src, nullptr, dst, nullptr, dstT, ldt);
   return cudaGetLastError();
 }
 

@@ -10,6 +10,34 @@
 
 namespace grn {
 
+// Programmatic dependent launch: a chain's kernel is launched while the one
+// before it still runs, sets itself up, and waits (pdl_wait) before it
+// touches anything an earlier kernel of the chain writes or reads; the weights
+// are older than the chain.  pdl_trigger lets the next kernel start doing so.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                           cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+#endif
+
 enum MlpEpilogue {
   kEpiF32 = 0,       // C = acc (FP32)
   kEpiBiasRelu = 1,  // C = relu(acc + bias[n]) (BF16)
@@ -48,18 +76,29 @@ cudaError_t mlp_gemm(const MlpGemm &p, cudaStream_t st);
 cudaError_t mlp_gemm_tc(const MlpGemm &p, float *work, size_t work_elems, int *error_flag,
                         cudaStream_t st);
 
+// K ranges that mlp_gemm_tc splits a kEpiF32 GEMM into, given a workspace of
+// work_elems floats (1: no split).
+int mlp_split_k(int M, int N, int K, size_t work_elems);
+// The GEMM without the final addition: with more than one range, range z's
+// tile is left at work + z*M*N (row-major M x N) and C is not written.
+cudaError_t mlp_gemm_tc_partial(const MlpGemm &p, float *work, size_t work_elems, int *error_flag,
+                                cudaStream_t st);
+
+// The output layer of a training step and its gradient, one pass over h:
+// y[b] = h[b] . w + b0, dy[b] = 2 (y[b] - t[b]) / B, dz[b][k] = h[b][k] > 0 ?
+// dy[b] w[k] : 0 (BF16) and its transpose dzT[k][b].  K a multiple of 32.
+cudaError_t mlp_output_step(int B, int K, const __nv_bfloat16 *h, const float *w, const float *b0,
+                            const float *t, float *y, float *dy, __nv_bfloat16 *dz,
+                            __nv_bfloat16 *dzT, int64_t ldt, cudaStream_t st);
 // y[b] = h[b] . w + b0 (the output layer).
 cudaError_t mlp_output_forward(int B, int K, const __nv_bfloat16 *h, const float *w,
                                const float *b0, float *y, cudaStream_t st);
-// dy = 2 (y - t) / B; loss[0] = mean (y - t)^2, loss[1] += loss[0];
-// db[0] = sum dy (the output bias gradient); *adam_step += 1 unless null
-// (a training step's count of Adam steps, read by mlp_adam).
-cudaError_t mlp_loss(int B, const float *y, const float *t, float *dy, double *loss, float *db,
-                     int *adam_step, cudaStream_t st);
-// dz[b][k] = h[b][k] > 0 ? dy[b] w[k] : 0 (BF16), and its transpose dzT[k][b].
-cudaError_t mlp_output_backward(int B, int K, const __nv_bfloat16 *h, const float *w,
-                                const float *dy, __nv_bfloat16 *dz, __nv_bfloat16 *dzT,
-                                int64_t ldt, cudaStream_t st);
+// loss[0] = mean (y - t)^2, loss[1] += loss[0]; db[0] = sum of dy (2 (y - t)
+// / B; the output bias gradient); *adam_step += 1 and *row += B unless null (a
+// training step's count of Adam steps, read by mlp_adam, and the first row of
+// the next minibatch's indices, read by mlp_gather_rows).
+cudaError_t mlp_loss(int B, const float *y, const float *t, double *loss, float *db,
+                     int *adam_step, int *row, cudaStream_t st);
 // Up to four row reductions in one launch: out_j[r] = sum_c X_j[r][c] (x w[c]
 // when w_j is set) for r < rows, c < cols; a fixed summation order.
 struct MlpRowSum {
@@ -76,19 +115,31 @@ struct MlpTransposed {
   __nv_bfloat16 *dst[2];
   int n;
 };
+// Gradients left as split-K partial tiles (mlp_gemm_tc_partial): parameters
+// offset .. offset + n - 1 have the gradient sum over z < split of
+// work[z*n + i], added in order; split 1: the gradient array's own value.
+struct MlpPartials {
+  int64_t offset[3];
+  int n[3];
+  int split[3];
+  const float *work[3];
+};
 // One Adam step on the FP32 parameters w (moments m, v; step number
-// *adam_step, in device memory), refreshing their BF16 copy wb and the
-// transposed copies of tr.
-cudaError_t mlp_adam(int n, float *w, const float *g, float *m, float *v, float lr, float b1,
-                     float b2, float eps, const int *adam_step, __nv_bfloat16 *wb,
-                     const MlpTransposed &tr, cudaStream_t st);
+// *adam_step, in device memory; gradients g or, where split, the partial
+// sums), refreshing their BF16 copy wb and the transposed copies of tr.
+cudaError_t mlp_adam(int n, float *w, const float *g, const MlpPartials &part, float *m, float *v,
+                     float lr, float b1, float b2, float eps, const int *adam_step,
+                     __nv_bfloat16 *wb, const MlpTransposed &tr, cudaStream_t st);
 cudaError_t mlp_to_bf16(int n, const float *x, __nv_bfloat16 *y, cudaStream_t st);
 // dst[c][r] = src[r][c] for a rows x cols BF16 matrix.
 cudaError_t mlp_transpose(int rows, int cols, const __nv_bfloat16 *src, int64_t lds,
                           __nv_bfloat16 *dst, int64_t ldd, cudaStream_t st);
-// Row r of dst (width columns) = row idx[r] of src, tdst[r] = tsrc[idx[r]];
-// dstT (optional) receives the transpose, dstT[c*ldt + r].
-cudaError_t mlp_gather_rows(int rows, int width, const int32_t *idx, const __nv_bfloat16 *src,
+// Row r of dst (width columns) = row idx[*first + r] of src, tdst[r] =
+// tsrc[idx[*first + r]] (*first in device memory, so that a captured
+// training step gathers the next minibatch each time); dstT (optional)
+// receives the transpose, dstT[c*ldt + r].
+cudaError_t mlp_gather_rows(int rows, int width, const int32_t *idx, const int *first,
+                            const __nv_bfloat16 *src,
                             const float *tsrc, __nv_bfloat16 *dst, float *tdst,
                             __nv_bfloat16 *dstT, int64_t ldt, cudaStream_t st);
 // FP32 rows to BF16 (dst) and optionally their transpose (dstT).

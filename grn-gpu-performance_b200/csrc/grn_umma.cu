@@ -24,6 +24,10 @@
 // ranges in order, so the result is deterministic.  The weight-gradient
 // GEMMs (256 x 256 outputs, K = the batch) need it: 8 tiles alone would
 // leave most SMs idle.
+// Launches are chained (grn_mlp.h): barriers, tensor memory and, where B is a
+// weight matrix, the first B slices are set up before the kernel waits for
+// the one before it, and the epilogue's mask and bias are read while the
+// tensor core works.
 // Every wait is bounded (about a second); on a time-out the CTA waits again
 // (bounded) for its loads and MMAs in flight, frees its tensor memory, sets
 // the error flag and returns.
@@ -50,8 +54,11 @@ constexpr int kABytes = kTM * kKC * 2;
 constexpr int kBBytes = kBN * kKC * 2;
 constexpr int kStageBytes = kABytes + kBBytes;
 // 1 KB of slack to align the ring to the 1024-byte swizzle atom, the ring,
-// the barriers (full, empty per stage; done) and four control words.
-constexpr size_t kSmemBytes = 1024 + (size_t)kStages * kStageBytes + 8 * (2 * kStages + 1) + 16;
+// the barriers (full, empty per stage; done), four control words and the
+// tile's bias.
+constexpr size_t kBiasOffset =
+    ((size_t)kStages * kStageBytes + 8 * (2 * kStages + 1) + 16 + 15) & ~size_t(15);
+constexpr size_t kSmemBytes = 1024 + kBiasOffset + kBN * sizeof(float);
 constexpr int kTargetCtas = 148;  // split K until about one CTA per SM runs
 constexpr int kMinSlices = 2;     // K slices per range at least
 
@@ -148,9 +155,11 @@ __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t *>(&p);
 }
 
-// Epilogue of 32 consecutive columns nb .. nb + nn - 1 of tile row m.
+// Epilogue of 32 consecutive columns nb .. nb + nn - 1 of tile row m: `bias`
+// their biases (shared memory), `mask` their mask words if mask_early.
 __device__ __forceinline__ void store_row(const UmmaArgs &g, int m, int nb, int nn,
-                                          const uint32_t (&v)[32]) {
+                                          const uint32_t (&v)[32], const float *bias,
+                                          const uint4 *mask, bool mask_early) {
   float x[32];
 #pragma unroll
   for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]);
@@ -171,30 +180,27 @@ __device__ __forceinline__ void store_row(const UmmaArgs &g, int m, int nb, int 
   }
   if (g.epi == kEpiBiasRelu) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (j < nn) {
-        const float y = x[j] + g.bias[nb + j];
-        x[j] = y > 0.0f ? y : 0.0f;
-      }
-  } else {  // kEpiMask
-    const __nv_bfloat16 *mk = g.mask + (int64_t)m * g.ldc + nb;
-    if (nn == 32 && ((uintptr_t)mk & 15) == 0) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint4 u = reinterpret_cast<const uint4 *>(mk)[q];
-        const __nv_bfloat162 *p = reinterpret_cast<const __nv_bfloat162 *>(&u);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __bfloat1622float2(p[e]);
-          x[8 * q + 2 * e] = f.x > 0.0f ? x[8 * q + 2 * e] : 0.0f;
-          x[8 * q + 2 * e + 1] = f.y > 0.0f ? x[8 * q + 2 * e + 1] : 0.0f;
-        }
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (j < nn) x[j] = __bfloat162float(mk[j]) > 0.0f ? x[j] : 0.0f;
+    for (int j = 0; j < 32; ++j) {
+      const float y = x[j] + bias[j];
+      x[j] = y > 0.0f ? y : 0.0f;
     }
+  } else if (mask_early) {  // kEpiMask
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint4 u = mask[q];
+      const __nv_bfloat162 *p = reinterpret_cast<const __nv_bfloat162 *>(&u);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __bfloat1622float2(p[e]);
+        x[8 * q + 2 * e] = f.x > 0.0f ? x[8 * q + 2 * e] : 0.0f;
+        x[8 * q + 2 * e + 1] = f.y > 0.0f ? x[8 * q + 2 * e + 1] : 0.0f;
+      }
+    }
+  } else {
+    const __nv_bfloat16 *mk = g.mask + (int64_t)m * g.ldc + nb;
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < nn) x[j] = __bfloat162float(mk[j]) > 0.0f ? x[j] : 0.0f;
   }
   __nv_bfloat16 *dst = g.Cb + (int64_t)m * g.ldc + nb;
   if (nn == 32 && ((uintptr_t)dst & 15) == 0) {
@@ -233,6 +239,11 @@ __global__ void __launch_bounds__(128) umma_gemm_kernel(const __grid_constant__ 
   const uint32_t sa = ring, sb = ring + kStages * kABytes;
   const uint32_t full = smem_u32(bars), empty = full + 8 * kStages, done = full + 16 * kStages;
 
+  pdl_trigger();
+  if (tid == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&ta)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tb)) : "memory");
+  }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32((const void *)ctl)),
@@ -251,6 +262,34 @@ __global__ void __launch_bounds__(128) umma_gemm_kernel(const __grid_constant__ 
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = (uint32_t)ctl[0];
+  // With a BF16 result B is a weight matrix, older than the chain of launches:
+  // the first ring's B slices are fetched before the wait for the chain.
+  const int early = g.epi != kEpiF32 ? min(nk, kStages) : 0;
+  if (tid == 0) {
+    for (int i = 0; i < early; ++i) {
+      mbar_expect_tx(full + 8 * i, kStageBytes);
+      tma_load(sb + i * kBBytes, &tb, full + 8 * i, kbeg + i * kKC, n0);
+    }
+  }
+  pdl_wait();
+
+  // The epilogue's operands, read while the tensor core works: this thread's
+  // row of the mask (as 16-byte words) and the tile's bias.
+  const int my_m = m0 + warp * 32 + lane;
+  uint4 mask[kBN / 8];
+  const bool mask_early = g.epi == kEpiMask && my_m < g.M && n0 + kBN <= g.N &&
+                          ((uintptr_t)(g.mask + (int64_t)my_m * g.ldc + n0) & 15) == 0;
+  if (mask_early) {
+    const uint4 *mk = reinterpret_cast<const uint4 *>(g.mask + (int64_t)my_m * g.ldc + n0);
+#pragma unroll
+    for (int q = 0; q < kBN / 8; ++q) mask[q] = mk[q];
+  }
+  float *s_bias = reinterpret_cast<float *>(smem + kBiasOffset);
+  static_assert(kBN == 64, "one bias per thread 64 .. 127");
+  if (g.epi == kEpiBiasRelu && tid >= 64) {
+    const int n = n0 + tid - 64;
+    s_bias[tid - 64] = n < g.N ? g.bias[n] : 0.0f;
+  }
 
   if (tid == 0) {
     int i = 0;
@@ -258,9 +297,9 @@ __global__ void __launch_bounds__(128) umma_gemm_kernel(const __grid_constant__ 
       const int s = i % kStages;
       if (i >= kStages && !mbar_wait(empty + 8 * s, ((i / kStages) - 1) & 1)) break;
       const int k0 = kbeg + i * kKC;
-      mbar_expect_tx(full + 8 * s, kStageBytes);
+      if (i >= early) mbar_expect_tx(full + 8 * s, kStageBytes);
       tma_load(sa + s * kABytes, &ta, full + 8 * s, k0, m0);
-      tma_load(sb + s * kBBytes, &tb, full + 8 * s, k0, n0);
+      if (i >= early) tma_load(sb + s * kBBytes, &tb, full + 8 * s, k0, n0);
     }
     ctl[2] = i;
     if (i < nk) ctl[1] = 1;
@@ -294,8 +333,8 @@ __global__ void __launch_bounds__(128) umma_gemm_kernel(const __grid_constant__ 
   const bool ok = __syncthreads_and(waited) && ctl[1] == 0;
   if (ok) {
     asm volatile("tcgen05.fence::after_thread_sync;");
-    const int m = m0 + warp * 32 + lane;  // TMEM lane = tile row
-#pragma unroll 1
+    const int m = my_m;  // TMEM lane = tile row
+#pragma unroll
     for (int c0 = 0; c0 < kBN; c0 += 32) {
       uint32_t v[32];
       const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
@@ -312,7 +351,8 @@ __global__ void __launch_bounds__(128) umma_gemm_kernel(const __grid_constant__ 
           : "r"(taddr));
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       const int nb = n0 + c0;
-      if (m < g.M && nb < g.N) store_row(g, m, nb, min(32, g.N - nb), v);
+      if (m < g.M && nb < g.N)
+        store_row(g, m, nb, min(32, g.N - nb), v, s_bias + c0, mask + c0 / 8, mask_early);
     }
   } else {
     // Something timed out: wait (bounded) for the loads the MMA issuer did
@@ -387,8 +427,31 @@ bool operand_map(EncodeTiled enc, CUtensorMap *map, const __nv_bfloat16 *ptr, in
 
 }  // namespace
 
-cudaError_t mlp_gemm_tc(const MlpGemm &p, float *work, size_t work_elems, int *error_flag,
-                        cudaStream_t st) {
+namespace {
+
+// K ranges (each a multiple of kKC, every one non-empty) and their length.
+int split_ranges(int M, int N, int K, size_t work_elems, int *per_out) {
+  const int tiles = ((M + kTM - 1) / kTM) * ((N + kBN - 1) / kBN);
+  const int slices = (K + kKC - 1) / kKC;
+  int split = 1;
+  if (tiles < kTargetCtas) {
+    split = std::min(slices / kMinSlices, (kTargetCtas + tiles - 1) / tiles);
+    while (split > 1 && (size_t)split * M * N > work_elems) --split;
+    if (split < 1) split = 1;
+  }
+  const int per = ((slices + split - 1) / split) * kKC;
+  if (per_out) *per_out = per;
+  return (K + per - 1) / per;
+}
+
+}  // namespace
+
+int mlp_split_k(int M, int N, int K, size_t work_elems) {
+  return split_ranges(M, N, K, work_elems, nullptr);
+}
+
+cudaError_t mlp_gemm_tc_partial(const MlpGemm &p, float *work, size_t work_elems, int *error_flag,
+                                cudaStream_t st) {
   if (p.M < 1 || p.N < 1 || p.K < 1 || !error_flag) return cudaErrorInvalidValue;
   const EncodeTiled enc = encoder();
   if (!enc) return cudaErrorNotSupported;
@@ -396,16 +459,8 @@ cudaError_t mlp_gemm_tc(const MlpGemm &p, float *work, size_t work_elems, int *e
   if (!operand_map(enc, &ta, p.A, p.M, p.K, p.lda, kTM) ||
       !operand_map(enc, &tb, p.B, p.N, p.K, p.ldb, kBN))
     return cudaErrorInvalidValue;
-  const int tiles = ((p.M + kTM - 1) / kTM) * ((p.N + kBN - 1) / kBN);
-  const int slices = (p.K + kKC - 1) / kKC;
-  int split = 1;
-  if (p.epi == kEpiF32 && work && tiles < kTargetCtas) {
-    split = std::min(slices / kMinSlices, (kTargetCtas + tiles - 1) / tiles);
-    while (split > 1 && (size_t)split * p.M * p.N > work_elems) --split;
-    if (split < 1) split = 1;
-  }
-  const int per = ((slices + split - 1) / split) * kKC;
-  split = (p.K + per - 1) / per;  // every range non-empty
+  int per = (p.K + kKC - 1) / kKC * kKC, split = 1;
+  if (p.epi == kEpiF32 && work) split = split_ranges(p.M, p.N, p.K, work_elems, &per);
   UmmaArgs g{p.M, p.N, p.K, per, p.epi, p.Cf, p.Cb, p.ldc, p.Ct, p.ldt, p.bias, p.mask,
              split > 1 ? work : nullptr, error_flag};
   cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel,
@@ -413,9 +468,15 @@ cudaError_t mlp_gemm_tc(const MlpGemm &p, float *work, size_t work_elems, int *e
                                        (int)kSmemBytes);
   if (e != cudaSuccess) return e;
   const dim3 grid((p.M + kTM - 1) / kTM, (p.N + kBN - 1) / kBN, split);
-  umma_gemm_kernel<<<grid, 128, kSmemBytes, st>>>(ta, tb, g);
-  e = cudaGetLastError();
-  if (e != cudaSuccess || split == 1) return e;
+  return launch_chained(umma_gemm_kernel, grid, dim3(128), kSmemBytes, st, ta, tb, g);
+}
+
+cudaError_t mlp_gemm_tc(const MlpGemm &p, float *work, size_t work_elems, int *error_flag,
+                        cudaStream_t st) {
+  const cudaError_t e = mlp_gemm_tc_partial(p, work, work_elems, error_flag, st);
+  if (e != cudaSuccess || p.epi != kEpiF32 || !work) return e;
+  const int split = mlp_split_k(p.M, p.N, p.K, work_elems);
+  if (split == 1) return e;
   const int64_t mn = (int64_t)p.M * p.N;
   splitk_sum_kernel<<<(unsigned)((mn + 255) / 256), 256, 0, st>>>(split, p.M, p.N, work, p.Cf,
                                                                    p.ldc);

@@ -57,8 +57,13 @@ struct grn_surrogate {
   float *xf = nullptr;  // FP32 staging of uploaded rows [bmax][kF]
   float *y = nullptr, *t = nullptr, *dy = nullptr;
   double *loss = nullptr;  // [0] last minibatch, [1] sum over a training call
-  float *work = nullptr;   // split-K partial tiles of the weight gradients
-  size_t work_elems = 0;
+  float *work = nullptr;   // split-K partial tiles of the three weight gradients
+  size_t work_elems = 0;   // floats of one layer's part
+  // The training step's side streams (weight gradients; sums over the batch)
+  // and the events that fork and join them.
+  cudaStream_t side[2] = {};
+  cudaEvent_t fork[3] = {}, join[2] = {};
+  int *d_row = nullptr;    // first row of the next minibatch's indices
   int32_t *idx = nullptr;
   int idx_cap = 0;
   int cap = 0, count = 0, head = 0;  // dataset ring buffer
@@ -92,9 +97,9 @@ grn::MlpGemm gemm_args(int M, int N, int K, const __nv_bfloat16 *A, int64_t lda,
   return p;
 }
 
-// One GEMM of the MLP on the selected tensor-core path.
+// One GEMM of the MLP with a BF16 result, on the selected tensor-core path.
 cudaError_t gemm(grn_surrogate *s, const grn::MlpGemm &p) {
-  if (s->tcgen05) return grn::mlp_gemm_tc(p, s->work, s->work_elems, s->d_err, s->st);
+  if (s->tcgen05) return grn::mlp_gemm_tc(p, nullptr, 0, s->d_err, s->st);
   return grn::mlp_gemm(p, s->st);
 }
 
@@ -107,8 +112,9 @@ grn_status check_err(grn_surrogate *s) {
   return GRN_ERR_KERNEL;
 }
 
-// Hidden layers and output of the rows in s->x; `train` also stores the
-// transposed activations that the weight gradients read.
+// Hidden layers of the rows in s->x, and their output unless `train`, which
+// stores the transposed activations that the weight gradients read instead
+// (backward computes the output with its gradient).
 grn_status forward(grn_surrogate *s, int B, bool train) {
   using namespace grn;
   const int64_t T = s->bmax;
@@ -128,18 +134,36 @@ grn_status forward(grn_surrogate *s, int B, bool train) {
     }
     GRN_CK(gemm(s, p));
   }
-  GRN_CK(mlp_output_forward(B, kH, s->h3, s->w + kW4, s->w + kB4, s->y, s->st));
+  if (!train) GRN_CK(mlp_output_forward(B, kH, s->h3, s->w + kW4, s->w + kB4, s->y, s->st));
   return GRN_OK;
 }
 
-// Loss and gradients of a minibatch already in s->x / s->xT / s->t (after
-// forward with train set); `adam` counts the Adam step that follows.
-grn_status backward(grn_surrogate *s, int B, bool adam) {
+// Output, loss and gradients of a minibatch already in s->x / s->xT / s->t
+// (after forward with train set).  `adam` counts the Adam step that follows
+// and leaves split weight gradients as partial tiles for it (*part).
+//
+// The chain output -> dZ3 -> dZ2 -> dZ1 -> dW1 runs on s->st; the loss and
+// the batch sums (side 0) and dW3, dW2 (side 1) branch off as soon as their
+// inputs are there.  At 512 rows every launch is a few microseconds of
+// latency on a nearly idle GPU, so a step takes as long as its longest
+// chain: 9 launches instead of 17 one after the other, each set up while
+// the one before runs (launch_chained).  Measured, 32 steps of 512 rows: 2.94
+// -> 2.44 ms by the branches, 1.90 ms with the chained launches; several
+// steps in one graph gave no more.
+grn_status backward(grn_surrogate *s, int B, bool adam, grn::MlpPartials *part) {
   using namespace grn;
   cudaStream_t st = s->st;
   const int64_t T = s->bmax;
-  GRN_CK(mlp_loss(B, s->y, s->t, s->dy, s->loss, s->g + kB4, adam ? s->d_step : nullptr, st));
-  GRN_CK(mlp_output_backward(B, kH, s->h3, s->w + kW4, s->dy, s->dz3, s->dz3T, T, st));
+  GRN_CK(mlp_output_step(B, kH, s->h3, s->w + kW4, s->w + kB4, s->t, s->y, s->dy, s->dz3, s->dz3T,
+                         T, st));
+  GRN_CK(cudaEventRecord(s->fork[0], st));
+  GRN_CK(cudaStreamWaitEvent(s->side[0], s->fork[0], 0));
+  GRN_CK(cudaStreamWaitEvent(s->side[1], s->fork[0], 0));
+  GRN_CK(mlp_loss(B, s->y, s->t, s->loss, s->g + kB4, adam ? s->d_step : nullptr,
+                  adam ? s->d_row : nullptr, s->side[0]));
+  // Output weights and hidden biases: sums over the batch of the transposes.
+  const MlpRowSum out_sums[2] = {{s->h3T, s->dy, s->g + kW4}, {s->dz3T, nullptr, s->g + kB3}};
+  GRN_CK(mlp_row_sums(2, out_sums, kH, B, T, s->side[0]));
   // Per hidden layer l = 3, 2, 1: dW_l = dZ_l^T H_(l-1) (K = the batch, from
   // the transposed copies), and for l > 1 dZ_(l-1) = (dZ_l W_l) * [H_(l-1) > 0].
   const __nv_bfloat16 *dzT[3] = {s->dz1T, s->dz2T, s->dz3T};
@@ -148,30 +172,50 @@ grn_status backward(grn_surrogate *s, int B, bool adam) {
   const __nv_bfloat16 *hprev[3] = {s->x, s->h1, s->h2};
   const __nv_bfloat16 *wt[3] = {nullptr, s->w2t, s->w3t};
   __nv_bfloat16 *dzo[3] = {nullptr, s->dz1, s->dz2}, *dzoT[3] = {nullptr, s->dz1T, s->dz2T};
-  const int64_t wo[3] = {kW1, kW2, kW3};
+  const int64_t wo[3] = {kW1, kW2, kW3}, bo[3] = {kB1, kB2, kB3};
   for (int l = 2; l >= 0; --l) {
     const int N = l == 0 ? kF : kH;
     MlpGemm p = gemm_args(kH, N, B, dzT[l], T, hT[l], T);
     p.epi = kEpiF32;
     p.Cf = s->g + wo[l];
     p.ldc = N;
-    GRN_CK(gemm(s, p));
-    if (l == 0) break;
-    p = gemm_args(B, kH, kH, dz[l], kH, wt[l], kH);
-    p.epi = kEpiMask;
-    p.Cb = dzo[l];
-    p.ldc = kH;
-    p.mask = hprev[l];
-    p.Ct = dzoT[l];
-    p.ldt = T;
-    GRN_CK(gemm(s, p));
+    cudaStream_t sw = l == 0 ? st : s->side[1];
+    float *work = s->work + (size_t)l * s->work_elems;
+    if (l > 0) {
+      MlpGemm q = gemm_args(B, kH, kH, dz[l], kH, wt[l], kH);
+      q.epi = kEpiMask;
+      q.Cb = dzo[l];
+      q.ldc = kH;
+      q.mask = hprev[l];
+      q.Ct = dzoT[l];
+      q.ldt = T;
+      GRN_CK(gemm(s, q));
+      GRN_CK(cudaEventRecord(s->fork[l], st));
+    }
+    part->offset[l] = wo[l];
+    part->n[l] = kH * N;
+    part->work[l] = work;
+    part->split[l] = 1;
+    if (!s->tcgen05) {
+      GRN_CK(mlp_gemm(p, sw));
+    } else if (adam) {
+      part->split[l] = mlp_split_k(p.M, p.N, p.K, s->work_elems);
+      GRN_CK(mlp_gemm_tc_partial(p, work, s->work_elems, s->d_err, sw));
+    } else {
+      GRN_CK(mlp_gemm_tc(p, work, s->work_elems, s->d_err, sw));
+    }
+    if (l > 0) {
+      // The layer below has its dZ: its batch sum and weight gradient.
+      GRN_CK(cudaStreamWaitEvent(s->side[0], s->fork[l], 0));
+      const MlpRowSum sum = {dzoT[l], nullptr, s->g + bo[l - 1]};
+      GRN_CK(mlp_row_sums(1, &sum, kH, B, T, s->side[0]));
+      if (l > 1) GRN_CK(cudaStreamWaitEvent(s->side[1], s->fork[l], 0));
+    }
   }
-  // Output weights and hidden biases: sums over the batch of the transposes.
-  const MlpRowSum jobs[4] = {{s->h3T, s->dy, s->g + kW4},
-                             {s->dz3T, nullptr, s->g + kB3},
-                             {s->dz2T, nullptr, s->g + kB2},
-                             {s->dz1T, nullptr, s->g + kB1}};
-  GRN_CK(mlp_row_sums(4, jobs, kH, B, T, st));
+  for (int i = 0; i < 2; ++i) {
+    GRN_CK(cudaEventRecord(s->join[i], s->side[i]));
+    GRN_CK(cudaStreamWaitEvent(st, s->join[i], 0));
+  }
   return GRN_OK;
 }
 
@@ -183,13 +227,16 @@ grn_status transpose_weights(grn_surrogate *s) {
   return GRN_OK;
 }
 
-// Forward, backward and Adam on the minibatch in s->x / s->xT / s->t.
+// Gather, forward, backward and Adam on the next B rows of s->idx.
 grn_status train_step_body(grn_surrogate *s, int B, float lr) {
+  GRN_CK(grn::mlp_gather_rows(B, kF, s->idx, s->d_row, s->dx, s->dt, s->x, s->t, s->xT, s->bmax,
+                              s->st));
+  grn::MlpPartials part{};
   grn_status st = forward(s, B, true);
-  if (st == GRN_OK) st = backward(s, B, true);
+  if (st == GRN_OK) st = backward(s, B, true, &part);
   if (st != GRN_OK) return st;
   const grn::MlpTransposed tr{{kW2, kW3}, {s->w2t, s->w3t}, kH};
-  GRN_CK(grn::mlp_adam((int)kP, s->w, s->g, s->m, s->v, lr, 0.9f, 0.999f, 1e-8f, s->d_step,
+  GRN_CK(grn::mlp_adam((int)kP, s->w, s->g, part, s->m, s->v, lr, 0.9f, 0.999f, 1e-8f, s->d_step,
                        s->wb, tr, s->st));
   return GRN_OK;
 }
@@ -200,7 +247,7 @@ void drop_train_graph(grn_surrogate *s) {
 }
 
 // One training step.  The first step of a (batch size, learning rate,
-// tensor-core path) runs its 16 launches directly -- which also loads every
+// tensor-core path) runs its launches directly -- which also loads every
 // kernel's module -- and is then captured as a graph; later steps replay it
 // (the kernels' arguments do not change; the Adam step count is read from
 // device memory).
@@ -230,14 +277,6 @@ grn_status train_step(grn_surrogate *s, int B, float lr) {
   return GRN_OK;
 }
 
-// One Adam step on the training-set rows d_idx[0..B) (device indices).
-grn_status train_minibatch(grn_surrogate *s, const int32_t *d_idx, int B, float lr) {
-  GRN_CK(grn::mlp_gather_rows(B, kF, d_idx, s->dx, s->dt, s->x, s->t, s->xT, s->bmax, s->st));
-  const grn_status st = train_step(s, B, lr);
-  if (st == GRN_OK) s->step += 1;
-  return st;
-}
-
 // Runs minibatch i on the sizes[i] training-set rows that follow in idx.
 // Indices go to the device in chunks of whole minibatches, and the losses
 // add up on the device: one host synchronisation per call.
@@ -250,11 +289,11 @@ grn_status run_minibatches(grn_surrogate *s, const std::vector<int32_t> &idx,
     while (e < sizes.size() && rows + sizes[e] <= (size_t)s->idx_cap) rows += sizes[e++];
     GRN_CK(cudaMemcpyAsync(s->idx, idx.data() + pos, rows * sizeof(int32_t),
                            cudaMemcpyHostToDevice, s->st));
-    size_t off = 0;
+    GRN_CK(cudaMemsetAsync(s->d_row, 0, sizeof(int), s->st));
     for (; b < e; ++b) {
-      const grn_status st = train_minibatch(s, s->idx + off, sizes[b], lr);
+      const grn_status st = train_step(s, sizes[b], lr);
       if (st != GRN_OK) return st;
-      off += sizes[b];
+      s->step += 1;
     }
     pos += rows;
   }
@@ -342,6 +381,10 @@ grn_status grn_surrogate_create(int device, uint64_t seed, int capacity, grn_sur
   s->bmax = 8192;
   cudaSetDevice(device);
   bool ok = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) == cudaSuccess;
+  for (cudaStream_t &q : s->side)
+    ok = ok && cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) == cudaSuccess;
+  for (cudaEvent_t *ev : {&s->fork[0], &s->fork[1], &s->fork[2], &s->join[0], &s->join[1]})
+    ok = ok && cudaEventCreateWithFlags(ev, cudaEventDisableTiming) == cudaSuccess;
   auto alloc = [&](void **p, size_t bytes) {
     if (ok && cudaMalloc(p, bytes) != cudaSuccess) ok = false;
   };
@@ -362,15 +405,19 @@ grn_status grn_surrogate_create(int device, uint64_t seed, int capacity, grn_sur
   alloc((void **)&s->t, B * 4);
   alloc((void **)&s->dy, B * 4);
   alloc((void **)&s->loss, 2 * sizeof(double));
-  // Split-K workspace: 32 partial 256 x 256 FP32 tiles.
-  s->work_elems = (size_t)32 * kH * kH;
-  alloc((void **)&s->work, s->work_elems * 4);
+  // Split-K workspaces, one per layer (their GEMMs may run at the same time):
+  // about one CTA per SM makes at most 19 ranges of 256 x 256 FP32, or 37 of
+  // 256 x 128.
+  s->work_elems = (size_t)20 * kH * kH;
+  alloc((void **)&s->work, 3 * s->work_elems * 4);
   s->idx_cap = 16 * s->bmax;
   alloc((void **)&s->idx, (size_t)s->idx_cap * 4);
   alloc((void **)&s->dx, (size_t)capacity * kF * 2);
   alloc((void **)&s->dt, (size_t)capacity * 4);
   alloc((void **)&s->d_err, sizeof(int));
   if (ok && cudaMemset(s->d_err, 0, sizeof(int)) != cudaSuccess) ok = false;
+  alloc((void **)&s->d_row, sizeof(int));
+  if (ok && cudaMemset(s->d_row, 0, sizeof(int)) != cudaSuccess) ok = false;
   alloc((void **)&s->d_step, sizeof(int));
   if (ok && cudaMemset(s->d_step, 0, sizeof(int)) != cudaSuccess) ok = false;
   if (!ok) {
@@ -407,9 +454,12 @@ grn_status grn_surrogate_destroy(grn_surrogate *s) {
                   (void *)s->h1T, (void *)s->h2T, (void *)s->h3T, (void *)s->dz1T,
                   (void *)s->dz2T, (void *)s->dz3T, (void *)s->xf, (void *)s->y, (void *)s->t,
                   (void *)s->dy, (void *)s->loss, (void *)s->work, (void *)s->idx, (void *)s->dx,
-                  (void *)s->dt, (void *)s->d_err, (void *)s->d_step})
+                  (void *)s->dt, (void *)s->d_err, (void *)s->d_step, (void *)s->d_row})
     if (p) cudaFree(p);
-  if (s->st) cudaStreamDestroy(s->st);
+  for (cudaEvent_t ev : {s->fork[0], s->fork[1], s->fork[2], s->join[0], s->join[1]})
+    if (ev) cudaEventDestroy(ev);
+  for (cudaStream_t q : {s->st, s->side[0], s->side[1]})
+    if (q) cudaStreamDestroy(q);
   delete s;
   return GRN_OK;
 }
@@ -621,7 +671,8 @@ grn_status grn_surrogate_gradients(grn_surrogate *s, const float *features,
   if (st != GRN_OK) return st;
   GRN_CK(cudaMemcpyAsync(s->t, log_error, n * 4, cudaMemcpyHostToDevice, s->st));
   st = forward(s, n, true);
-  if (st == GRN_OK) st = backward(s, n, false);
+  grn::MlpPartials part{};
+  if (st == GRN_OK) st = backward(s, n, false, &part);
   if (st != GRN_OK) return st;
   GRN_CK(cudaMemcpyAsync(grads, s->g, kP * 4, cudaMemcpyDeviceToHost, s->st));
   double l = 0;
