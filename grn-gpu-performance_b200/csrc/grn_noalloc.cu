@@ -265,5 +265,6 @@ extern "C" grn_status grn_evaluate_batch_noalloc_status(void *cuda_stream, char 
                    flag == 3   ? "bounds check: a simulation kernel state access fell outside "
                                  "its buffer"
                    : flag == 2 ? "the simulation kernel's wait for a bulk copy timed out"
+                   : flag == 4 ? "the simulation kernel's wait for a neighbouring warp timed out"
                                : "the simulation kernel rejected a model record");
 }

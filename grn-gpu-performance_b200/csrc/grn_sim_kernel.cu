@@ -223,7 +223,11 @@ constexpr size_t kMbarOffset = (kCsumOffset + kMaxCluster * 8 + 15) & ~size_t(15
 constexpr size_t kStreamFailOffset = kMbarOffset + 16;
 // Bounds-checked build only: the regions that state accesses are checked
 // against (CheckRegions).
-constexpr size_t kCheckOffset = (kStreamFailOffset + 16 + 15) & ~size_t(15);
+// Steps without a block barrier (StepSync): finished work per chunk (int
+// [kMaxDone]).
+constexpr int kMaxDone = 128;
+constexpr size_t kDoneOffset = kStreamFailOffset + 16;
+constexpr size_t kCheckOffset = (kDoneOffset + kMaxDone * 4 + 15) & ~size_t(15);
 constexpr size_t kCheckBytes = GRN_BOUNDS_CHECK ? 64 : 0;
 constexpr size_t kStateOffset = (kCheckOffset + kCheckBytes + 127) & ~size_t(127);
 
@@ -522,12 +526,14 @@ __device__ __forceinline__ float update_cell(float c, float h, float lim, float 
 }
 
 // State accesses of the step: byte offsets from the shared-memory state area
-// (a constant address, so that an offset is all a load needs), or from a
-// global pointer.
+// (a constant address, so that an offset is all a load needs), or unsigned
+// ones from a global pointer that is the same for the whole block (a uniform
+// base and a 32-bit offset; a slot is smaller than 4 GB).
 template <int N, bool GL>
 __device__ __forceinline__ const float *state_at(const char *gl, int off) {
   return chk<N>(reinterpret_cast<const float *>(
-      GL ? gl + off : reinterpret_cast<const char *>(grn_dyn_smem) + kStateOffset + off));
+      GL ? gl + (uint32_t)off
+         : reinterpret_cast<const char *>(grn_dyn_smem) + kStateOffset + off));
 }
 template <bool GL>
 __device__ __forceinline__ float4 load4(const char *gl, int off) {
@@ -536,12 +542,12 @@ __device__ __forceinline__ float4 load4(const char *gl, int off) {
 
 // Planes a step reads and writes.  Plane k of the current state is at shared
 // offset sm + k * PSb for k < n_sm, else at gl + k * PSb; its next state at
-// sm_out + k * PSb, or gl_out + k * out_stride.
+// sm_out + k * PSb, or (a staged band) at gl_out + k * out_stride.
 struct Planes {
   int sm, sm_out;
   const char *gl;
   char *gl_out;
-  size_t out_stride;
+  int out_stride;
   int n_sm;
 };
 
@@ -580,9 +586,9 @@ __device__ __forceinline__ void link_terms(float4 (&t)[R], const float4 &ab, int
                                            const Geom &g) {
   float4 x[R];
   if (SPILL && slot >= pl.n_sm) {
-    const char *q = pl.gl + (size_t)slot * g.PSb;
+    const int o = slot * g.PSb + st.base;
 #pragma unroll
-    for (int i = 0; i < R; ++i) x[i] = load4<true>(q, st.base + i * g.RSb);
+    for (int i = 0; i < R; ++i) x[i] = load4<true>(pl.gl, o + i * g.RSb);
   } else {
     const int o = slot * g.PSb + (pl.sm + st.base);
 #pragma unroll
@@ -787,14 +793,14 @@ __device__ __forceinline__ void gene_step(const ProgSmem &P, int k, const Planes
   regulation<R, EXACT, SPILL>(P, ctl, pl, st, g, h);
   const auto update = [&](auto diffuses) {
     constexpr bool D = decltype(diffuses)::value;
-    char *const out = pl.gl_out + p * pl.out_stride;
+    const int o = p * g.PSb;
     if (SPILL && p >= pl.n_sm)
-      update_strip<R, EXACT, RAGGED, D, true, true, CL>(
-          gn, h, pl.gl + (size_t)p * g.PSb, 0, out, 0, st, g, halo, dt, min_conc, mx);
+      update_strip<R, EXACT, RAGGED, D, true, true, CL>(gn, h, pl.gl, o, pl.gl_out, o, st, g, halo,
+                                                        dt, min_conc, mx);
     else
       update_strip<R, EXACT, RAGGED, D, false, BAND, CL>(
-          gn, h, nullptr, pl.sm + p * g.PSb, out, BAND ? 0 : pl.sm_out + p * g.PSb, st, g, halo, dt,
-          min_conc, mx);
+          gn, h, nullptr, pl.sm + o, pl.gl_out, BAND ? p * pl.out_stride : pl.sm_out + o, st, g,
+          halo, dt, min_conc, mx);
   };
   if (ctl & 16) update(True{});
   else update(False{});
@@ -845,6 +851,53 @@ __device__ __forceinline__ double cell_sum(int cells, F term, double *dred, int 
   return s;
 }
 
+// ---- steps without a block barrier ----------------------------------------
+//
+// A chunk's step s needs, of the step before, only the chunks within one row
+// above and below it (and those chunks' own earlier reads, which the same
+// counts cover, before it overwrites the older buffer).  So where no step's
+// maximum has to be known before the next step, a warp waits for its
+// neighbours' counts instead of a block barrier, and warps drift apart by up
+// to a step per chunk: their loads, MUFU bursts and waits overlap.
+// Measured with the barrier and without (G cell-updates/s): 64 x 64 198 and
+// 219.  Testing every step's maximum one step late, so that models with an
+// early-exit threshold could run the same way, took more than the barrier
+// (202; 51 x 37 with early exit 100 -> 94), so those keep it.
+struct StepSync {
+  int *done;           // [chunk] finished work: gene parts (owned chunks) or
+                       // genes (walked ones), since the experiment began
+  volatile int *fail;  // a wait ran out
+};
+
+// Waits until *p >= target in every lane (own p); false, and *fail set, after
+// about a second or once another warp has given up.
+__device__ __forceinline__ bool wait_counts(const int *p, int target, volatile int *fail) {
+  const uint32_t a = smem_addr(p);
+  for (uint32_t i = 0; i < (1u << 24); ++i) {
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    if (__all_sync(kFull, v >= target)) {
+      __syncwarp();
+      return true;
+    }
+    if ((i & 1023u) == 1023u && *fail) return false;
+  }
+  *fail = 1;
+  return false;
+}
+
+// Chunk c's step reads cells of the chunks c - reach .. c + reach.
+__device__ __forceinline__ int chunk_reach(const Geom &g) { return (g.Wg + 31) / 32; }
+
+// `work` of a step on chunk c is finished.
+__device__ __forceinline__ void finish_chunk(const StepSync &y, int c, int work, int lane) {
+  __syncwarp();
+  if (lane == 0)
+    asm volatile("red.release.cta.shared::cta.add.u32 [%0], %1;" ::"r"(smem_addr(y.done + c)),
+                 "r"(work)
+                 : "memory");
+}
+
 // Where a model's state lives during one step: genes p < n_sm are double
 // buffered in shared-memory planes p and p + n_sm; the others in the
 // block's global slot, planes p and p + gmax.  `par` selects the buffer
@@ -867,7 +920,7 @@ __device__ __forceinline__ Planes planes_of(const StatePtrs &sp, const Geom &g, 
   const size_t gl_half = (size_t)sp.gmax * g.PSb;
   char *gl = reinterpret_cast<char *>(sp.gl);
   return Planes{opaque(par ? half : 0),   opaque(par ? 0 : half), gl + (par ? gl_half : 0),
-                gl + (par ? 0 : gl_half), (size_t)g.PSb,          sp.n_sm};
+                gl + (par ? 0 : gl_half), 0,                      sp.n_sm};
 }
 
 // Genes first, first + splits, .. of the program for one strip.
@@ -882,10 +935,12 @@ __device__ __forceinline__ void strip_step(const ProgSmem &P, const Planes &pl, 
 }
 
 // A warp's range of walked items, of the first `chunks` chunks.
-template <int R, bool EXACT, bool RAGGED, bool SPILL, bool BAND, bool CL>
-__device__ __forceinline__ void walk_step(const ProgSmem &P, const Planes &pl, int G,
+// SYNC: waits for the neighbouring chunks' step s - 1 (false if that fails).
+template <int R, bool EXACT, bool RAGGED, bool SPILL, bool BAND, bool CL, bool SYNC>
+__device__ __forceinline__ bool walk_step(const ProgSmem &P, const Planes &pl, int G,
                                           const Geom &g, const Halo &halo, int chunks, int warp,
-                                          int lane, float dt, float min_conc, float &mx) {
+                                          int lane, float dt, float min_conc, float &mx,
+                                          const StepSync &sync, int s) {
   const int end = uniform(P.start[warp + 1]);
   int at = uniform(P.start[warp]);
 #pragma unroll 1
@@ -893,34 +948,51 @@ __device__ __forceinline__ void walk_step(const ProgSmem &P, const Planes &pl, i
     const int chunk = at >> 4;
     const Strip<R> st = strip_at<R>(chunk * 32 + lane, g);
     const int stop = (end >> 4) == chunk ? end & 15 : G;
+    if constexpr (SYNC) {
+      const int lo = max(chunk - chunk_reach(g), 0);
+      const int hi = min(chunk + chunk_reach(g), chunks - 1);
+      if (s > 1 && !wait_counts(sync.done + min(lo + lane, hi), G * (s - 1), sync.fail))
+        return false;
+    }
 #pragma unroll 1
     for (int k = at & 15; k < stop; ++k)
       gene_step<R, EXACT, RAGGED, SPILL, BAND, CL>(P, k, pl, st, g, halo, dt, min_conc, mx);
+    if constexpr (SYNC) finish_chunk(sync, chunk, stop - (at & 15), lane);
     at = (chunk + 1) << 4;
   }
+  return true;
 }
 
-// One step of the whole block by the model's class: all planes in shared
+// One step of the warp's work by the model's class: all planes in shared
 // memory or some in the global slot; the exact path always takes the general
 // form.
-template <int R, bool LOOP, bool RAGGED, bool CL>
-__device__ __forceinline__ void block_step(bool exact, const ProgSmem &P, const StatePtrs &sp,
+template <int R, bool LOOP, bool RAGGED, bool CL, bool SYNC>
+__device__ __forceinline__ bool block_step(bool exact, const ProgSmem &P, const StatePtrs &sp,
                                            int G, const Geom &g, const Strip<R> &st,
-                                           const Halo &halo, int first, int splits, int chunks,
-                                           int warp, int lane, int par, float dt, float min_conc,
-                                           float &mx) {
+                                           const Halo &halo, int own, int first, int splits,
+                                           int chunks, int warp, int lane, int par, float dt,
+                                           float min_conc, float &mx, const StepSync &sync,
+                                           int s) {
   const Planes pl = planes_of(sp, g, par);
+  bool ok = true;
+  if constexpr (SYNC && !LOOP) {
+    const int lo = max(own - chunk_reach(g), 0), hi = min(own + chunk_reach(g), chunks - 1);
+    if (s > 1 && !wait_counts(sync.done + min(lo + lane, hi), splits * (s - 1), sync.fail))
+      return false;
+  }
   const auto run = [&](auto e, auto spill) {
     constexpr bool E = decltype(e)::value, S = decltype(spill)::value;
     if constexpr (LOOP)
-      walk_step<R, E, RAGGED, S, false, CL>(P, pl, G, g, halo, chunks, warp, lane, dt, min_conc,
-                                            mx);
+      ok = walk_step<R, E, RAGGED, S, false, CL, SYNC>(P, pl, G, g, halo, chunks, warp, lane, dt,
+                                                       min_conc, mx, sync, s);
     else
       strip_step<R, E, RAGGED, S, CL>(P, pl, G, g, st, halo, first, splits, dt, min_conc, mx);
   };
   if (exact) run(True{}, True{});
   else if (sp.n_sm < G) run(False{}, True{});
   else run(False{}, False{});
+  if constexpr (SYNC && !LOOP) finish_chunk(sync, own, 1, lane);
+  return ok;
 }
 
 // ---- streaming schedule -------------------------------------------------
@@ -945,14 +1017,14 @@ __device__ __forceinline__ void band_step(bool exact, const ProgSmem &P, const f
   const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const Planes pl{(int)(reinterpret_cast<const unsigned char *>(stage) - grn_dyn_smem) -
                       (int)kStateOffset,
-                  0, nullptr, reinterpret_cast<char *>(out), gps * sizeof(float), G};
+                  0, nullptr, reinterpret_cast<char *>(out), (int)(gps * sizeof(float)), G};
   const int chunks = (gb.Q + 31) / 32;
   if (exact)
-    walk_step<R, true, RAGGED, false, true, false>(P, pl, G, gb, Halo{}, chunks, warp, lane, dt,
-                                                   min_conc, mx);
+    walk_step<R, true, RAGGED, false, true, false, false>(P, pl, G, gb, Halo{}, chunks, warp, lane,
+                                                          dt, min_conc, mx, StepSync{}, 0);
   else
-    walk_step<R, false, RAGGED, false, true, false>(P, pl, G, gb, Halo{}, chunks, warp, lane, dt,
-                                                    min_conc, mx);
+    walk_step<R, false, RAGGED, false, true, false, false>(P, pl, G, gb, Halo{}, chunks, warp, lane,
+                                                           dt, min_conc, mx, StepSync{}, 0);
 }
 
 // One Euler step of the streaming schedule.  Stages alternate by band; the
@@ -1193,6 +1265,9 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
   float *s_cmax = reinterpret_cast<float *>(smem + kCmaxOffset);
   double *s_csum = reinterpret_cast<double *>(smem + kCsumOffset);
 
+  // Owned chunks step without a block barrier where they can (walked ones lose
+  // by it: 100 x 100 147 G cell-updates/s with the barrier, 138 without).
+  constexpr bool FREE = !LOOP && !CL && !TRACE && ST == 0;
   const int NT = blockDim.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = uniform(tid >> 5), n_warps = NT >> 5;
   int rank = 0, C = 1;
@@ -1239,12 +1314,14 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kMbarOffset);
   volatile int *s_stream_fail = reinterpret_cast<volatile int *>(smem + kStreamFailOffset);
   uint32_t mphase = 0;  // streaming: next wait parity of each stage
+  int *s_done = reinterpret_cast<int *>(smem + kDoneOffset);
+  volatile int *s_fail = s_stream_fail;
+  if (tid == 0) *s_fail = 0;  // barriers follow before its first use
   if constexpr (ST) {
     if (tid == 0) {
       mbar_init(bars, 1);
       mbar_init(bars + 1, 1);
       mbar_init_fence();
-      *s_stream_fail = 0;
     }
     __syncthreads();
   }
@@ -1267,8 +1344,9 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
   Strip<kStripRows> fixed;
   int fixed_part = 0;
   const int splits = LOOP ? 0 : max(1, n_warps / chunks);
+  const int own = warp % chunks;
   if constexpr (!LOOP) {
-    fixed = strip_at<kStripRows>((warp % chunks) * 32 + lane, g);
+    fixed = strip_at<kStripRows>(own * 32 + lane, g);
     fixed_part = warp / chunks;
     if (fixed_part >= splits) fixed_part = GRN_MAX_GENES;  // no work
   }
@@ -1342,6 +1420,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
       // buffer's cells are all written by the first step.  A band's halo rows
       // start as the neighbouring grid rows.
       const float *init = A.initial + (size_t)e * A.n_in * A.W * A.H;
+      for (int i = tid; i < kMaxDone; i += NT) s_done[i] = 0;
       zero_floats(sp.sm, 2 * sp.n_sm * g.PS);
       if (sp.n_sm < G) {
         zero_floats(sp.gl + (size_t)sp.n_sm * g.PS, (G - sp.n_sm) * g.PS);
@@ -1387,6 +1466,42 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
       float change = 1.0f;
       int step = 0;
       int par = 0;  // buffer holding the current values
+      if constexpr (FREE) {
+        // Fast models that stop early only on a change of exactly 0: every
+        // rate is then 0 and the state stays as it is, so the steps after it
+        // change nothing, and the last step with a rate tells when it was.
+        if (!exact && A.change_bound <= 0.0f && A.n_steps > 0 && chunks <= kMaxDone &&
+            min(chunks, 2 * chunk_reach(g) + 1) <= 32) {
+          const StepSync sync{s_done, s_fail};
+          float mx = 0.0f;
+          int last = 0;  // steps up to the warp's last one with a rate
+          if (LOOP || fixed_part < splits) {
+            for (int s = 1; s <= A.n_steps; ++s) {
+              mx = 0.0f;
+              if (!block_step<kStripRows, LOOP, RAGGED, CL, true>(
+                      false, P, sp, G, g, fixed, halo, own, fixed_part, splits, chunks, warp, lane,
+                      (s - 1) & 1, dt, min_conc, mx, sync, s))
+                break;
+              if (__any_sync(kFull, mx > 0.0f)) last = s;
+            }
+          }
+          step = A.n_steps;
+          par = step & 1;
+          change = block_max(mx, s_red, 0, lane, warp, n_warps);
+          last = __float_as_int(block_max(__int_as_float(last), s_red, 1, lane, warp, n_warps));
+          if (*s_fail) {
+            if (tid == 0) {
+              atomicExch(A.error_flag, 4);
+              A.raw_error[orig] = __longlong_as_double(0x7ff8000000000000ll);
+            }
+            return;  // every thread of the block: read after the barriers
+          }
+          if (A.change_bound == 0.0f && last < step) {
+            step = last + 1;
+            change = 0.0f;
+          }
+        }
+      }
       while (step < A.n_steps && change > A.change_bound) {
         float mx = 0.0f;
         int adv = 1;  // Euler steps this iteration advanced
@@ -1418,9 +1533,9 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
             return;  // every thread of the block: the decision is block-uniform
           }
         } else {
-          block_step<kStripRows, LOOP, RAGGED, CL>(exact, P, sp, G, g, fixed, halo, fixed_part,
-                                                   splits, chunks, warp, lane, par, dt, min_conc,
-                                                   mx);
+          block_step<kStripRows, LOOP, RAGGED, CL, false>(exact, P, sp, G, g, fixed, halo, own,
+                                                          fixed_part, splits, chunks, warp, lane,
+                                                          par, dt, min_conc, mx, StepSync{}, 0);
         }
         if constexpr (CL)  // also orders the halo rows stored by this step
           change = cluster_max(mx, s_cmax + par * kMaxCluster * 32, rank, C, lane, warp, n_warps);

@@ -119,11 +119,13 @@ grn_status fail(grn_ctx *ctx, grn_status s, const std::string &msg) {
 
 // The kernel's error flag: 1 a model record it cannot run, 2 a bounded
 // wait for a bulk copy that ran out (streaming schedule), 3 a state access
-// outside its buffer (bounds-checked build only).
+// outside its buffer (bounds-checked build only), 4 a bounded wait for a
+// neighbouring warp's step that ran out.
 grn_status kernel_flag_error(grn_ctx *ctx, int32_t flag) {
   return fail(ctx, GRN_ERR_KERNEL,
               flag == 3   ? "bounds check: a simulation kernel state access fell outside its buffer"
               : flag == 2 ? "the simulation kernel's wait for a bulk copy timed out"
+              : flag == 4 ? "the simulation kernel's wait for a neighbouring warp timed out"
                           : "the simulation kernel rejected a model record");
 }
 
