@@ -214,20 +214,21 @@ constexpr size_t kRedOffset = kProgOffset + sizeof(ProgSmem);  // float [2][32]
 constexpr size_t kDredOffset = kRedOffset + 2 * 32 * 4;  // double [32]
 constexpr size_t kWorkOffset = kDredOffset + 32 * 8;     // int [2]
 // Cluster exchange slots: step maxima float [2][kMaxCluster][32] (by step
-// parity, CTA and warp) and per-CTA fitness sums double [kMaxCluster].
+// parity, CTA and warp; the fitness sums' lanes between the steps) and the
+// fitness sum double.
 constexpr size_t kCmaxOffset = kWorkOffset + 16;
 constexpr size_t kCsumOffset = kCmaxOffset + 2 * kMaxCluster * 32 * 4;
 // Two mbarriers of the streaming schedule's copy stages, then its copy
 // time-out flag (int).
-constexpr size_t kMbarOffset = (kCsumOffset + kMaxCluster * 8 + 15) & ~size_t(15);
+constexpr size_t kMbarOffset = (kCsumOffset + 8 + 15) & ~size_t(15);
 constexpr size_t kStreamFailOffset = kMbarOffset + 16;
 // Bounds-checked build only: the regions that state accesses are checked
 // against (CheckRegions).
-// Steps without a block barrier (StepSync): finished work per chunk (int
-// [kMaxDone]).
-constexpr int kMaxDone = 128;
+// Steps without a block barrier (StepSync): finished work per chunk (int [32])
+// and the halo counts (int [2]).
+constexpr int kMaxDone = 32;
 constexpr size_t kDoneOffset = kStreamFailOffset + 16;
-constexpr size_t kCheckOffset = (kDoneOffset + kMaxDone * 4 + 15) & ~size_t(15);
+constexpr size_t kCheckOffset = (kDoneOffset + (kMaxDone + 2) * 4 + 15) & ~size_t(15);
 constexpr size_t kCheckBytes = GRN_BOUNDS_CHECK ? 64 : 0;
 constexpr size_t kStateOffset = (kCheckOffset + kCheckBytes + 127) & ~size_t(127);
 
@@ -827,24 +828,32 @@ __device__ __forceinline__ float block_max(float v, float *red, int parity, int 
   return published_max(red, parity, lane, n_warps);
 }
 
-// The experiment's fitness sum over the block's cells (simstate.cpp:135-158)
+// The experiment's fitness sum over the grid's cells (simstate.cpp:135-158)
 // in FP64.  Cell i belongs to lane i % 32 of virtual warp (i / 32) %
-// kSumWarps, whatever the block size, and the virtual warps' sums are added
-// in order, so every schedule and block size gives the same bits.  Every
-// thread gets the sum.
+// kSumWarps, whatever the block size, a virtual lane adds its cells in order,
+// and the virtual warps' sums are added in order, so every schedule, block and
+// cluster size gives the same bits.
 constexpr int kSumWarps = 16;
+constexpr int kSumLanes = kSumWarps * 32;
+static_assert(kSumLanes * 8 <= 2 * kMaxCluster * 32 * 4 && kCmaxOffset % 8 == 0, "lane sums fit");
 
+// A virtual lane's sum v continued over the cells first .. end - 1.
 template <typename F>
-__device__ __forceinline__ double cell_sum(int cells, F term, double *dred, int lane, int warp,
-                                           int n_warps) {
-  for (int vw = warp; vw < kSumWarps; vw += n_warps) {
-    double v = 0.0;
-    for (int i = vw * 32 + lane; i < cells; i += kSumWarps * 32) v = term(i, v);
+__device__ __forceinline__ double lane_sum(double v, int slot, int first, int end, F term) {
+  const int d = (slot - first) & (kSumLanes - 1);
+  for (int i = first + d; i < end; i += kSumLanes) v = term(i, v);
+  return v;
+}
+
+// The virtual lanes' sums of virtual warp vw into dred[vw].
+__device__ __forceinline__ void warp_sum(double v, double *dred, int vw, int lane) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFull, v, o);
-    if (lane == 0) dred[vw] = v;
-  }
-  __syncthreads();
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFull, v, o);
+  if (lane == 0) dred[vw] = v;
+}
+
+// The whole sum, in every thread of the block (after a barrier).
+__device__ __forceinline__ double total_sum(const double *dred) {
   double s = 0.0;
 #pragma unroll
   for (int w = 0; w < kSumWarps; ++w) s += dred[w];
@@ -863,39 +872,64 @@ __device__ __forceinline__ double cell_sum(int cells, F term, double *dred, int 
 // 219.  Testing every step's maximum one step late, so that models with an
 // early-exit threshold could run the same way, took more than the barrier
 // (202; 51 x 37 with early exit 100 -> 94), so those keep it.
+//
+// A cluster's CTAs step the same way: a warp that has stored edge rows into a
+// neighbouring CTA's halo adds to that CTA's halo count, and a warp whose
+// chunk reads a halo row also waits for it, so no cluster barrier is passed
+// until the experiment ends (100 x 100 on 2 CTAs per model: 136 -> 152 G
+// cell-updates/s; one such model on 8 CTAs 1.23 -> 1.08 ms for 500 steps).
 struct StepSync {
-  int *done;           // [chunk] finished work: gene parts (owned chunks) or
-                       // genes (walked ones), since the experiment began
+  int *done;           // [chunk] gene parts finished since the experiment began
   volatile int *fail;  // a wait ran out
+  const int *wait;     // the count this lane waits for: a chunk's, or the halo
+                       // count of the CTA above (lane 30) or below (lane 31)
+  int per_step;        // what it grows by in a step
+  bool edge;           // the warp waits for a halo count (cluster scope)
+  uint32_t up, down;   // cluster addresses of the neighbours' halo counts that
+                       // this warp adds to (0: none)
 };
 
-// Waits until *p >= target in every lane (own p); false, and *fail set, after
-// about a second or once another warp has given up.
-__device__ __forceinline__ bool wait_counts(const int *p, int target, volatile int *fail) {
-  const uint32_t a = smem_addr(p);
+// Waits until this lane's count has reached `steps` steps, in every lane;
+// false, and *fail set, after about a second or once another warp has given
+// up.
+template <bool CL>
+__device__ __forceinline__ bool wait_counts(const StepSync &y, int steps) {
+  const uint32_t a = smem_addr(y.wait);
+  const int target = y.per_step * steps;
   for (uint32_t i = 0; i < (1u << 24); ++i) {
     int v;
-    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    if (CL && y.edge)
+      asm volatile("ld.acquire.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    else
+      asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     if (__all_sync(kFull, v >= target)) {
       __syncwarp();
       return true;
     }
-    if ((i & 1023u) == 1023u && *fail) return false;
+    if ((i & 1023u) == 1023u && *y.fail) return false;
   }
-  *fail = 1;
+  *y.fail = 1;
   return false;
 }
 
 // Chunk c's step reads cells of the chunks c - reach .. c + reach.
 __device__ __forceinline__ int chunk_reach(const Geom &g) { return (g.Wg + 31) / 32; }
 
-// `work` of a step on chunk c is finished.
-__device__ __forceinline__ void finish_chunk(const StepSync &y, int c, int work, int lane) {
+// The warp's part of a step on chunk c is finished.
+template <bool CL>
+__device__ __forceinline__ void finish_chunk(const StepSync &y, int c, int lane) {
   __syncwarp();
-  if (lane == 0)
-    asm volatile("red.release.cta.shared::cta.add.u32 [%0], %1;" ::"r"(smem_addr(y.done + c)),
-                 "r"(work)
+  if (lane == 0) {
+    asm volatile("red.release.cta.shared::cta.add.u32 [%0], 1;" ::"r"(smem_addr(y.done + c))
                  : "memory");
+    if constexpr (CL) {
+      if (y.up)
+        asm volatile("red.release.cluster.shared::cluster.add.u32 [%0], 1;" ::"r"(y.up) : "memory");
+      if (y.down)
+        asm volatile("red.release.cluster.shared::cluster.add.u32 [%0], 1;" ::"r"(y.down)
+                     : "memory");
+    }
+  }
 }
 
 // Where a model's state lives during one step: genes p < n_sm are double
@@ -935,12 +969,10 @@ __device__ __forceinline__ void strip_step(const ProgSmem &P, const Planes &pl, 
 }
 
 // A warp's range of walked items, of the first `chunks` chunks.
-// SYNC: waits for the neighbouring chunks' step s - 1 (false if that fails).
-template <int R, bool EXACT, bool RAGGED, bool SPILL, bool BAND, bool CL, bool SYNC>
-__device__ __forceinline__ bool walk_step(const ProgSmem &P, const Planes &pl, int G,
+template <int R, bool EXACT, bool RAGGED, bool SPILL, bool BAND, bool CL>
+__device__ __forceinline__ void walk_step(const ProgSmem &P, const Planes &pl, int G,
                                           const Geom &g, const Halo &halo, int chunks, int warp,
-                                          int lane, float dt, float min_conc, float &mx,
-                                          const StepSync &sync, int s) {
+                                          int lane, float dt, float min_conc, float &mx) {
   const int end = uniform(P.start[warp + 1]);
   int at = uniform(P.start[warp]);
 #pragma unroll 1
@@ -948,24 +980,17 @@ __device__ __forceinline__ bool walk_step(const ProgSmem &P, const Planes &pl, i
     const int chunk = at >> 4;
     const Strip<R> st = strip_at<R>(chunk * 32 + lane, g);
     const int stop = (end >> 4) == chunk ? end & 15 : G;
-    if constexpr (SYNC) {
-      const int lo = max(chunk - chunk_reach(g), 0);
-      const int hi = min(chunk + chunk_reach(g), chunks - 1);
-      if (s > 1 && !wait_counts(sync.done + min(lo + lane, hi), G * (s - 1), sync.fail))
-        return false;
-    }
 #pragma unroll 1
     for (int k = at & 15; k < stop; ++k)
       gene_step<R, EXACT, RAGGED, SPILL, BAND, CL>(P, k, pl, st, g, halo, dt, min_conc, mx);
-    if constexpr (SYNC) finish_chunk(sync, chunk, stop - (at & 15), lane);
     at = (chunk + 1) << 4;
   }
-  return true;
 }
 
 // One step of the warp's work by the model's class: all planes in shared
 // memory or some in the global slot; the exact path always takes the general
-// form.
+// form.  SYNC (owned chunks): between the waits of step s and its counts;
+// false if a wait ran out.
 template <int R, bool LOOP, bool RAGGED, bool CL, bool SYNC>
 __device__ __forceinline__ bool block_step(bool exact, const ProgSmem &P, const StatePtrs &sp,
                                            int G, const Geom &g, const Strip<R> &st,
@@ -974,25 +999,22 @@ __device__ __forceinline__ bool block_step(bool exact, const ProgSmem &P, const 
                                            float min_conc, float &mx, const StepSync &sync,
                                            int s) {
   const Planes pl = planes_of(sp, g, par);
-  bool ok = true;
-  if constexpr (SYNC && !LOOP) {
-    const int lo = max(own - chunk_reach(g), 0), hi = min(own + chunk_reach(g), chunks - 1);
-    if (s > 1 && !wait_counts(sync.done + min(lo + lane, hi), splits * (s - 1), sync.fail))
-      return false;
+  if constexpr (SYNC) {
+    if (s > 1 && !wait_counts<CL>(sync, s - 1)) return false;
   }
   const auto run = [&](auto e, auto spill) {
     constexpr bool E = decltype(e)::value, S = decltype(spill)::value;
     if constexpr (LOOP)
-      ok = walk_step<R, E, RAGGED, S, false, CL, SYNC>(P, pl, G, g, halo, chunks, warp, lane, dt,
-                                                       min_conc, mx, sync, s);
+      walk_step<R, E, RAGGED, S, false, CL>(P, pl, G, g, halo, chunks, warp, lane, dt, min_conc,
+                                            mx);
     else
       strip_step<R, E, RAGGED, S, CL>(P, pl, G, g, st, halo, first, splits, dt, min_conc, mx);
   };
   if (exact) run(True{}, True{});
   else if (sp.n_sm < G) run(False{}, True{});
   else run(False{}, False{});
-  if constexpr (SYNC && !LOOP) finish_chunk(sync, own, 1, lane);
-  return ok;
+  if constexpr (SYNC) finish_chunk<CL>(sync, own, lane);
+  return true;
 }
 
 // ---- streaming schedule -------------------------------------------------
@@ -1020,11 +1042,11 @@ __device__ __forceinline__ void band_step(bool exact, const ProgSmem &P, const f
                   0, nullptr, reinterpret_cast<char *>(out), (int)(gps * sizeof(float)), G};
   const int chunks = (gb.Q + 31) / 32;
   if (exact)
-    walk_step<R, true, RAGGED, false, true, false, false>(P, pl, G, gb, Halo{}, chunks, warp, lane,
-                                                          dt, min_conc, mx, StepSync{}, 0);
+    walk_step<R, true, RAGGED, false, true, false>(P, pl, G, gb, Halo{}, chunks, warp, lane, dt,
+                                                   min_conc, mx);
   else
-    walk_step<R, false, RAGGED, false, true, false, false>(P, pl, G, gb, Halo{}, chunks, warp, lane,
-                                                           dt, min_conc, mx, StepSync{}, 0);
+    walk_step<R, false, RAGGED, false, true, false>(P, pl, G, gb, Halo{}, chunks, warp, lane, dt,
+                                                    min_conc, mx);
 }
 
 // One Euler step of the streaming schedule.  Stages alternate by band; the
@@ -1210,16 +1232,6 @@ __device__ __forceinline__ void write_planes(const SimArgs &A, const StatePtrs &
   }
 }
 
-// Cluster-wide combine of one value per CTA: CTA `rank` stores v into slot
-// `rank` of every CTA's array, then the cluster barrier.  Every CTA then
-// reads the same C slots.
-template <typename T>
-__device__ __forceinline__ void cluster_share(T *slots, T v, int rank, int C) {
-  cg::cluster_group cl = cg::this_cluster();
-  if ((int)threadIdx.x < C) *cl.map_shared_rank(slots + rank, threadIdx.x) = v;
-  cl.sync();
-}
-
 // Max of a non-negative, non-NaN float over the cluster's CTAs with one
 // cluster barrier: every warp stores its max into slot [rank][warp] of every
 // CTA's array.  The barrier also orders the step's halo rows.
@@ -1267,7 +1279,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
 
   // Owned chunks step without a block barrier where they can (walked ones lose
   // by it: 100 x 100 147 G cell-updates/s with the barrier, 138 without).
-  constexpr bool FREE = !LOOP && !CL && !TRACE && ST == 0;
+  constexpr bool FREE = !LOOP && !TRACE && ST == 0;
   const int NT = blockDim.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = uniform(tid >> 5), n_warps = NT >> 5;
   int rank = 0, C = 1;
@@ -1351,6 +1363,34 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
     if (fixed_part >= splits) fixed_part = GRN_MAX_GENES;  // no work
   }
 
+  StepSync sync{s_done, s_fail, s_done, 0, false, 0, 0};
+  bool free_steps = false;  // the counts' lanes are enough for this grid
+  if constexpr (FREE) {
+    const int reach = chunk_reach(g);
+    free_steps = min(chunks, 2 * reach + 1) <= (CL ? 30 : 32) && chunks <= kMaxDone;
+    sync.wait = s_done + min(max(own - reach, 0) + lane, min(own + reach, chunks - 1));
+    sync.per_step = splits;
+    if constexpr (CL) {
+      // Chunks with a band's first row of strips, and with a full band's last.
+      const int Q = strip_count<kStripRows>(Hb, g.Wg);
+      const int n_first = (g.Wg + 31) / 32, n_last = (Q - 1) / 32 - (Q - g.Wg) / 32 + 1;
+      const bool first = rank > 0 && own < n_first;
+      const bool last = rank < C - 1 && own >= (Q - g.Wg) / 32 && own <= (Q - 1) / 32;
+      if (first && lane == 30) {
+        sync.wait = s_done + kMaxDone;
+        sync.per_step = n_last * splits;
+      }
+      if (last && lane == 31) {
+        sync.wait = s_done + kMaxDone + 1;
+        sync.per_step = n_first * splits;
+      }
+      sync.edge = first || last;
+      const uint32_t counts = smem_addr(s_done + kMaxDone);
+      if (first) sync.up = cluster_addr(counts + 4, rank - 1);
+      if (last) sync.down = cluster_addr(counts, rank + 1);
+    }
+  }
+
   for (int iter = 0;; ++iter) {
     int m;
     if constexpr (CL) {
@@ -1420,7 +1460,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
       // buffer's cells are all written by the first step.  A band's halo rows
       // start as the neighbouring grid rows.
       const float *init = A.initial + (size_t)e * A.n_in * A.W * A.H;
-      for (int i = tid; i < kMaxDone; i += NT) s_done[i] = 0;
+      for (int i = tid; i < kMaxDone + 2; i += NT) s_done[i] = 0;
       zero_floats(sp.sm, 2 * sp.n_sm * g.PS);
       if (sp.n_sm < G) {
         zero_floats(sp.gl + (size_t)sp.n_sm * g.PS, (G - sp.n_sm) * g.PS);
@@ -1470,31 +1510,37 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
         // Fast models that stop early only on a change of exactly 0: every
         // rate is then 0 and the state stays as it is, so the steps after it
         // change nothing, and the last step with a rate tells when it was.
-        if (!exact && A.change_bound <= 0.0f && A.n_steps > 0 && chunks <= kMaxDone &&
-            min(chunks, 2 * chunk_reach(g) + 1) <= 32) {
-          const StepSync sync{s_done, s_fail};
+        if (!exact && A.change_bound <= 0.0f && A.n_steps > 0 && free_steps) {
           float mx = 0.0f;
           int last = 0;  // steps up to the warp's last one with a rate
-          if (LOOP || fixed_part < splits) {
+          if (fixed_part < splits) {
             for (int s = 1; s <= A.n_steps; ++s) {
               mx = 0.0f;
               if (!block_step<kStripRows, LOOP, RAGGED, CL, true>(
                       false, P, sp, G, g, fixed, halo, own, fixed_part, splits, chunks, warp, lane,
-                      (s - 1) & 1, dt, min_conc, mx, sync, s))
+                      (s - 1) & 1, dt, min_conc, mx, sync, s)) {
+                last = 0x7fffffff;
                 break;
+              }
               if (__any_sync(kFull, mx > 0.0f)) last = s;
             }
           }
           step = A.n_steps;
           par = step & 1;
-          change = block_max(mx, s_red, 0, lane, warp, n_warps);
-          last = __float_as_int(block_max(__int_as_float(last), s_red, 1, lane, warp, n_warps));
-          if (*s_fail) {
+          if constexpr (CL) {
+            change = cluster_max(mx, s_cmax, rank, C, lane, warp, n_warps);
+            last = __float_as_int(cluster_max(__int_as_float(last), s_cmax + kMaxCluster * 32, rank,
+                                              C, lane, warp, n_warps));
+          } else {
+            change = block_max(mx, s_red, 0, lane, warp, n_warps);
+            last = __float_as_int(block_max(__int_as_float(last), s_red, 1, lane, warp, n_warps));
+          }
+          if (last == 0x7fffffff) {
             if (tid == 0) {
               atomicExch(A.error_flag, 4);
               A.raw_error[orig] = __longlong_as_double(0x7ff8000000000000ll);
             }
-            return;  // every thread of the block: read after the barriers
+            return;  // every thread of the block (the cluster): a shared value
           }
           if (A.change_bound == 0.0f && last < step) {
             step = last + 1;
@@ -1558,7 +1604,9 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
 
       // Fitness of the experiment (simstate.cpp:135-158), FP64 sums.
       const float *tgt = A.target + (size_t)e * A.n_target * A.W * A.H;
-      const auto term = [&](int i, double acc) {
+      const int cell0 = g.y0 * g.W;  // the band's first cell
+      const auto term = [&](int cell, double acc) {
+        const int i = cell - cell0;
         const int y = A.inv_w ? (int)__umulhi((uint32_t)i, A.inv_w) : i / g.W, x = i - y * g.W;
         for (int kk = 0; kk < A.n_target; ++kk) {
           const double a = *chk<1>(plane_of(sp, g, A.n_in + kk, par) + cell_offset(g, y, x));
@@ -1572,11 +1620,34 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
         }
         return acc;
       };
-      double dist = cell_sum(g.W * g.H, term, s_dred, lane, warp, n_warps);
+      const int cell1 = cell0 + g.H * g.W;
+      double dist = 0.0;
       if constexpr (CL) {
-        cluster_share(s_csum, dist, rank, C);
-        dist = 0.0;
-        for (int r = 0; r < C; ++r) dist += s_csum[r];
+        // The virtual lanes' sums go from band to band (in the slots of the
+        // step maxima, which nobody reads now), so that they add the cells in
+        // the order of one CTA.
+        double *s_acc = reinterpret_cast<double *>(s_cmax);
+        for (int r = 0; r < C; ++r) {
+          cg::this_cluster().sync();
+          if (rank != r) continue;
+          for (int vw = warp; vw < kSumWarps; vw += n_warps) {
+            const int slot = vw * 32 + lane;
+            const double v = lane_sum(r > 0 ? s_acc[slot] : 0.0, slot, cell0, cell1, term);
+            if (r < C - 1) *cg::this_cluster().map_shared_rank(s_acc + slot, r + 1) = v;
+            else warp_sum(v, s_dred, vw, lane);
+          }
+          if (r == C - 1) {
+            __syncthreads();
+            if (tid < C) *cg::this_cluster().map_shared_rank(s_csum, tid) = total_sum(s_dred);
+          }
+        }
+        cg::this_cluster().sync();
+        dist = s_csum[0];
+      } else {
+        for (int vw = warp; vw < kSumWarps; vw += n_warps)
+          warp_sum(lane_sum(0.0, vw * 32 + lane, cell0, cell1, term), s_dred, vw, lane);
+        __syncthreads();
+        dist = total_sum(s_dred);
       }
       if (A.fitness_kind == GRN_FITNESS_MSE)
         dist /= (double)g.W * g.Hg * A.n_target;

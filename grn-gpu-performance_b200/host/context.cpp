@@ -277,12 +277,12 @@ int stream2_rows(int W, int H, int genes, size_t room) {
 //   - a gene of a chunk takes about 98 cycles of an SM whose planes are in
 //     shared memory and which holds 28 warps or more; 12 warps take 1.12x, 8
 //     warps 1.46x, 4 warps 1.86x that (32 x 32 grids);
-//   - walked items 1.12x owned chunks, a cluster's chunks 1.15x;
+//   - walked items 1.12x owned chunks, a cluster's chunks 1.05x;
 //   - genes in global slots 1.35x while what the CTAs touch of them stays in
 //     L2 (100 x 100, walked, 2 of 4 genes spilled: 142 against 194), 1.8x
 //     past that (116 x 206: 111); staged bands 1.35x and two steps per pass
 //     1.7x (256 x 256, 8 genes, 24 links: staged 63, walked 43);
-//   - a step's barrier 300 cycles, a cluster's 1200 (2 CTAs) to 6100 (16).
+//   - a step's waits 300 cycles, a cluster's 700 (2 CTAs) to 3500 (16).
 double plan_cost(const grn_ctx *ctx, const LaunchPlan &p, int max_genes, int n_models,
                  double slot_bytes) {
   const int C = std::max(1, p.cluster);
@@ -300,10 +300,10 @@ double plan_cost(const grn_ctx *ctx, const LaunchPlan &p, int max_genes, int n_m
     const double spilled_max = std::max(0.0, 1.0 - (double)(p.planes / 2) / max_genes);
     const bool l2 = slot_bytes * genes / max_genes * p.blocks <= 8e7;
     f *= 1.0 + (l2 ? 0.35 : 0.8) * 0.5 * (spilled + spilled_max);
-    if (C > 1) f *= 1.15;
+    if (C > 1) f *= 1.05;
     else if (p.v.loop) f *= 1.12;
   }
-  const double sync = C == 1 ? 300 : 500 + 350 * C;
+  const double sync = C == 1 ? 300 : 300 + 200 * C;
   const double step = per_sm * chunks * genes * 98 * f + sync;
   return step * std::max(1.0, (double)n_models / resident);
 }
