@@ -139,7 +139,7 @@ extern "C" grn_status grn_evaluate_batch_noalloc(
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
   const int W = params->dim_x, H = params->dim_y;
   const bool ragged = (W % 4) != 0;
-  const size_t plane_bytes = (size_t)plane_floats(W, H) * sizeof(float);
+  const size_t plane_bytes = (size_t)plane_floats(W, H, 1, 0) * sizeof(float);
   const size_t fixed = sim_fixed_smem_bytes();
   int fit = (size_t)optin > fixed ? (int)(((size_t)optin - fixed) / plane_bytes) : 0;
   fit &= ~1;
@@ -170,7 +170,7 @@ extern "C" grn_status grn_evaluate_batch_noalloc(
       best.planes = planes;
       best.smem_bytes = smem;
       best.blocks_per_sm = occ;
-      best.slot_floats = planes / 2 < max_genes ? 2LL * gmax * plane_floats(W, H) : 0;
+      best.slot_floats = planes / 2 < max_genes ? 2LL * gmax * plane_floats(W, H, 1, 0) : 0;
     }
   }
   if (best_score < 0)
@@ -209,7 +209,7 @@ extern "C" grn_status grn_evaluate_batch_noalloc(
   a.n_exp = n_experiments;
   a.n_in = params->n_input_morphogens;
   a.n_target = params->n_target_morphogens;
-  set_geometry(&a, W, H, 1);
+  set_geometry(&a, W, H, 1, 0);
   a.gmax = best.gmax;
   a.n_steps = params->num_sim_steps;
   a.fitness_kind = params->fitness_kind;

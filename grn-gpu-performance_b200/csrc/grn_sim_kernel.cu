@@ -410,9 +410,9 @@ __device__ __forceinline__ void build_program(const ModelSmem &M, ProgSmem &P, i
 // A state plane holds the W x H grid as rows of RS = row_floats(W) floats
 // (whole float4 groups, ending in at least one zero cell) plus one zero row
 // above and one below, and rows for whole strips (strip_rows):
-// PS = (strip_rows(H) + 2) * RS floats, row y at (y + 1) * RS.  The zero rows
-// make the
-// up/down neighbours of the first and last rows read +0.0, which leaves the
+// PS = plane_floats, row y at row_offset(y + 1): `pad` zero floats follow the
+// row above the grid and then every two rows, i.e. every row of strips
+// (strip_pad; 0 where streamed).  The zero rows make the up/down neighbours of the first and last rows read +0.0, which leaves the
 // reference's neighbour sum unchanged.  Steps write data groups only; when W
 // is not a multiple of 4 the cells past W of a row's last group are written
 // as 0, otherwise a zero group ends the row: either way the cell after a
@@ -424,7 +424,8 @@ __device__ __forceinline__ void build_program(const ModelSmem &M, ProgSmem &P, i
 // step, or zero at the grid border).
 struct Geom {
   int W, H, Wg, RS, PS, Q;  // Q: strips of the band
-  int RSb, PSb;             // RS, PS in bytes
+  int pad;                  // floats after every two rows (0: streamed bands)
+  int RSb, PSb, SSb;        // RS, PS and a row of strips (R * RS + pad) in bytes
   bool edges;               // chunks do not hold whole rows of groups
   int y0, Hg;               // first grid row of the band, grid height
   uint32_t inv_wg;          // ceil(2^32 / Wg): q / Wg by multiplication
@@ -465,7 +466,7 @@ __device__ __forceinline__ Strip<R> strip_at(int q, const Geom &g) {
   s.rows = min(R, g.H - y);
   s.el = gx == 0 || (q & 31) == 0;
   s.er = gx == g.Wg - 1 || (q & 31) == 31;
-  s.base = 4 * ((y + 1) * g.RS + x0);
+  s.base = (ys + 1) * g.SSb - (R - 1) * g.RSb + 4 * x0;
   s.first = s.valid && y == 0 && g.y0 > 0;
   s.last = s.valid && y + R >= g.H && g.y0 + g.H < g.Hg;
   const int yg = y + g.y0;
@@ -486,7 +487,7 @@ __device__ __forceinline__ Strip<R> strip_at(int q, const Geom &g) {
 }
 
 __device__ __forceinline__ int cell_offset(const Geom &g, int y, int x) {
-  return (y + 1) * g.RS + x;
+  return (int)row_offset(y + 1, g.RS, g.pad) + x;
 }
 
 // ---- the step ------------------------------------------------------------
@@ -553,12 +554,12 @@ struct Planes {
 };
 
 // Where a band's edge rows also go: the halo rows of the neighbouring CTAs'
-// planes, `rows` bytes further down (up) than the row's own place, in their
-// shared memory (cluster addresses of their state areas) or their global
-// slots (slot_bytes before and after this CTA's).
+// planes, up_rows bytes further down (down_rows bytes further up) than the
+// row's own place, in their shared memory (cluster addresses of their state
+// areas) or their global slots (slot_bytes before and after this CTA's).
 struct Halo {
   uint32_t up, down;
-  int rows;
+  int up_rows, down_rows;
   int64_t slot_bytes;
 };
 
@@ -704,8 +705,8 @@ __device__ __forceinline__ void update_strip(const GeneSmem &gn, const float4 (&
 #pragma unroll
   for (int i = 0; i < R; ++i) c[i + 1] = load4<SG>(src_gl, o + i * g.RSb);
   if constexpr (DIFFUSES) {
-    c[0] = load4<SG>(src_gl, o - g.RSb);
-    c[R + 1] = load4<SG>(src_gl, o + R * g.RSb);
+    c[0] = load4<SG>(src_gl, o + (R - 1) * g.RSb - g.SSb);
+    c[R + 1] = load4<SG>(src_gl, o + g.SSb);
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const float l = __shfl_up_sync(kFull, c[i + 1].w, 1);
@@ -773,9 +774,9 @@ __device__ __forceinline__ void update_strip(const GeneSmem &gn, const float4 (&
     }
     if constexpr (CL) {
       if (i == 0 && st.first)
-        halo_store<DG>(halo.up, dst_gl - halo.slot_bytes, row + halo.rows, nv);
+        halo_store<DG>(halo.up, dst_gl - halo.slot_bytes, row + halo.up_rows, nv);
       if (i == st.rows - 1 && st.last)
-        halo_store<DG>(halo.down, dst_gl + halo.slot_bytes, row - halo.rows, nv);
+        halo_store<DG>(halo.down, dst_gl + halo.slot_bytes, row - halo.down_rows, nv);
     }
   }
 }
@@ -1297,6 +1298,8 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
   g.RS = A.row_floats;
   g.PS = A.plane_floats;
   g.RSb = A.row_bytes;
+  g.pad = A.row_pad;
+  g.SSb = kStripRows * g.RSb + 4 * g.pad;
   g.edges = 32 % g.Wg != 0;
   g.PSb = A.plane_bytes;
   g.Q = strip_count<kStripRows>(g.H, A.Wg);
@@ -1343,7 +1346,9 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
     const uint32_t state = smem_addr(smem + kStateOffset);
     if (rank > 0) halo.up = cluster_addr(state, rank - 1);
     if (rank < C - 1) halo.down = cluster_addr(state, rank + 1);
-    halo.rows = Hb * g.RSb;
+    // The first row (plane row 1) to plane row Hb + 1, the last one (Hb) to 0.
+    halo.up_rows = 4 * (int)(row_offset(Hb + 1, g.RS, g.pad) - row_offset(1, g.RS, g.pad));
+    halo.down_rows = 4 * (int)row_offset(Hb, g.RS, g.pad);
     halo.slot_bytes = A.slot_floats * (int64_t)sizeof(float);
   }
 
@@ -1474,7 +1479,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
           const int x0 = 4 * (i - rr * g.Wg), y = g.y0 - 1 + rr;  // grid row
           if (y < 0 || y >= g.Hg) continue;
           const float *src = init + ((size_t)kk * g.Hg + y) * g.W + x0;
-          float *dst = chk<4>(pl + rr * g.RS + x0);
+          float *dst = chk<4>(pl + cell_offset(g, rr - 1, x0));
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             if (x0 + j < g.W) dst[j] = src[j];

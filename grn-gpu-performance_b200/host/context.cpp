@@ -334,7 +334,7 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
       const int own = v.stream == 2 ? GRN_SCHEDULE_STREAM2 : GRN_SCHEDULE_STREAM;
       if (sched != GRN_SCHEDULE_AUTO && sched != own) continue;
       if (ft && ft != v.max_threads) continue;
-      const size_t plane_bytes = (size_t)grn::plane_floats(W, H) * sizeof(float);
+      const size_t plane_bytes = (size_t)grn::plane_floats(W, H, 1, 0) * sizeof(float);
       const int fit = optin > fixed ? (int)((optin - fixed) / plane_bytes) & ~1 : 0;
       if (sched == GRN_SCHEDULE_AUTO && fit / 2 >= max_genes) continue;
       const size_t room = optin > fixed ? optin - fixed : 0;
@@ -349,7 +349,7 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
       if (ctas < 1) continue;
       plan.schedule = own;
       plan.threads = v.max_threads;
-      plan.slot_floats = 2LL * max_genes * grn::plane_floats(W, H);
+      plan.slot_floats = 2LL * max_genes * grn::plane_floats(W, H, 1, 0);
       plan.cluster = 1;
       plan.band_rows = R;
       plan.blocks = std::max(1, std::min(n_models, ctas));
@@ -367,16 +367,23 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
       const int Hb = (H + C - 1) / C;
       if (C > 1 && (C - 1) * Hb >= H) continue;  // every band non-empty
       const int chunks = grn::strip_chunks(W, Hb);
-      const size_t plane_bytes = (size_t)grn::plane_floats(W, H, C) * sizeof(float);
-      int fit = optin > fixed ? (int)((optin - fixed) / plane_bytes) : 0;
-      fit &= ~1;
-      const int smem_planes = std::min(fit, 2 * max_genes);
+      // Planes of padded rows of strips (strip_pad) where they keep as many
+      // genes on chip as unpadded ones and cost no resident CTA (below).
+      const auto plane_size = [&](int pad) {
+        return (size_t)grn::plane_floats(W, H, C, pad) * sizeof(float);
+      };
+      const auto planes_of = [&](int pad) {
+        const int fit = optin > fixed ? (int)((optin - fixed) / plane_size(pad)) & ~1 : 0;
+        return std::min(fit, 2 * max_genes);
+      };
+      const int smem_planes = planes_of(0);
+      const int pad = planes_of(grn::strip_pad(W)) == smem_planes ? grn::strip_pad(W) : 0;
       if (C > 1 && sched == GRN_SCHEDULE_AUTO) {
         // A cluster pays where it keeps more genes on chip, or where models
         // are fewer than SMs.
         const int fit1 =
             optin > fixed
-                ? (int)((optin - fixed) / ((size_t)grn::plane_floats(W, H) * sizeof(float))) & ~1
+                ? (int)((optin - fixed) / ((size_t)grn::plane_floats(W, H, 1, 0) * sizeof(float))) & ~1
                 : 0;
         if (fit1 >= 2 * max_genes && 2 * n_models > ctx->n_sm) continue;
         if (C > 4 && C * n_models > ctx->n_sm) continue;
@@ -406,29 +413,40 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
         for (int gv = 0; gv < (offer_global ? 2 : 1); ++gv) {
           plan.planes = (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? 0 : smem_planes;
           const bool spills = plan.planes / 2 < max_genes;
-          plan.smem_bytes = fixed + plan.planes * plane_bytes;
+          const auto resident = [&](int p, int *ctas) -> grn_status {
+            plan.row_pad = p;
+            plan.smem_bytes = fixed + plan.planes * plane_size(p);
+            if (C == 1) {
+              GRN_CUDA(ctx, grn::sim_occupancy(v, threads, plan.smem_bytes, &plan.blocks_per_sm));
+              *ctas = plan.blocks_per_sm * ctx->n_sm;
+            } else {
+              int clusters = 0;
+              GRN_CUDA(ctx, grn::sim_cluster_occupancy(v, threads, plan.smem_bytes, C, &clusters));
+              *ctas = clusters * C;
+              plan.blocks_per_sm = 1;
+            }
+            return GRN_OK;
+          };
           int ctas = 0;  // resident CTAs on the device
-          if (C == 1) {
-            GRN_CUDA(ctx, grn::sim_occupancy(v, threads, plan.smem_bytes, &plan.blocks_per_sm));
-            ctas = plan.blocks_per_sm * ctx->n_sm;
-          } else {
-            int clusters = 0;
-            GRN_CUDA(ctx, grn::sim_cluster_occupancy(v, threads, plan.smem_bytes, C, &clusters));
-            ctas = clusters * C;
-            plan.blocks_per_sm = 1;
+          grn_status s = resident(0, &ctas);
+          if (s == GRN_OK && plan.planes > 0 && pad > 0) {
+            int padded = 0;
+            s = resident(pad, &padded);
+            if (s == GRN_OK && padded < ctas) s = resident(0, &ctas);
           }
+          if (s != GRN_OK) return s;
           if (ctas < 1) continue;
           plan.schedule = C > 1                                      ? GRN_SCHEDULE_CLUSTER
                           : (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? GRN_SCHEDULE_GLOBAL
                           : v.loop                                    ? GRN_SCHEDULE_WALK_ITEMS
                                                                       : GRN_SCHEDULE_FIXED_ITEMS;
           plan.threads = threads;
-          plan.slot_floats = spills ? 2LL * max_genes * grn::plane_floats(W, H, C) : 0;
+          plan.slot_floats = spills ? 2LL * max_genes * grn::plane_floats(W, H, C, plan.row_pad) : 0;
           plan.cluster = C;
           plan.blocks = C > 1 ? C * std::max(1, std::min(n_models, ctas / C))
                               : std::max(1, std::min(n_models, ctas));
           out->push_back({plan_cost(ctx, plan, max_genes, n_models,
-                                    spills ? 2.0 * max_genes * plane_bytes : 0.0),
+                                    spills ? 2.0 * max_genes * plane_size(plan.row_pad) : 0.0),
                           plan});
         }
     }
@@ -461,7 +479,7 @@ bool same_plan(const LaunchPlan &a, const grn_ctx::Tuned &t) {
 // Sets the plan's state planes and global state slots in `a` (allocating
 // the slots if they grew).
 grn_status bind_state(grn_ctx *ctx, const LaunchPlan &plan, grn::SimArgs *a) {
-  grn::set_geometry(a, a->W, a->H, plan.cluster);
+  grn::set_geometry(a, a->W, a->H, plan.cluster, plan.row_pad);
   a->planes = plan.planes;
   a->gmax = plan.gmax;
   a->band_rows = plan.band_rows;
