@@ -1050,30 +1050,41 @@ __device__ __forceinline__ void band_step(bool exact, const ProgSmem &P, const f
                                                     min_conc, mx);
 }
 
-// One Euler step of the streaming schedule.  Stages alternate by band; the
-// copy of band b + 2 is issued (thread 0) once every thread has finished
-// band b.  mphase holds each stage's next wait parity across steps.
+// One Euler step of the streaming schedule.  Stages alternate by band.  The
+// warps pass no block barrier between bands: a warp goes on to the next band
+// once that band's copy has arrived, and the last warp to finish band b
+// issues the copy of band b + 2 into its stage.  Bound by issue slots and the
+// MUFU pipe (each about half busy) and by the waits for them, so warps help:
+// 256 x 256, 8 genes, 592 models x 100 steps, kernel ms with 16 warps and a
+// barrier per band 54.3, 20 warps 53.0, 20 warps without the barrier 50.4.
+// In a 50-step sample 16 warps took 1.10x as long without the barrier, 24
+// warps (72 registers, bands of 6 rows) 1.30x.
+// mphase holds each stage's
+// next wait parity across steps; `counts` are the stages' finished warps (0
+// between steps) and the copies issued for each in this step.
 // Returns false (the same in every thread) if a copy did not complete in
 // time; the copies still in flight have then been waited for (bounded).
-// A thread whose wait runs out raises *fail and computes its band from
-// whatever the stage holds; the band's one barrier then makes the decision
-// block-wide (the model's results are discarded on that path).  *fail is 0
-// on entry and is never cleared: the kernel returns after a failure.
+// A warp whose wait runs out raises *fail and leaves, as do the others at
+// their next wait; the barrier at the end makes the decision block-wide.
+// *fail is 0 on entry and is never cleared: the kernel returns after a
+// failure.
 template <bool RAGGED>
 __device__ bool stream_step(const SimArgs &A, const ProgSmem &P, const StatePtrs &sp,
                             const Geom &g, int G, int par, bool exact,
                             float dt, float min_conc, float &mx, uint64_t *bars,
-                            uint32_t &mphase, volatile int *fail, int R) {
+                            uint32_t &mphase, int *counts, volatile int *fail, int R) {
   const int nb = (g.H + R - 1) / R;
   const int SPS = (R + 2) * g.RS;
   float *stage0 = sp.sm;
   const size_t gps = (size_t)g.PS;
   const float *gl_cur = sp.gl + (par ? sp.gmax : 0) * gps;
   float *gl_nxt = sp.gl + (par ? 0 : sp.gmax) * gps;
+  volatile int *issued = counts + 2;
   auto issue = [&](int b) {
     float *st = stage0 + (b & 1) * sp.gmax * SPS;
     const int rows = min(R + 2, g.H + 2 - b * R);  // plane rows b*R .. b*R + rows - 1
     const uint32_t bytes = (uint32_t)rows * g.RS * 4u;
+    issued[b & 1] = b / 2 + 1;
     fence_proxy_async_shared();
     mbar_expect_tx(bars + (b & 1), bytes * (uint32_t)G);
     for (int p = 0; p < G; ++p) {
@@ -1085,13 +1096,16 @@ __device__ bool stream_step(const SimArgs &A, const ProgSmem &P, const StatePtrs
   // Test hook: withhold band 1's copy, so that its wait runs out.
   const bool withhold = A.test_hooks & kHookWithholdBandCopy;
   if (threadIdx.x == 0) {
+    issued[1] = 0;
     issue(0);
     if (nb > 1 && !withhold) issue(1);
   }
+  const uint32_t mphase0 = mphase;
   for (int b = 0; b < nb; ++b) {
     const int s = b & 1;
-    const uint32_t parity = (mphase >> s) & 1u;
-    if (!mbar_wait(bars + s, parity)) *fail = 1;
+    const bool arrived = mbar_wait(bars + s, (mphase >> s) & 1u);
+    if (!arrived) *fail = 1;
+    if (!__all_sync(kFull, arrived && !*fail)) break;
     mphase ^= 1u << s;
     Geom gb = g;
     gb.y0 = b * R;
@@ -1101,17 +1115,29 @@ __device__ bool stream_step(const SimArgs &A, const ProgSmem &P, const StatePtrs
     gb.Q = strip_count<kStripRows>(gb.H, g.Wg);
     band_step<kStripRows, RAGGED>(exact, P, stage0 + s * sp.gmax * SPS, G, gb,
                           gl_nxt + (size_t)gb.y0 * g.RS, gps, dt, min_conc, mx);
-    __syncthreads();  // stage s is free again; *fail is the same for every thread
-    if (*fail) {
-      // Bounded second waits for copies that may still be in flight: the
-      // timed-out one (unless withheld) and the one issued ahead.
-      if (!withhold) mbar_wait(bars + s, parity);
-      if (b + 1 < nb) mbar_wait(bars + (s ^ 1), (mphase >> (s ^ 1)) & 1u);
-      return false;
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+      // Releases this warp's reads of the stage; the last one acquires all.
+      int n;
+      asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;"
+                   : "=r"(n)
+                   : "r"(smem_addr(counts + s))
+                   : "memory");
+      if (n == (int)(blockDim.x >> 5) - 1) {
+        counts[s] = 0;
+        if (b + 2 < nb) issue(b + 2);
+      }
     }
-    if (threadIdx.x == 0 && b + 2 < nb) issue(b + 2);
+    __syncwarp();
   }
   fence_proxy_async_global();  // this step's writes before the next step's copies
+  __syncthreads();             // *fail is the same for every thread
+  if (*fail) {
+    // Bounded second waits for the copies that may still be in flight.
+    for (int s = 0; s < 2; ++s)
+      if (issued[s] > 0) mbar_wait(bars + s, ((mphase0 >> s) ^ (issued[s] - 1)) & 1u);
+    return false;
+  }
   return true;
 }
 
@@ -1575,7 +1601,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
           }
           if (ok && single)
             ok = stream_step<RAGGED>(A, P, sp, g, G, par, exact, dt, min_conc, mx, bars,
-                                         mphase, s_stream_fail, A.band_rows);
+                                         mphase, s_done, s_stream_fail, A.band_rows);
           if (!ok) {
             if (tid == 0) {
               atomicExch(A.error_flag, 2);
@@ -1692,9 +1718,9 @@ const VariantEntry kVariants[] = {
     // trace frames (one model at a time: any grid, any gene count)
     GRN_VARIANT(512, true, false, true, 0),
     // streaming (bands staged by bulk copies)
-    GRN_VARIANT(512, true, false, false, 1),
+    GRN_VARIANT(640, true, false, false, 1),
     // streaming with temporal blocking: two Euler steps per pass
-    GRN_VARIANT(512, true, false, false, 2),
+    GRN_VARIANT(640, true, false, false, 2),
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 

@@ -239,7 +239,7 @@ int stream_rows(int W, int H, int genes, size_t room, int threads) {
   if (r > 1 && r < H) r &= ~1L;
   // Of the counts that fit, the one whose items (chunks x genes) leave the
   // least of the block's warps idle in the last round; a band also costs a
-  // barrier and two halo rows, about half a row's work.
+  // wait and two halo rows, about half a row's work.
   const int warps = threads / 32;
   long best = r;
   double best_eff = 0;
@@ -333,22 +333,23 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
       // Streaming: only where the planes do not all fit shared memory.
       const int own = v.stream == 2 ? GRN_SCHEDULE_STREAM2 : GRN_SCHEDULE_STREAM;
       if (sched != GRN_SCHEDULE_AUTO && sched != own) continue;
-      if (ft && ft != v.max_threads) continue;
+      if (ft && ft != 512) continue;
+      const int threads = ft ? ft : v.max_threads;
       const size_t plane_bytes = (size_t)grn::plane_floats(W, H, 1, 0) * sizeof(float);
       const int fit = optin > fixed ? (int)((optin - fixed) / plane_bytes) & ~1 : 0;
       if (sched == GRN_SCHEDULE_AUTO && fit / 2 >= max_genes) continue;
       const size_t room = optin > fixed ? optin - fixed : 0;
       const int R = v.stream == 2 ? stream2_rows(W, H, max_genes, room)
-                                  : stream_rows(W, H, max_genes, room, v.max_threads);
+                                  : stream_rows(W, H, max_genes, room, threads);
       if (R < 1) continue;
       const size_t rows = v.stream == 2 ? (size_t)max_genes * (2 * R + 6)
                                         : (size_t)2 * max_genes * (R + 2);
       plan.smem_bytes = fixed + (rows + 1) * row_bytes;
-      GRN_CUDA(ctx, grn::sim_occupancy(v, v.max_threads, plan.smem_bytes, &plan.blocks_per_sm));
+      GRN_CUDA(ctx, grn::sim_occupancy(v, threads, plan.smem_bytes, &plan.blocks_per_sm));
       const int ctas = plan.blocks_per_sm * ctx->n_sm;
       if (ctas < 1) continue;
       plan.schedule = own;
-      plan.threads = v.max_threads;
+      plan.threads = threads;
       plan.slot_floats = 2LL * max_genes * grn::plane_floats(W, H, 1, 0);
       plan.cluster = 1;
       plan.band_rows = R;
