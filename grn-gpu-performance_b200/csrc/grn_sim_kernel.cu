@@ -508,6 +508,26 @@ __device__ __forceinline__ int cell_offset(const Geom &g, int y, int x) {
 // 256 x 256 with 8 genes, 592 x 100 66.7 -> 57.0; one 32 x 32 model x 500
 // 0.53 -> 0.35.
 
+// How a model's step is evaluated: kFast and kClamp the fast combine (see
+// regulation) and the simplified update, with minConc 0 and above it; kExact
+// the reference's comparisons throughout.  48 x 40, 600 models x 300 steps
+// with minConc 0.01: kExact 2.33 ms, kClamp 1.96.  kClamp has one form (some
+// planes may be in the global slot) and steps with a barrier: compiled into
+// the barrier-free loop as well it gave 1.88, but cost kFast there 1% (64 x 64)
+// to 3% (32 x 32).
+enum Path { kFast, kClamp, kExact };
+
+template <int P>
+struct PathTag {
+  static constexpr int value = P;
+};
+
+// The new value n of a cell with rate r under minConc: a zero rate keeps the
+// value (n) whatever it is.
+__device__ __forceinline__ float clamped(float n, float r, float min_conc) {
+  return n < min_conc && r != 0.0f ? 0.0f : n;
+}
+
 // Euler update of one cell (modelsimulator.cpp:224-275), the exact path:
 //   r = lim*h - deg*c (+ dif*(s - tot*c) for diffusing genes)
 // with the reference's guard on the diffusion term, "a zero rate keeps the
@@ -686,11 +706,11 @@ __device__ __forceinline__ void regulation(const ProgSmem &P, int ctl, const Pla
 // New values of one gene for the strip, from its current plane (at src_gl,
 // or shared offset src) to its next one (dst_gl, dst).  `mx` takes the
 // max |rate| of the strip's real cells.
-// Fast path (minConc 0 and a non-negative finite state, host-checked): the
-// reference's diffusion guard only ever skips adding dif*0, a zero rate
-// gives c + dt*0 = c, and the clamp is a max with 0, so these simplify
-// without changing any result.
-template <int R, bool EXACT, bool RAGGED, bool DIFFUSES, bool SG, bool DG, bool CL>
+// Fast paths (a non-negative finite state, host-checked): the reference's
+// diffusion guard only ever skips adding dif*0, a zero rate gives c + dt*0 =
+// c, and with minConc 0 the clamp is a max with 0, so these simplify without
+// changing any result.
+template <int R, int PATH, bool RAGGED, bool DIFFUSES, bool SG, bool DG, bool CL>
 __device__ __forceinline__ void update_strip(const GeneSmem &gn, const float4 (&h)[R],
                                              const char *src_gl, int src, char *dst_gl, int dst,
                                              const Strip<R> &st, const Geom &g,
@@ -735,7 +755,7 @@ __device__ __forceinline__ void update_strip(const GeneSmem &gn, const float4 (&
     }
     float4 nv;
     float m, m1, m2, m3;
-    if constexpr (!EXACT) {
+    if constexpr (PATH != kExact) {
       float2 r01 = fma2(hi2(ld), lo2(ci), mul2(lo2(ld), lo2(h[i])));
       float2 r23 = fma2(hi2(ld), hi2(ci), mul2(lo2(ld), hi2(h[i])));
       if constexpr (DIFFUSES) {
@@ -744,8 +764,12 @@ __device__ __forceinline__ void update_strip(const GeneSmem &gn, const float4 (&
       }
       const float2 n01 = fma2(f2(dt), r01, lo2(ci));
       const float2 n23 = fma2(f2(dt), r23, hi2(ci));
-      nv = make_float4(fmaxf(n01.x, 0.0f), fmaxf(n01.y, 0.0f), fmaxf(n23.x, 0.0f),
-                       fmaxf(n23.y, 0.0f));
+      if constexpr (PATH == kClamp)
+        nv = make_float4(clamped(n01.x, r01.x, min_conc), clamped(n01.y, r01.y, min_conc),
+                         clamped(n23.x, r23.x, min_conc), clamped(n23.y, r23.y, min_conc));
+      else
+        nv = make_float4(fmaxf(n01.x, 0.0f), fmaxf(n01.y, 0.0f), fmaxf(n23.x, 0.0f),
+                         fmaxf(n23.y, 0.0f));
       m = fabsf(r01.x);
       m1 = fabsf(r01.y);
       m2 = fabsf(r23.x);
@@ -784,7 +808,7 @@ __device__ __forceinline__ void update_strip(const GeneSmem &gn, const float4 (&
 // One gene (entry k of the program) for the strip.  SPILL: genes n_sm and on
 // live in the global slot.  BAND: the source planes are a staged band in
 // shared memory, the destination is global.
-template <int R, bool EXACT, bool RAGGED, bool SPILL, bool BAND, bool CL>
+template <int R, int PATH, bool RAGGED, bool SPILL, bool BAND, bool CL>
 __device__ __forceinline__ void gene_step(const ProgSmem &P, int k, const Planes &pl,
                                           const Strip<R> &st, const Geom &g, const Halo &halo,
                                           float dt, float min_conc, float &mx) {
@@ -792,15 +816,15 @@ __device__ __forceinline__ void gene_step(const ProgSmem &P, int k, const Planes
   const int ctl = uniform(gn.ctl);
   const int p = ctl & 15;
   float4 h[R];
-  regulation<R, EXACT, SPILL>(P, ctl, pl, st, g, h);
+  regulation<R, PATH == kExact, SPILL>(P, ctl, pl, st, g, h);
   const auto update = [&](auto diffuses) {
     constexpr bool D = decltype(diffuses)::value;
     const int o = p * g.PSb;
     if (SPILL && p >= pl.n_sm)
-      update_strip<R, EXACT, RAGGED, D, true, true, CL>(gn, h, pl.gl, o, pl.gl_out, o, st, g, halo,
+      update_strip<R, PATH, RAGGED, D, true, true, CL>(gn, h, pl.gl, o, pl.gl_out, o, st, g, halo,
                                                         dt, min_conc, mx);
     else
-      update_strip<R, EXACT, RAGGED, D, false, BAND, CL>(
+      update_strip<R, PATH, RAGGED, D, false, BAND, CL>(
           gn, h, nullptr, pl.sm + o, pl.gl_out, BAND ? p * pl.out_stride : pl.sm_out + o, st, g,
           halo, dt, min_conc, mx);
   };
@@ -959,18 +983,18 @@ __device__ __forceinline__ Planes planes_of(const StatePtrs &sp, const Geom &g, 
 }
 
 // Genes first, first + splits, .. of the program for one strip.
-template <int R, bool EXACT, bool RAGGED, bool SPILL, bool CL>
+template <int R, int PATH, bool RAGGED, bool SPILL, bool CL>
 __device__ __forceinline__ void strip_step(const ProgSmem &P, const Planes &pl, int G,
                                            const Geom &g, const Strip<R> &st, const Halo &halo,
                                            int first, int splits, float dt, float min_conc,
                                            float &mx) {
 #pragma unroll 1
   for (int k = first; k < G; k += splits)
-    gene_step<R, EXACT, RAGGED, SPILL, false, CL>(P, k, pl, st, g, halo, dt, min_conc, mx);
+    gene_step<R, PATH, RAGGED, SPILL, false, CL>(P, k, pl, st, g, halo, dt, min_conc, mx);
 }
 
 // A warp's range of walked items, of the first `chunks` chunks.
-template <int R, bool EXACT, bool RAGGED, bool SPILL, bool BAND, bool CL>
+template <int R, int PATH, bool RAGGED, bool SPILL, bool BAND, bool CL>
 __device__ __forceinline__ void walk_step(const ProgSmem &P, const Planes &pl, int G,
                                           const Geom &g, const Halo &halo, int chunks, int warp,
                                           int lane, float dt, float min_conc, float &mx) {
@@ -983,17 +1007,17 @@ __device__ __forceinline__ void walk_step(const ProgSmem &P, const Planes &pl, i
     const int stop = (end >> 4) == chunk ? end & 15 : G;
 #pragma unroll 1
     for (int k = at & 15; k < stop; ++k)
-      gene_step<R, EXACT, RAGGED, SPILL, BAND, CL>(P, k, pl, st, g, halo, dt, min_conc, mx);
+      gene_step<R, PATH, RAGGED, SPILL, BAND, CL>(P, k, pl, st, g, halo, dt, min_conc, mx);
     at = (chunk + 1) << 4;
   }
 }
 
 // One step of the warp's work by the model's class: all planes in shared
-// memory or some in the global slot; the exact path always takes the general
-// form.  SYNC (owned chunks): between the waits of step s and its counts;
+// memory or some in the global slot; the clamped and exact paths always take
+// the general form.  SYNC (owned chunks): between the waits of step s and its counts;
 // false if a wait ran out.
 template <int R, bool LOOP, bool RAGGED, bool CL, bool SYNC>
-__device__ __forceinline__ bool block_step(bool exact, const ProgSmem &P, const StatePtrs &sp,
+__device__ __forceinline__ bool block_step(int path, const ProgSmem &P, const StatePtrs &sp,
                                            int G, const Geom &g, const Strip<R> &st,
                                            const Halo &halo, int own, int first, int splits,
                                            int chunks, int warp, int lane, int par, float dt,
@@ -1004,16 +1028,18 @@ __device__ __forceinline__ bool block_step(bool exact, const ProgSmem &P, const 
     if (s > 1 && !wait_counts<CL>(sync, s - 1)) return false;
   }
   const auto run = [&](auto e, auto spill) {
-    constexpr bool E = decltype(e)::value, S = decltype(spill)::value;
+    constexpr int E = decltype(e)::value;
+    constexpr bool S = decltype(spill)::value;
     if constexpr (LOOP)
       walk_step<R, E, RAGGED, S, false, CL>(P, pl, G, g, halo, chunks, warp, lane, dt, min_conc,
                                             mx);
     else
       strip_step<R, E, RAGGED, S, CL>(P, pl, G, g, st, halo, first, splits, dt, min_conc, mx);
   };
-  if (exact) run(True{}, True{});
-  else if (sp.n_sm < G) run(False{}, True{});
-  else run(False{}, False{});
+  if (path == kExact) run(PathTag<kExact>{}, True{});
+  else if (path == kClamp) run(PathTag<kClamp>{}, True{});
+  else if (sp.n_sm < G) run(PathTag<kFast>{}, True{});
+  else run(PathTag<kFast>{}, False{});
   if constexpr (SYNC) finish_chunk<CL>(sync, own, lane);
   return true;
 }
@@ -1034,7 +1060,7 @@ __device__ __forceinline__ bool block_step(bool exact, const ProgSmem &P, const 
 // band's items.  `out` addresses the band's cells as a plane does: cell (x,
 // local row y) of gene p at out + p * gps + (y + 1) * RS + x.
 template <int R, bool RAGGED>
-__device__ __forceinline__ void band_step(bool exact, const ProgSmem &P, const float *stage,
+__device__ __forceinline__ void band_step(int path, const ProgSmem &P, const float *stage,
                                           int G, const Geom &gb, float *out, size_t gps,
                                           float dt, float min_conc, float &mx) {
   const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -1042,12 +1068,13 @@ __device__ __forceinline__ void band_step(bool exact, const ProgSmem &P, const f
                       (int)kStateOffset,
                   0, nullptr, reinterpret_cast<char *>(out), (int)(gps * sizeof(float)), G};
   const int chunks = (gb.Q + 31) / 32;
-  if (exact)
-    walk_step<R, true, RAGGED, false, true, false>(P, pl, G, gb, Halo{}, chunks, warp, lane, dt,
-                                                   min_conc, mx);
-  else
-    walk_step<R, false, RAGGED, false, true, false>(P, pl, G, gb, Halo{}, chunks, warp, lane, dt,
-                                                    min_conc, mx);
+  const auto run = [&](auto e) {
+    walk_step<R, decltype(e)::value, RAGGED, false, true, false>(
+        P, pl, G, gb, Halo{}, chunks, warp, lane, dt, min_conc, mx);
+  };
+  if (path == kFast) run(PathTag<kFast>{});
+  else if (path == kClamp) run(PathTag<kClamp>{});
+  else run(PathTag<kExact>{});
 }
 
 // One Euler step of the streaming schedule.  Stages alternate by band.  The
@@ -1070,7 +1097,7 @@ __device__ __forceinline__ void band_step(bool exact, const ProgSmem &P, const f
 // failure.
 template <bool RAGGED>
 __device__ bool stream_step(const SimArgs &A, const ProgSmem &P, const StatePtrs &sp,
-                            const Geom &g, int G, int par, bool exact,
+                            const Geom &g, int G, int par, int path,
                             float dt, float min_conc, float &mx, uint64_t *bars,
                             uint32_t &mphase, int *counts, volatile int *fail, int R) {
   const int nb = (g.H + R - 1) / R;
@@ -1113,7 +1140,7 @@ __device__ bool stream_step(const SimArgs &A, const ProgSmem &P, const StatePtrs
     gb.PS = SPS;
     gb.PSb = 4 * SPS;
     gb.Q = strip_count<kStripRows>(gb.H, g.Wg);
-    band_step<kStripRows, RAGGED>(exact, P, stage0 + s * sp.gmax * SPS, G, gb,
+    band_step<kStripRows, RAGGED>(path, P, stage0 + s * sp.gmax * SPS, G, gb,
                           gl_nxt + (size_t)gb.y0 * g.RS, gps, dt, min_conc, mx);
     __syncwarp();
     if ((threadIdx.x & 31) == 0) {
@@ -1166,7 +1193,7 @@ __device__ bool stream_step(const SimArgs &A, const ProgSmem &P, const StatePtrs
 // time, after a bounded wait for the copy still in flight.
 template <bool RAGGED>
 __device__ bool stream_step2(const SimArgs &A, const ProgSmem &P, const StatePtrs &sp,
-                             const Geom &g, int G, int par, bool exact,
+                             const Geom &g, int G, int par, int path,
                              float dt, float min_conc, float &mx1, float &mx2, uint64_t *bars,
                              uint32_t &mphase, volatile int *fail) {
   const int R = A.band_rows;
@@ -1208,7 +1235,7 @@ __device__ bool stream_step2(const SimArgs &A, const ProgSmem &P, const StatePtr
     // Stage row of grid row y is y - bR + 2; g1's row 0 is grid row y1 - 1.
     const float *st1 = stage + (y1 - b * R + 1) * g.RS;
     float *out1 = inter + (y1 - b * R) * g.RS;  // cell rows land at y - (bR - 1)
-    band_step<kStripRows, RAGGED>(exact, P, st1, G, g1, out1, (size_t)IPS, dt, min_conc, mx1);
+    band_step<kStripRows, RAGGED>(path, P, st1, G, g1, out1, (size_t)IPS, dt, min_conc, mx1);
     // Intermediate rows outside the grid are the planes' zero rows.
     const int zlo = (b == 0) ? 0 : -1;                            // grid row -1
     const int zhi = (b * R + R >= g.H) ? g.H - (b * R - 1) : -1;  // grid row H
@@ -1232,7 +1259,7 @@ __device__ bool stream_step2(const SimArgs &A, const ProgSmem &P, const StatePtr
     g2.PS = IPS;
     g2.PSb = 4 * IPS;
     g2.Q = strip_count<kStripRows>(g2.H, g.Wg);
-    band_step<kStripRows, RAGGED>(exact, P, inter, G, g2, gl_nxt + (size_t)g2.y0 * g.RS, gps, dt,
+    band_step<kStripRows, RAGGED>(path, P, inter, G, g2, gl_nxt + (size_t)g2.y0 * g.RS, gps, dt,
                           min_conc, mx2);
     __syncthreads();  // the intermediate is free again
   }
@@ -1463,6 +1490,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
     sp.n_sm = min(G, A.planes / 2);
     const bool exact = !(A.fast_ok && (M.hdr.flags & kFlagFast) &&
                          G <= GRN_MAX_GENES);
+    const int path = exact ? kExact : min_conc > 0.0f ? kClamp : kFast;
     const bool bad = G < 1 || G > GRN_MAX_GENES || M.hdr.n_links < 0 ||
                      M.hdr.n_links > GRN_MAX_LINKS || (sp.n_sm < G && sp.gl == nullptr) ||
                      ((sp.n_sm < G || ST) && G > A.gmax) || (!LOOP && chunks > n_warps) ||
@@ -1541,14 +1569,14 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
         // Fast models that stop early only on a change of exactly 0: every
         // rate is then 0 and the state stays as it is, so the steps after it
         // change nothing, and the last step with a rate tells when it was.
-        if (!exact && A.change_bound <= 0.0f && A.n_steps > 0 && free_steps) {
+        if (path == kFast && A.change_bound <= 0.0f && A.n_steps > 0 && free_steps) {
           float mx = 0.0f;
           int last = 0;  // steps up to the warp's last one with a rate
           if (fixed_part < splits) {
             for (int s = 1; s <= A.n_steps; ++s) {
               mx = 0.0f;
               if (!block_step<kStripRows, LOOP, RAGGED, CL, true>(
-                      false, P, sp, G, g, fixed, halo, own, fixed_part, splits, chunks, warp, lane,
+                      kFast, P, sp, G, g, fixed, halo, own, fixed_part, splits, chunks, warp, lane,
                       (s - 1) & 1, dt, min_conc, mx, sync, s)) {
                 last = 0x7fffffff;
                 break;
@@ -1590,7 +1618,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
           bool ok = true, single = true;
           if (ST == 2 && step + 2 <= A.n_steps) {
             float mx2 = 0.0f;
-            ok = stream_step2<RAGGED>(A, P, sp, g, G, par, exact, dt, min_conc, mx, mx2,
+            ok = stream_step2<RAGGED>(A, P, sp, g, G, par, path, dt, min_conc, mx, mx2,
                                           bars, mphase, s_stream_fail);
             if (ok) {
               const float b1 = block_max(mx, s_red, par ^ 1, lane, warp, n_warps);
@@ -1600,7 +1628,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
             }
           }
           if (ok && single)
-            ok = stream_step<RAGGED>(A, P, sp, g, G, par, exact, dt, min_conc, mx, bars,
+            ok = stream_step<RAGGED>(A, P, sp, g, G, par, path, dt, min_conc, mx, bars,
                                          mphase, s_done, s_stream_fail, A.band_rows);
           if (!ok) {
             if (tid == 0) {
@@ -1610,7 +1638,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
             return;  // every thread of the block: the decision is block-uniform
           }
         } else {
-          block_step<kStripRows, LOOP, RAGGED, CL, false>(exact, P, sp, G, g, fixed, halo, own,
+          block_step<kStripRows, LOOP, RAGGED, CL, false>(path, P, sp, G, g, fixed, halo, own,
                                                           fixed_part, splits, chunks, warp, lane,
                                                           par, dt, min_conc, mx, StepSync{}, 0);
         }

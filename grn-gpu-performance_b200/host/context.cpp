@@ -96,7 +96,7 @@ struct grn_ctx {
   std::string last_tuning;  // the last autotuning's candidates and times
   int n_tunings = 0;         // autotuning runs so far
   double tuning_ms = 0;      // their host wall time
-  // minConc is 0 and the uploaded initial states are finite, non-negative
+  // minConc is finite, not negative, and the uploaded initial states are finite, non-negative
   // and at most 1e6: the kernel's fast path then gives the same results as
   // the exact one for every model whose step size keeps its state bounded
   // (see the kernel's update_cell and euler_bounded).
@@ -1118,7 +1118,7 @@ grn_status grn_set_experiments(grn_ctx *ctx, int n_experiments, const double *in
   // The fast path's bound on the state (the kernel's euler_bounded) also
   // needs the initial values below kFastMaxInitial.
   constexpr double kFastMaxInitial = 1.0e6;
-  bool ok = ctx->p.min_conc == 0.0;
+  bool ok = ctx->p.min_conc >= 0.0 && std::isfinite(ctx->p.min_conc);
   for (size_t i = 0; ok && i < ni; ++i) {
     const double v = fi[i];  // the value the kernel starts from
     ok = std::isfinite(v) && v >= 0 && v <= kFastMaxInitial;
