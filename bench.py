@@ -19,8 +19,8 @@ uneven_64x64: 4096 models, 2-8 genes, 1-24 links, 64x64 grid, 2000 steps).
           launch -- 3 per used link per cell-update (lg2, ex2, rcp of each
           Hill term in the reference formulation) -- over the mean launch
           time, against 16 MUFU/clk/SM x SMs x max SM clock.  The kernel
-          issues fewer MUFU ops than that (one lg2 per regulator product and
-          one ex2 + rcp per regulated product, in exponent form); those are
+          issues fewer MUFU ops than that (one lg2 per used link and one
+          ex2 + rcp per regulated product, in exponent form); those are
           reported as issued_mufu.  fp32_frac: algorithmic FP32 ops
           (6 L + 7 G + 8 G_dif per cell-update) against 128/clk/SM.
   cpu_baseline  the FP64 oracle (a port of the reference's CPU evaluator) on

@@ -266,7 +266,7 @@ grn_status pack_batch(const grn_model_batch *batch, int n_morphogens, float dt, 
     out->max_links = std::max(out->max_links, c.links);
     out->sum_genes += c.genes;
     out->sum_links += c.links;
-    out->sfu_per_cell_step += c.lg_genes + 2 * c.reg_genes;
+    out->sfu_per_cell_step += c.links + 2 * c.reg_genes;
     out->fma_per_cell_step += 2 * c.links + 6 * c.genes + 6 * c.dif_genes;
     out->sum_dif_genes += c.dif_genes;
     out->alg_sfu_per_cell_step += 3 * c.links;

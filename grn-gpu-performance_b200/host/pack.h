@@ -46,7 +46,7 @@ struct PackedHost {
   int max_links = 0;
   double sum_genes = 0;
   double sum_links = 0;
-  int64_t sfu_per_cell_step = 0;  // sum over models of lg + 2 * reg genes
+  int64_t sfu_per_cell_step = 0;  // sum over models of links + 2 * reg genes
   int64_t fma_per_cell_step = 0;  // rough FP32-pipe op count, summed
   double sum_dif_genes = 0;
   int64_t alg_sfu_per_cell_step = 0;   // sum of 3 L (reference formulation)
