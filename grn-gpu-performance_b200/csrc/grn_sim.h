@@ -24,7 +24,8 @@ struct SimArgs {
   int32_t n_target;          // target morphogens
   int32_t W, H;              // grid width (x) and height (y)
   int32_t Wg;                // float4 groups per row = ceil(W / 4)
-  uint32_t inv_wg;           // ceil(2^32 / Wg) (unused when Wg is 1)
+  uint32_t inv_wg;           // inverse(Wg) (unused when Wg is 1)
+  int32_t wg_shift;          // inverse_shift(Wg)
   uint32_t inv_w;            // ceil(2^32 / W): a cell's row by multiplication, or 0
                              // where that is not exact
   int32_t row_floats, row_bytes;      // one padded state row
@@ -156,6 +157,26 @@ inline int strip_chunks(int W, int rows) {
   return ((strip_rows(rows) / kStripRows) * ((W + 3) / 4) + 31) / 32;
 }
 
+// Division by a number d that is the same for a whole launch (Granlund and
+// Montgomery, "Division by invariant integers using multiplication", 1994):
+// with 2^k < d <= 2^(k+1) and inv = ceil(2^(32+k) / d), which fits 32 bits,
+// (i * inv) >> (32 + k) is floor(i / d) for every 0 <= i < 2^31: it exceeds
+// i / d by i * e / (d * 2^(32+k)) with e < d <= 2^(k+1), i.e. by less than
+// 1 / d.
+inline int inverse_shift(int d) {
+  int k = 0;
+  while (((int64_t)2 << k) < d) ++k;
+  return k;
+}
+inline uint32_t inverse(int d) {
+  const uint64_t p = (uint64_t)1 << (32 + inverse_shift(d));
+  return d > 1 ? (uint32_t)((p + d - 1) / d) : 0u;
+}
+// Row of group i in rows of Wg float4 groups.
+GRN_HOST_DEVICE inline int group_row(int i, int Wg, uint32_t inv_wg, int wg_shift) {
+  return Wg == 1 ? i : (int)((uint32_t)(((uint64_t)(uint32_t)i * inv_wg) >> 32) >> wg_shift);
+}
+
 // SimArgs::change_bound.
 inline float float_below(double x) {
   const float f = (float)x;
@@ -167,11 +188,10 @@ inline void set_geometry(SimArgs *a, int W, int H, int cluster, int pad) {
   a->W = W;
   a->H = H;
   a->Wg = (W + 3) / 4;
-  const auto inverse = [](int d) {
-    return d > 1 ? (uint32_t)((((uint64_t)1 << 32) + d - 1) / d) : 0u;
-  };
   a->inv_wg = inverse(a->Wg);
-  a->inv_w = (int64_t)W * H * W < (int64_t)1 << 32 ? inverse(W) : 0u;
+  a->wg_shift = inverse_shift(a->Wg);
+  const uint32_t w_inv = W > 1 ? (uint32_t)((((uint64_t)1 << 32) + W - 1) / W) : 0u;
+  a->inv_w = (int64_t)W * H * W < (int64_t)1 << 32 ? w_inv : 0u;
   a->row_floats = row_floats(W);
   a->row_bytes = 4 * a->row_floats;
   a->row_pad = pad;

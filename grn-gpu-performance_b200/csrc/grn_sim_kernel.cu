@@ -428,7 +428,8 @@ struct Geom {
   int RSb, PSb, SSb;        // RS, PS and a row of strips (R * RS + pad) in bytes
   bool edges;               // chunks do not hold whole rows of groups
   int y0, Hg;               // first grid row of the band, grid height
-  uint32_t inv_wg;          // ceil(2^32 / Wg): q / Wg by multiplication
+  uint32_t inv_wg;          // q / Wg by multiplication (group_row)
+  int wg_shift;
 };
 
 // Strips of R rows x 4 columns in H rows of Wg groups.
@@ -460,8 +461,7 @@ __device__ __forceinline__ Strip<R> strip_at(int q, const Geom &g) {
   Strip<R> s;
   s.valid = q < g.Q;
   const int qc = s.valid ? q : g.Q - 1;
-  // Exact while q * Wg < 2^32 (dimensions up to 4096: Wg <= 1024, q < 2^21).
-  const int ys = g.Wg == 1 ? qc : (int)__umulhi((uint32_t)qc, g.inv_wg);
+  const int ys = group_row(qc, g.Wg, g.inv_wg, g.wg_shift);
   const int gx = qc - ys * g.Wg, y = R * ys, x0 = 4 * gx;
   s.rows = min(R, g.H - y);
   s.el = gx == 0 || (q & 31) == 0;
@@ -1357,6 +1357,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
   g.PSb = A.plane_bytes;
   g.Q = strip_count<kStripRows>(g.H, A.Wg);
   g.inv_wg = A.inv_wg;
+  g.wg_shift = A.wg_shift;
   const float dt = A.dt, min_conc = A.min_conc;
   uint4 *Mw = reinterpret_cast<uint4 *>(smem);
 
@@ -1529,7 +1530,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
       for (int kk = 0; kk < min(A.n_in, G); ++kk) {
         float *pl = plane_of(sp, g, kk, 0);
         for (int i = tid; i < (g.H + 2) * g.Wg; i += NT) {
-          const int rr = g.Wg == 1 ? i : (int)__umulhi((uint32_t)i, g.inv_wg);
+          const int rr = group_row(i, g.Wg, g.inv_wg, g.wg_shift);
           const int x0 = 4 * (i - rr * g.Wg), y = g.y0 - 1 + rr;  // grid row
           if (y < 0 || y >= g.Hg) continue;
           const float *src = init + ((size_t)kk * g.Hg + y) * g.W + x0;
