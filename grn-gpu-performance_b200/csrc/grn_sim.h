@@ -66,6 +66,8 @@ struct SimArgs {
 
 // Test hooks (grn_set_test_hooks): make a bounded wait run out on purpose.
 constexpr int32_t kHookWithholdBandCopy = 1;  // streaming: band 1's copy is never issued
+constexpr int32_t kHookWithholdChunkCount = 8;  // steps without a block barrier: no wait for
+                                                // chunk 0 (of a cluster's first CTA) ends
 
 // One compiled kernel variant.
 struct KernelVariant {

@@ -915,13 +915,16 @@ struct StepSync {
 };
 
 // Waits until this lane's count has reached `steps` steps, in every lane;
-// false, and *fail set, after about a second or once another warp has given
-// up.
+// false, and *fail set, after 2^24 polls (0.5 to 1 s measured; a step takes
+// microseconds) or once another warp has given up.  Every decision to leave is
+// a vote: lanes that read *fail at different moments must not part ways at the
+// vote of the next poll.
+constexpr uint32_t kMaxPolls = 1u << 24;
 template <bool CL>
 __device__ __forceinline__ bool wait_counts(const StepSync &y, int steps) {
   const uint32_t a = smem_addr(y.wait);
   const int target = y.per_step * steps;
-  for (uint32_t i = 0; i < (1u << 24); ++i) {
+  for (uint32_t i = 0; i < kMaxPolls; ++i) {
     int v;
     if (CL && y.edge)
       asm volatile("ld.acquire.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
@@ -931,7 +934,7 @@ __device__ __forceinline__ bool wait_counts(const StepSync &y, int steps) {
       __syncwarp();
       return true;
     }
-    if ((i & 1023u) == 1023u && *y.fail) return false;
+    if ((i & 1023u) == 1023u && __any_sync(kFull, *y.fail)) return false;
   }
   *y.fail = 1;
   return false;
@@ -1521,6 +1524,11 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
       // start as the neighbouring grid rows.
       const float *init = A.initial + (size_t)e * A.n_in * A.W * A.H;
       for (int i = tid; i < kMaxDone + 2; i += NT) s_done[i] = 0;
+      if constexpr (FREE) {
+        // Test hook: chunk 0's count starts so far back that no wait for it ends.
+        if ((A.test_hooks & kHookWithholdChunkCount) && rank == 0 && tid == 0)
+          s_done[0] = -(1 << 30);
+      }
       zero_floats(sp.sm, 2 * sp.n_sm * g.PS);
       if (sp.n_sm < G) {
         zero_floats(sp.gl + (size_t)sp.n_sm * g.PS, (G - sp.n_sm) * g.PS);

@@ -35,6 +35,7 @@ SCHEDULE_STREAM2 = 6
 TEST_WITHHOLD_BAND_COPY = 1
 TEST_FAIL_DEVICE_ALLOC = 2
 TEST_CORRUPT_RECORD = 4
+TEST_WITHHOLD_CHUNK_COUNT = 8
 SCORE_PARENT_ERROR, SCORE_PAIRED = 0, 1
 SCHEDULE_NAMES = {0: "auto", 1: "fixed_items", 2: "walk_items", 3: "global", 4: "cluster",
                   5: "stream", 6: "stream2"}

@@ -1050,7 +1050,7 @@ grn_status grn_autotune_report(const grn_ctx *ctx, char *buf, int buf_len) {
 
 grn_status grn_set_test_hooks(grn_ctx *ctx, int hooks) {
   if (!ctx || (hooks & ~(GRN_TEST_WITHHOLD_BAND_COPY | GRN_TEST_FAIL_DEVICE_ALLOC |
-                         GRN_TEST_CORRUPT_RECORD)))
+                         GRN_TEST_CORRUPT_RECORD | GRN_TEST_WITHHOLD_CHUNK_COUNT)))
     return GRN_ERR_INVALID_ARGUMENT;
   ctx->test_hooks = hooks;
   return GRN_OK;

@@ -255,6 +255,12 @@ grn_status grn_set_host_threads(grn_ctx *ctx, int n_threads);
  * record check rejects (GRN_ERR_KERNEL, that model's raw error NaN). */
 #define GRN_TEST_FAIL_DEVICE_ALLOC 2
 #define GRN_TEST_CORRUPT_RECORD 4
+/* GRN_TEST_WITHHOLD_CHUNK_COUNT: where warps step without a block barrier
+ * (owned chunks of fast models without an early-exit threshold), no wait for
+ * a model's first chunk ends, so the bounded waits run out (about one second
+ * per model), the model's raw error becomes NaN and the call returns
+ * GRN_ERR_KERNEL; the context stays usable. */
+#define GRN_TEST_WITHHOLD_CHUNK_COUNT 8
 grn_status grn_set_test_hooks(grn_ctx *ctx, int hooks);
 
 /* ------------------------------------------------------------ experiments */
