@@ -179,6 +179,13 @@ GRN_HOST_DEVICE inline int group_row(int i, int Wg, uint32_t inv_wg, int wg_shif
   return Wg == 1 ? i : (int)((uint32_t)(((uint64_t)(uint32_t)i * inv_wg) >> 32) >> wg_shift);
 }
 
+// Whether a count of finished work has come up to `target`, both modulo 2^32:
+// counts grow by up to 32 a step, so long runs wrap, and no count is ever more
+// than a few steps from its target.
+GRN_HOST_DEVICE inline bool count_reached(uint32_t count, uint32_t target) {
+  return (int32_t)(count - target) >= 0;
+}
+
 // SimArgs::change_bound.
 inline float float_below(double x) {
   const float f = (float)x;

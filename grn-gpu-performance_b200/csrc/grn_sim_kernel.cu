@@ -923,14 +923,14 @@ constexpr uint32_t kMaxPolls = 1u << 24;
 template <bool CL>
 __device__ __forceinline__ bool wait_counts(const StepSync &y, int steps) {
   const uint32_t a = smem_addr(y.wait);
-  const int target = y.per_step * steps;
+  const uint32_t target = (uint32_t)y.per_step * (uint32_t)steps;
   for (uint32_t i = 0; i < kMaxPolls; ++i) {
-    int v;
+    uint32_t v;
     if (CL && y.edge)
       asm volatile("ld.acquire.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     else
       asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    if (__all_sync(kFull, v >= target)) {
+    if (__all_sync(kFull, count_reached(v, target))) {
       __syncwarp();
       return true;
     }

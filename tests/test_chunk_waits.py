@@ -1,7 +1,10 @@
 """The bounded waits of steps without a block barrier.  A count that never
 comes (test hook): the warps that wait for it give up together, the block or
 the whole cluster leaves, the call reports it within seconds, and the same
-context then gives the right result."""
+context then gives the right result.  Counts of long runs wrap (CPU, over the
+kernel's own header)."""
+import os
+import subprocess
 import time
 
 import numpy as np
@@ -10,9 +13,19 @@ import pytest
 import grn_b200 as grn
 import synth
 
-pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 
 
+def test_counts_wrap(tmp_path):
+    exe = str(tmp_path / "chunk_counts")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-I" + os.path.join(CUDA_HOME, "include"),
+                    os.path.join(ROOT, "tests", "cpp", "chunk_counts.cpp"), "-o", exe], check=True)
+    out = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert out.returncode == 0, out.stdout
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("W,H,sched,cluster", [
     (64, 64, grn.SCHEDULE_FIXED_ITEMS, 0),   # 16 chunks, waits of both neighbours
     (8, 8, grn.SCHEDULE_FIXED_ITEMS, 0),     # one chunk, which waits for its own parts
@@ -40,6 +53,7 @@ def test_a_missing_count_is_reported(W, H, sched, cluster):
     np.testing.assert_array_equal(raw, want)
 
 
+@pytest.mark.gpu
 def test_the_hook_leaves_barrier_steps_alone():
     """Models with an early-exit threshold pass a barrier and wait for no count."""
     params, batch, init, tgt = synth.workload("uneven_64x64", seed=5, n_models=3, steps=40)
