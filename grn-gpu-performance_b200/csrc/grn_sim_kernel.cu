@@ -224,11 +224,12 @@ constexpr size_t kMbarOffset = (kCsumOffset + 8 + 15) & ~size_t(15);
 constexpr size_t kStreamFailOffset = kMbarOffset + 16;
 // Bounds-checked build only: the regions that state accesses are checked
 // against (CheckRegions).
-// Steps without a block barrier (StepSync): finished work per chunk (int [32])
-// and the halo counts (int [2]).
+// Steps without a block barrier (StepSync): finished work per chunk (int [32]),
+// the halo counts (int [2]) and the last vote with a rate (int).
 constexpr int kMaxDone = 32;
+constexpr int kDoneInts = kMaxDone + 3;
 constexpr size_t kDoneOffset = kStreamFailOffset + 16;
-constexpr size_t kCheckOffset = (kDoneOffset + (kMaxDone + 2) * 4 + 15) & ~size_t(15);
+constexpr size_t kCheckOffset = (kDoneOffset + kDoneInts * 4 + 15) & ~size_t(15);
 constexpr size_t kCheckBytes = GRN_BOUNDS_CHECK ? 64 : 0;
 constexpr size_t kStateOffset = (kCheckOffset + kCheckBytes + 127) & ~size_t(127);
 
@@ -960,6 +961,40 @@ __device__ __forceinline__ void finish_chunk(const StepSync &y, int c, int lane)
   }
 }
 
+// Whether a model is at rest is looked at every kVoteSteps steps.  A warp whose
+// part has a rate in step s, such a step, raises *alive to s (in every CTA of a
+// cluster).  *alive below s - lag at step s then means that no part of the grid
+// had a rate in step s - lag, and that none has had one since: warps are never
+// further apart than the chunks between them (each is at most a step ahead of
+// its neighbours), fewer than lag, so every warp has been through step s - lag,
+// and its word is here by way of the counts.  For the same reason all warps
+// come to the same answer at the same step.  A model that comes to rest runs
+// lag + kVoteSteps steps more at most.  4 models of 64 x 64 that rest
+// after 150 steps, asked for 400,000: 1524 -> 0.8 ms.  Models that never rest
+// pay a word per warp and vote: 64 x 64, 4096 x 500 39.11 -> 39.13 ms; 32 x 32,
+// 64 x 500 0.440 -> 0.435 (a block barrier every 64 steps instead: 39.85 and
+// 0.434).
+constexpr int kVoteSteps = 64;
+template <bool CL>
+__device__ __forceinline__ bool at_rest(int *alive, int s, bool rate, int C, int lane) {
+  constexpr int lag = CL ? kMaxCluster * kMaxDone + kVoteSteps : kVoteSteps;
+  static_assert(kMaxDone <= kVoteSteps && lag % kVoteSteps == 0, "lag covers all chunks");
+  if (rate) {
+    if constexpr (CL) {
+      if (lane < C)
+        asm volatile("red.relaxed.cluster.shared::cluster.max.s32 [%0], %1;" ::"r"(
+                         cluster_addr(smem_addr(alive), lane)),
+                     "r"(s)
+                     : "memory");
+    } else if (lane == 0) {
+      asm volatile("red.relaxed.cta.shared::cta.max.s32 [%0], %1;" ::"r"(smem_addr(alive)), "r"(s)
+                   : "memory");
+    }
+  }
+  const int seen = *reinterpret_cast<volatile int *>(alive);
+  return !__any_sync(kFull, seen >= s - lag);
+}
+
 // Where a model's state lives during one step: genes p < n_sm are double
 // buffered in shared-memory planes p and p + n_sm; the others in the
 // block's global slot, planes p and p + gmax.  `par` selects the buffer
@@ -1523,7 +1558,7 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
       // buffer's cells are all written by the first step.  A band's halo rows
       // start as the neighbouring grid rows.
       const float *init = A.initial + (size_t)e * A.n_in * A.W * A.H;
-      for (int i = tid; i < kMaxDone + 2; i += NT) s_done[i] = 0;
+      for (int i = tid; i < kDoneInts; i += NT) s_done[i] = 0;
       if constexpr (FREE) {
         // Test hook: chunk 0's count starts so far back that no wait for it ends.
         if ((A.test_hooks & kHookWithholdChunkCount) && rank == 0 && tid == 0)
@@ -1577,20 +1612,28 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
       if constexpr (FREE) {
         // Fast models that stop early only on a change of exactly 0: every
         // rate is then 0 and the state stays as it is, so the steps after it
-        // change nothing, and the last step with a rate tells when it was.
+        // change nothing, and the last step with a rate tells when it was.  They
+        // are not run to the end (at_rest).
         if (path == kFast && A.change_bound <= 0.0f && A.n_steps > 0 && free_steps) {
           float mx = 0.0f;
           int last = 0;  // steps up to the warp's last one with a rate
           if (fixed_part < splits) {
-            for (int s = 1; s <= A.n_steps; ++s) {
-              mx = 0.0f;
-              if (!block_step<kStripRows, LOOP, RAGGED, CL, true>(
-                      kFast, P, sp, G, g, fixed, halo, own, fixed_part, splits, chunks, warp, lane,
-                      (s - 1) & 1, dt, min_conc, mx, sync, s)) {
-                last = 0x7fffffff;
-                break;
+            bool go = true;
+            for (int s = 1; go && s <= A.n_steps;) {
+              const int end = s + min(A.n_steps - s, kVoteSteps - 1);
+              for (; s <= end; ++s) {
+                mx = 0.0f;
+                if (!block_step<kStripRows, LOOP, RAGGED, CL, true>(
+                        kFast, P, sp, G, g, fixed, halo, own, fixed_part, splits, chunks, warp,
+                        lane, (s - 1) & 1, dt, min_conc, mx, sync, s)) {
+                  last = 0x7fffffff;
+                  go = false;
+                  break;
+                }
+                if (__any_sync(kFull, mx > 0.0f)) last = s;
               }
-              if (__any_sync(kFull, mx > 0.0f)) last = s;
+              if (go && A.change_bound == 0.0f && end < A.n_steps)
+                go = !at_rest<CL>(s_done + kMaxDone + 2, end, last == end, C, lane);
             }
           }
           step = A.n_steps;
