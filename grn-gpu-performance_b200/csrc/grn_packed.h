@@ -34,13 +34,15 @@ constexpr int kConstSlot = 255;
 
 // Header flags.
 constexpr uint32_t kFlagNone = 0u;
-// Every link has a finite K > 0, a finite Hill coefficient 0 < n <= 32 and
+// Every link has a finite K > 0, a finite Hill coefficient 0 <= n <= 32 and
 // 0 < K^n <= 1e300, and every gene finite rates: on a bounded non-negative
-// state no link term can be NaN or constant, so the kernel may combine terms
+// state no link term can be NaN, so the kernel may combine terms
 // with min/max (see the kernel's regulation).  pack_batch also clears
 // the flag where the run's step size could leave the state unbounded
 // (euler_bounded in host/pack.h), so the kernel tests only the flag.
 constexpr uint32_t kFlagFast = 1u;
+// Some link has the constant term 0 (kConstSlot).
+constexpr uint32_t kFlagConstantTerm = 2u;
 
 struct alignas(16) PackedHeader {
   int32_t orig_index;  // position of the model in the caller's batch

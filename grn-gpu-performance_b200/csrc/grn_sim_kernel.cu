@@ -510,13 +510,18 @@ __device__ __forceinline__ int cell_offset(const Geom &g, int y, int x) {
 // 0.53 -> 0.35.
 
 // How a model's step is evaluated: kFast and kClamp the fast combine (see
-// regulation) and the simplified update, with minConc 0 and above it; kExact
-// the reference's comparisons throughout.  48 x 40, 600 models x 300 steps
-// with minConc 0.01: kExact 2.33 ms, kClamp 1.96.  kClamp has one form (some
-// planes may be in the global slot) and steps with a barrier: compiled into
-// the barrier-free loop as well it gave 1.88, but cost kFast there 1% (64 x 64)
-// to 3% (32 x 32).
-enum Path { kFast, kClamp, kExact };
+// regulation) and the simplified update, with minConc 0 and above it; kConst
+// that update and the reference's comparison order in the combine, for fast
+// models with constant link terms, under any minConc; kExact the reference's
+// comparisons throughout.  48 x 40, 600 models x 300 steps with minConc 0.01:
+// kExact 2.33 ms, kClamp 1.96.  kClamp and kConst have one form (some
+// planes may be in the global slot) and step with a barrier: compiled into
+// the barrier-free loop as well kClamp gave 1.88, but cost kFast there 1% (64 x
+// 64) to 3% (32 x 32).  Models with constant terms (ms, kExact -> kConst): 64 x
+// 64, 592 x 500 8.74 -> 7.62; 100 x 100, 296 x 300 8.61 -> 7.35; 32 x 32, 64 x
+// 500 0.73 -> 0.61.  Constant terms taken in the fast combine, for the genes that
+// have them, gave 6.05, 5.80 and 0.48, but cost all other models 1% to 3%.
+enum Path { kFast, kClamp, kConst, kExact };
 
 template <int P>
 struct PathTag {
@@ -645,10 +650,10 @@ __device__ __forceinline__ float4 hill4(const float4 &v) {
 
 // Regulation of one gene (its ctl word) for the strip: the first link's
 // terms start the running exponents, OR links take the min, AND links the
-// max.  exact: the reference's comparison order, where a Hill coefficient
-// of 0 (kConstSlot) gives the constant term 0; in the fast path models have
+// max.  ORDERED: the reference's comparison order, where a Hill coefficient
+// of 0 (kConstSlot) gives the constant term 0; models on the other paths have
 // no such link.
-template <int R, bool EXACT, bool SPILL>
+template <int R, bool ORDERED, bool SPILL>
 __device__ __forceinline__ void regulation(const ProgSmem &P, int ctl, const Planes &pl,
                                            const Strip<R> &st, const Geom &g, float4 (&h)[R]) {
   const int n = ctl >> 21;
@@ -660,7 +665,7 @@ __device__ __forceinline__ void regulation(const ProgSmem &P, int ctl, const Pla
   const LinkSmem *L = P.link + ((ctl >> 5) & 255);
   const int n_or = (ctl >> 13) & 255;
   float4 v[R], t[R];
-  if constexpr (EXACT) {
+  if constexpr (ORDERED) {
 #pragma unroll
     for (int i = 0; i < R; ++i) v[i] = f4(__int_as_float(0x7fc00000));
 #pragma unroll 1
@@ -765,7 +770,7 @@ __device__ __forceinline__ void update_strip(const GeneSmem &gn, const float4 (&
       }
       const float2 n01 = fma2(f2(dt), r01, lo2(ci));
       const float2 n23 = fma2(f2(dt), r23, hi2(ci));
-      if constexpr (PATH == kClamp)
+      if constexpr (PATH != kFast)
         nv = make_float4(clamped(n01.x, r01.x, min_conc), clamped(n01.y, r01.y, min_conc),
                          clamped(n23.x, r23.x, min_conc), clamped(n23.y, r23.y, min_conc));
       else
@@ -817,7 +822,7 @@ __device__ __forceinline__ void gene_step(const ProgSmem &P, int k, const Planes
   const int ctl = uniform(gn.ctl);
   const int p = ctl & 15;
   float4 h[R];
-  regulation<R, PATH == kExact, SPILL>(P, ctl, pl, st, g, h);
+  regulation<R, PATH == kExact || PATH == kConst, SPILL>(P, ctl, pl, st, g, h);
   const auto update = [&](auto diffuses) {
     constexpr bool D = decltype(diffuses)::value;
     const int o = p * g.PSb;
@@ -1051,8 +1056,8 @@ __device__ __forceinline__ void walk_step(const ProgSmem &P, const Planes &pl, i
 }
 
 // One step of the warp's work by the model's class: all planes in shared
-// memory or some in the global slot; the clamped and exact paths always take
-// the general form.  SYNC (owned chunks): between the waits of step s and its counts;
+// memory or some in the global slot; the other paths always take the general
+// form.  SYNC (owned chunks): between the waits of step s and its counts;
 // false if a wait ran out.
 template <int R, bool LOOP, bool RAGGED, bool CL, bool SYNC>
 __device__ __forceinline__ bool block_step(int path, const ProgSmem &P, const StatePtrs &sp,
@@ -1076,6 +1081,7 @@ __device__ __forceinline__ bool block_step(int path, const ProgSmem &P, const St
   };
   if (path == kExact) run(PathTag<kExact>{}, True{});
   else if (path == kClamp) run(PathTag<kClamp>{}, True{});
+  else if (path == kConst) run(PathTag<kConst>{}, True{});
   else if (sp.n_sm < G) run(PathTag<kFast>{}, True{});
   else run(PathTag<kFast>{}, False{});
   if constexpr (SYNC) finish_chunk<CL>(sync, own, lane);
@@ -1112,6 +1118,7 @@ __device__ __forceinline__ void band_step(int path, const ProgSmem &P, const flo
   };
   if (path == kFast) run(PathTag<kFast>{});
   else if (path == kClamp) run(PathTag<kClamp>{});
+  else if (path == kConst) run(PathTag<kConst>{});
   else run(PathTag<kExact>{});
 }
 
@@ -1529,7 +1536,10 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
     sp.n_sm = min(G, A.planes / 2);
     const bool exact = !(A.fast_ok && (M.hdr.flags & kFlagFast) &&
                          G <= GRN_MAX_GENES);
-    const int path = exact ? kExact : min_conc > 0.0f ? kClamp : kFast;
+    const int path = exact                            ? kExact
+                     : M.hdr.flags & kFlagConstantTerm ? kConst
+                     : min_conc > 0.0f                ? kClamp
+                                                      : kFast;
     const bool bad = G < 1 || G > GRN_MAX_GENES || M.hdr.n_links < 0 ||
                      M.hdr.n_links > GRN_MAX_LINKS || (sp.n_sm < G && sp.gl == nullptr) ||
                      ((sp.n_sm < G || ST) && G > A.gmax) || (!LOOP && chunks > n_warps) ||

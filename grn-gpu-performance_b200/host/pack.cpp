@@ -127,7 +127,7 @@ grn_status pack_model(const grn_product *products, int n_products,
         if (!(kn > 0) || !(kn <= 1e300) || n > 32) hdr.flags &= ~kFlagFast;
       }
       if (n == 0) {
-        hdr.flags &= ~kFlagFast;  // a constant term: only the exact path has it
+        hdr.flags |= kFlagConstantTerm;
         pl.slot = kConstSlot;  // pow(x, 0) = pow(K, 0) = 1: Hill value 1/2
         pl.a = 0.0f;
         pl.b = 0.0f;
