@@ -333,7 +333,7 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
       // Streaming: only where the planes do not all fit shared memory.
       const int own = v.stream == 2 ? GRN_SCHEDULE_STREAM2 : GRN_SCHEDULE_STREAM;
       if (sched != GRN_SCHEDULE_AUTO && sched != own) continue;
-      if (ft && ft != 512) continue;
+      if (ft && (ft < 32 || ft % 32 != 0 || ft > v.max_threads)) continue;
       const int threads = ft ? ft : v.max_threads;
       const size_t plane_bytes = (size_t)grn::plane_floats(W, H, 1, 0) * sizeof(float);
       const int fit = optin > fixed ? (int)((optin - fixed) / plane_bytes) & ~1 : 0;
