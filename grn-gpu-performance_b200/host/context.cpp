@@ -360,7 +360,13 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
     if (sched == GRN_SCHEDULE_STREAM || sched == GRN_SCHEDULE_STREAM2) continue;
     if (sched == GRN_SCHEDULE_CLUSTER && !v.cluster) continue;
     if (sched != GRN_SCHEDULE_AUTO && sched != GRN_SCHEDULE_CLUSTER && v.cluster) continue;
-    if (sched == GRN_SCHEDULE_FIXED_ITEMS && v.loop) continue;
+    // A forced block of owned chunks takes grids of up to two groups a thread.
+    // Where odd heights make that more chunks than it has warps (a strip is two
+    // rows high), its warps walk them.
+    const bool walks = sched == GRN_SCHEDULE_FIXED_ITEMS && v.loop && !v.cluster &&
+                       v.max_threads == 512 && ft > 0 && ft <= 512 &&
+                       grn::strip_chunks(W, H) * 32 > ft && H * ((W + 3) / 4) <= 2 * ft;
+    if (sched == GRN_SCHEDULE_FIXED_ITEMS && v.loop && !walks) continue;
     if ((sched == GRN_SCHEDULE_WALK_ITEMS || sched == GRN_SCHEDULE_GLOBAL) && !v.loop) continue;
     for (int ci = 0; ci < (v.cluster ? 4 : 1); ++ci) {
       const int C = v.cluster ? kClusterSizes[ci] : 1;
@@ -439,7 +445,7 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
           if (ctas < 1) continue;
           plan.schedule = C > 1                                      ? GRN_SCHEDULE_CLUSTER
                           : (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? GRN_SCHEDULE_GLOBAL
-                          : v.loop                                    ? GRN_SCHEDULE_WALK_ITEMS
+                          : v.loop && !walks                          ? GRN_SCHEDULE_WALK_ITEMS
                                                                       : GRN_SCHEDULE_FIXED_ITEMS;
           plan.threads = threads;
           plan.slot_floats = spills ? 2LL * max_genes * grn::plane_floats(W, H, C, plan.row_pad) : 0;
