@@ -138,6 +138,13 @@ extern "C" grn_status grn_evaluate_batch_noalloc(
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
   const int W = params->dim_x, H = params->dim_y;
+  // A cell needs at least 8 floats of a state slot; grids of more cells than
+  // that leaves room for (whose sizes may not fit 32 bits) go no further.
+  if ((int64_t)W * H > (int64_t)GRN_NOALLOC_SCRATCH_BYTES / 32)
+    return put_error(err_buf, err_buf_len, GRN_ERR_CAPACITY,
+                     "one block's state slot needs more than the " +
+                         std::to_string((size_t)GRN_NOALLOC_SCRATCH_BYTES - slots_off) +
+                         " bytes left of GRN_NOALLOC_SCRATCH_BYTES");
   const bool ragged = (W % 4) != 0;
   const size_t plane_bytes = (size_t)plane_floats(W, H, 1, 0) * sizeof(float);
   const size_t fixed = sim_fixed_smem_bytes();
