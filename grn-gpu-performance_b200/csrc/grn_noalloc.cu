@@ -38,9 +38,17 @@
 namespace grn {
 namespace {
 
+// The second row of an odd height's last strip is read (and dropped) past its
+// plane's zero row.  Planes here hold no row for that: the read lands in the
+// next plane's zero row and, past the last slot, in kOverRead, so that a grid
+// that fills the scratch with its own rows fits.  A slot has at least 8 planes
+// of 3 rows, so a row takes at most 1/24 of the scratch.
+constexpr size_t kOverRead = GRN_NOALLOC_SCRATCH_BYTES / 24;
+
 // Reserved on each GPU when the module loads there, for the life of the
 // process.
-static __device__ __align__(256) unsigned char g_noalloc_scratch[GRN_NOALLOC_SCRATCH_BYTES];
+static __device__ __align__(256) unsigned char
+    g_noalloc_scratch[GRN_NOALLOC_SCRATCH_BYTES + kOverRead];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mutex;
@@ -146,9 +154,12 @@ extern "C" grn_status grn_evaluate_batch_noalloc(
                          std::to_string((size_t)GRN_NOALLOC_SCRATCH_BYTES - slots_off) +
                          " bytes left of GRN_NOALLOC_SCRATCH_BYTES");
   const bool ragged = (W % 4) != 0;
-  const size_t plane_bytes = (size_t)plane_floats(W, H, 1, 0) * sizeof(float);
+  const int64_t plane = (int64_t)(H + 2) * row_floats(W);  // no row past an odd height's
+  const size_t plane_bytes = (size_t)plane * sizeof(float);
   const size_t fixed = sim_fixed_smem_bytes();
-  int fit = (size_t)optin > fixed ? (int)(((size_t)optin - fixed) / plane_bytes) : 0;
+  // Past planes in shared memory, the row that an odd height's last strip reads.
+  const size_t over = (H % 2) * (size_t)row_floats(W) * sizeof(float);
+  int fit = (size_t)optin > fixed + over ? (int)(((size_t)optin - fixed - over) / plane_bytes) : 0;
   fit &= ~1;
   const int max_genes = ph.max_genes;
   // State slots are sized for a class of 4, 8 or 16 genes.
@@ -164,7 +175,7 @@ extern "C" grn_status grn_evaluate_batch_noalloc(
     if (!v.loop && parts < 1) continue;  // more chunks than warps
     const int threads = v.loop ? v.max_threads : chunks * parts * 32;
     const int planes = std::min(fit, 2 * max_genes);
-    const size_t smem = fixed + planes * plane_bytes;
+    const size_t smem = fixed + planes * plane_bytes + (planes > 0 ? over : 0);
     int occ = 0;
     if (sim_occupancy(v, threads, smem, &occ) != cudaSuccess || occ < 1) continue;
     const double score = (double)occ * threads * (v.loop ? 1.0 : 1.25);
@@ -177,7 +188,7 @@ extern "C" grn_status grn_evaluate_batch_noalloc(
       best.planes = planes;
       best.smem_bytes = smem;
       best.blocks_per_sm = occ;
-      best.slot_floats = planes / 2 < max_genes ? 2LL * gmax * plane_floats(W, H, 1, 0) : 0;
+      best.slot_floats = planes / 2 < max_genes ? 2LL * gmax * plane : 0;
     }
   }
   if (best_score < 0)
@@ -217,6 +228,8 @@ extern "C" grn_status grn_evaluate_batch_noalloc(
   a.n_in = params->n_input_morphogens;
   a.n_target = params->n_target_morphogens;
   set_geometry(&a, W, H, 1, 0);
+  a.plane_floats = (int32_t)plane;
+  a.plane_bytes = 4 * a.plane_floats;
   a.gmax = best.gmax;
   a.n_steps = params->num_sim_steps;
   a.fitness_kind = params->fitness_kind;

@@ -1419,7 +1419,12 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
     cr.sm_lo = sp.sm;
     cr.sm_hi = reinterpret_cast<const float *>(smem + dyn);
     cr.gl_lo = A.gstate;
-    cr.gl_hi = A.gstate ? A.gstate + (size_t)gridDim.x * (size_t)A.slot_floats : nullptr;
+    // Planes without a row past an odd height's zero row (the no-allocation
+    // entry's): the last slot's last strip reads one row further.
+    const bool over = C == 1 && (A.H & 1) && A.plane_floats == (A.H + 2) * A.row_floats;
+    cr.gl_hi = A.gstate ? A.gstate + (size_t)gridDim.x * (size_t)A.slot_floats +
+                              (over ? A.row_floats : 0)
+                        : nullptr;
     cr.flag = A.error_flag;
   }
   __syncthreads();

@@ -663,7 +663,9 @@ grn_status grn_evolution_set_surrogate_audit(grn_evolution *evo, int enable);
  * GPU and held until the process exits.  Under CUDA's lazy module loading
  * (the default) the module loads at the first grn_evaluate_batch_noalloc
  * call on a device; a caller that divides the device memory itself makes
- * that first call (one with no models is enough) before it does. */
+ * that first call (one with no models is enough) before it does.  1/24 more
+ * than this size is reserved (a row that the kernel reads past the last state
+ * slot, without using it). */
 #define GRN_NOALLOC_SCRATCH_BYTES (64u << 20)
 
 /* Batch evaluation that allocates no device memory.  No counterpart in the
