@@ -48,7 +48,8 @@ struct alignas(16) PackedHeader {
   int32_t orig_index;  // position of the model in the caller's batch
   int16_t n_genes;     // G: products in use
   int16_t n_links;     // L: links in the program
-  uint32_t lg_mask;    // bit g set: gene g is read by some link (needs lg2)
+  uint32_t lg_mask;    // bit g set: gene g is read by some link (descriptive: the
+                       // kernel takes lg2 per link)
   uint32_t flags;
 };
 
@@ -71,6 +72,16 @@ struct alignas(16) PackedLink {
 static_assert(sizeof(PackedHeader) == 16, "packed header is one word");
 static_assert(sizeof(PackedGene) == 16, "packed gene is one word");
 static_assert(sizeof(PackedLink) == 16, "packed link is one word");
+
+// Relative work of one gene with n links, in instructions per cell: the order of
+// the work queue (a model's is the sum over its genes) and the kernel's
+// distribution of genes over warps.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int gene_work(int n) {
+  return 13 + (n > 0 ? 5 + 5 * n : 0);
+}
 
 // Words of one model record.
 inline int record_words(int n_genes, int n_links) { return 1 + n_genes + n_links; }

@@ -340,10 +340,8 @@ __device__ __forceinline__ float comb(float run, float t) {
   else return comb_and(run, t);
 }
 
-// Relative cost of one gene of a strip, in instructions per cell.
 __device__ __forceinline__ int gene_cost(const PackedGene &g) {
-  const int n = g.n_or + g.n_and;
-  return 13 + (n > 0 ? 5 + 5 * n : 0);
+  return gene_work(g.n_or + g.n_and);
 }
 
 // Builds the program of the model in M (all threads; a barrier follows).

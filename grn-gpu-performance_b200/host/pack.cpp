@@ -163,13 +163,11 @@ grn_status pack_model(const grn_product *products, int n_products,
       return GRN_ERR_CAPACITY;
     }
     if (g.n_or + g.n_and > 0) ++c.reg_genes;
+    c.cost += gene_work(g.n_or + g.n_and) - gene_work(0);
   }
   hdr.n_links = (int16_t)plinks.size();
   c.links = (int)plinks.size();
-  c.lg_genes = __builtin_popcount(hdr.lg_mask);
-  // Relative cost of one cell-step: MUFU ops weigh 8 issue slots' worth of
-  // pipe time, a link ~5 instructions, a gene ~16.
-  c.cost = 8.0 * (c.lg_genes + 2 * c.reg_genes) / 4.0 + 5.0 * c.links + 16.0 * G;
+  c.cost += (double)G * gene_work(0);
 
   const size_t w0 = out->size();
   out->resize(w0 + record_words(G, (int)plinks.size()));

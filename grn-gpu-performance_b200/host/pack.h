@@ -16,7 +16,6 @@ namespace grn {
 struct ModelCost {
   int genes = 0;      // products in use
   int links = 0;      // links in the program
-  int lg_genes = 0;   // genes read by some link (lg2 per cell)
   int reg_genes = 0;  // genes with a non-zero regulation (ex2 + rcp per cell)
   int dif_genes = 0;  // diffusing genes
   double cost = 0;    // relative work of one cell-step
