@@ -357,7 +357,20 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
       out->push_back({plan_cost(ctx, plan, max_genes, n_models, 0), plan});
       continue;
     }
-    if (sched == GRN_SCHEDULE_STREAM || sched == GRN_SCHEDULE_STREAM2) continue;
+    // A forced streaming schedule takes every grid of which a band of one row
+    // would fit shared memory beside 5504 bytes.  Where the block's own data and
+    // the row past an odd band leave less, the planes are walked in global
+    // memory.
+    bool bandless = false;
+    if (sched == GRN_SCHEDULE_STREAM || sched == GRN_SCHEDULE_STREAM2) {
+      const size_t room = optin > fixed ? optin - fixed : 0;
+      const bool two = sched == GRN_SCHEDULE_STREAM2;
+      bandless = v.loop && !v.cluster &&
+                 (two ? stream2_rows(W, H, max_genes, room)
+                      : stream_rows(W, H, max_genes, room, v.max_threads)) < 1 &&
+                 (two ? 8 : 6) * max_genes * row_bytes + 5504 <= optin;
+      if (!bandless) continue;
+    }
     if (sched == GRN_SCHEDULE_CLUSTER && !v.cluster) continue;
     if (sched != GRN_SCHEDULE_AUTO && sched != GRN_SCHEDULE_CLUSTER && v.cluster) continue;
     // A forced block of owned chunks takes grids of up to two groups a thread.
@@ -418,7 +431,7 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
       }
       for (const int threads : sizes)
         for (int gv = 0; gv < (offer_global ? 2 : 1); ++gv) {
-          plan.planes = (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? 0 : smem_planes;
+          plan.planes = (sched == GRN_SCHEDULE_GLOBAL || bandless || gv == 1) ? 0 : smem_planes;
           const bool spills = plan.planes / 2 < max_genes;
           const auto resident = [&](int p, int *ctas) -> grn_status {
             plan.row_pad = p;
@@ -443,7 +456,8 @@ grn_status enumerate_plans(grn_ctx *ctx, int max_genes, int n_models, bool trace
           }
           if (s != GRN_OK) return s;
           if (ctas < 1) continue;
-          plan.schedule = C > 1                                      ? GRN_SCHEDULE_CLUSTER
+          plan.schedule = bandless                                   ? sched
+                          : C > 1                                    ? GRN_SCHEDULE_CLUSTER
                           : (sched == GRN_SCHEDULE_GLOBAL || gv == 1) ? GRN_SCHEDULE_GLOBAL
                           : v.loop && !walks                          ? GRN_SCHEDULE_WALK_ITEMS
                                                                       : GRN_SCHEDULE_FIXED_ITEMS;
