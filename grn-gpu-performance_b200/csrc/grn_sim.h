@@ -179,12 +179,11 @@ GRN_HOST_DEVICE inline int group_row(int i, int Wg, uint32_t inv_wg, int wg_shif
   return Wg == 1 ? i : (int)((uint32_t)(((uint64_t)(uint32_t)i * inv_wg) >> 32) >> wg_shift);
 }
 
-// Whether a count of finished work has come up to `target`, both modulo 2^32:
-// counts grow by up to 32 a step, so long runs wrap, and no count is ever more
-// than a few steps from its target.
-GRN_HOST_DEVICE inline bool count_reached(uint32_t count, uint32_t target) {
-  return (int32_t)(count - target) >= 0;
-}
+// Whether counts of finished work, which grow by at most one per warp of a block
+// and step, stay below 2^31 over n_steps.  (Comparing them modulo 2^32 instead
+// takes an instruction more per poll: 64 x 64, 592 models x 500 steps 5.74 ->
+// 5.77 ms.)
+GRN_HOST_DEVICE inline bool counts_fit(int n_steps) { return n_steps <= 0x7fffffff / 32; }
 
 // SimArgs::change_bound.
 inline float float_below(double x) {

@@ -927,14 +927,14 @@ constexpr uint32_t kMaxPolls = 1u << 24;
 template <bool CL>
 __device__ __forceinline__ bool wait_counts(const StepSync &y, int steps) {
   const uint32_t a = smem_addr(y.wait);
-  const uint32_t target = (uint32_t)y.per_step * (uint32_t)steps;
+  const int target = y.per_step * steps;  // counts_fit
   for (uint32_t i = 0; i < kMaxPolls; ++i) {
-    uint32_t v;
+    int v;
     if (CL && y.edge)
       asm volatile("ld.acquire.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     else
       asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    if (__all_sync(kFull, count_reached(v, target))) {
+    if (__all_sync(kFull, v >= target)) {
       __syncwarp();
       return true;
     }
@@ -1474,7 +1474,8 @@ __global__ void __launch_bounds__(NTMAX, 1) sim_kernel(const SimArgs A) {
   bool free_steps = false;  // the counts' lanes are enough for this grid
   if constexpr (FREE) {
     const int reach = chunk_reach(g);
-    free_steps = min(chunks, 2 * reach + 1) <= (CL ? 30 : 32) && chunks <= kMaxDone;
+    free_steps = min(chunks, 2 * reach + 1) <= (CL ? 30 : 32) && chunks <= kMaxDone &&
+                 counts_fit(A.n_steps);
     sync.wait = s_done + min(max(own - reach, 0) + lane, min(own + reach, chunks - 1));
     sync.per_step = splits;
     if constexpr (CL) {

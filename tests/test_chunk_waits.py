@@ -1,8 +1,8 @@
 """The bounded waits of steps without a block barrier.  A count that never
 comes (test hook): the warps that wait for it give up together, the block or
 the whole cluster leaves, the call reports it within seconds, and the same
-context then gives the right result.  Counts of long runs wrap (CPU, over the
-kernel's own header)."""
+context then gives the right result.  Runs whose counts could overflow keep the
+barrier (CPU, over the kernel's own header)."""
 import os
 import subprocess
 import time
@@ -17,7 +17,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 
 
-def test_counts_wrap(tmp_path):
+def test_runs_whose_counts_could_overflow(tmp_path):
     exe = str(tmp_path / "chunk_counts")
     subprocess.run(["g++", "-std=c++17", "-O2", "-I" + os.path.join(CUDA_HOME, "include"),
                     os.path.join(ROOT, "tests", "cpp", "chunk_counts.cpp"), "-o", exe], check=True)
