@@ -486,7 +486,8 @@ cudaError_t mlp_transpose(int rows, int cols, const __nv_bfloat16 *src, int64_t 
 }
 
 cudaError_t mlp_gather_rows(int rows, int width, const int32_t *idx, const int *first,
-                            const __nv_bfloat16 *src, const float *tsrc, __nv_bfloat16 *dst, float *tdst,
+                            const __nv_bfloat16 *src, const float *tsrc, __nv_bfloat16 *dst,
+                            float *tdst,
                             __nv_bfloat16 *dstT, int64_t ldt, cudaStream_t st) {
   if (rows < 1) return cudaSuccess;
   rows_to_bf16_kernel<<<tile_grid(rows, width), dim3(kTile, 8), 0, st>>>(

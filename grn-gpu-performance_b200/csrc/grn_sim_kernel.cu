@@ -9,16 +9,20 @@
 //     model from an atomic work counter (the host orders models by cost,
 //     longest first);
 //   - a model's state lives in shared memory for all Euler steps (planar
-//     [gene][y][x] FP32, rows padded to float4 groups), double buffered
-//     (one barrier per step); genes that do not fit use the same code on
-//     double-buffered global-memory slots, and grids too large for shared
-//     memory stream bands of rows through it (or split across a cluster);
+//     [gene][y][x] FP32, rows padded to float4 groups), double buffered;
+//     genes that do not fit use the same code on double-buffered
+//     global-memory slots, and grids too large for shared memory stream bands
+//     of rows through it (or split across a cluster);
+//   - one block (or cluster) barrier per step where the step's maximum may end
+//     the simulation or warps walk their items; owned chunks otherwise wait for
+//     the counts of the chunks next to their own (see "steps without a block
+//     barrier");
 //   - the work of a step is cut into warp items: 32 strips of 4 columns x 2
 //     rows, for one gene or all of them (see "the step" below).  A thread
 //     loads its own strip's rows once for both rows' neighbour sums; left and
-//     right neighbours come from 32-bit loads next to the group (every
-//     padded row ends in zero cells, so a row's borders read 0 without
-//     tests);
+//     right neighbours come from the neighbouring lanes, and from 32-bit loads
+//     next to the group where no lane holds them (every padded row ends in zero
+//     cells, so a row's borders read 0 without tests);
 //   - regulation is evaluated in exponent form (grn_packed.h): per link lg2
 //     of the regulator's cells, one FMA + min/max, and per regulated gene
 //     ex2 + rcp, on the MUFU pipe;
@@ -222,13 +226,13 @@ constexpr size_t kCsumOffset = kCmaxOffset + 2 * kMaxCluster * 32 * 4;
 // time-out flag (int).
 constexpr size_t kMbarOffset = (kCsumOffset + 8 + 15) & ~size_t(15);
 constexpr size_t kStreamFailOffset = kMbarOffset + 16;
-// Bounds-checked build only: the regions that state accesses are checked
-// against (CheckRegions).
 // Steps without a block barrier (StepSync): finished work per chunk (int [32]),
 // the halo counts (int [2]) and the last vote with a rate (int).
 constexpr int kMaxDone = 32;
 constexpr int kDoneInts = kMaxDone + 3;
 constexpr size_t kDoneOffset = kStreamFailOffset + 16;
+// Bounds-checked build only: the regions that state accesses are checked
+// against (CheckRegions).
 constexpr size_t kCheckOffset = (kDoneOffset + kDoneInts * 4 + 15) & ~size_t(15);
 constexpr size_t kCheckBytes = GRN_BOUNDS_CHECK ? 64 : 0;
 constexpr size_t kStateOffset = (kCheckOffset + kCheckBytes + 127) & ~size_t(127);
@@ -408,14 +412,16 @@ __device__ __forceinline__ void build_program(const ModelSmem &M, ProgSmem &P, i
 //
 // A state plane holds the W x H grid as rows of RS = row_floats(W) floats
 // (whole float4 groups, ending in at least one zero cell) plus one zero row
-// above and one below, and rows for whole strips (strip_rows):
-// PS = plane_floats, row y at row_offset(y + 1): `pad` zero floats follow the
+// above and one below, and rows for whole strips (strip_rows; the
+// no-allocation entry's planes have none, and their over-reads land in what
+// follows): PS = plane_floats, row y at row_offset(y + 1): `pad` zero floats follow the
 // row above the grid and then every two rows, i.e. every row of strips
-// (strip_pad; 0 where streamed).  The zero rows make the up/down neighbours of the first and last rows read +0.0, which leaves the
-// reference's neighbour sum unchanged.  Steps write data groups only; when W
-// is not a multiple of 4 the cells past W of a row's last group are written
-// as 0, otherwise a zero group ends the row: either way the cell after a
-// row's last cell, and the cell before the next row's first, read 0.
+// (strip_pad; 0 where streamed).  The zero rows make the up/down neighbours of
+// the first and last rows read +0.0, which leaves the reference's neighbour
+// sum unchanged.  Steps write data groups only; when W is not a multiple of 4
+// the cells past W of a row's last group are written as 0, otherwise a zero
+// group ends the row: either way the cell after a row's last cell, and the cell
+// before the next row's first, read 0.
 //
 // A cluster-split launch gives each CTA of a cluster a band of rows
 // [y0, y0 + H) of the Hg-row grid, held the same way: one halo row above and
@@ -1132,9 +1138,9 @@ __device__ __forceinline__ void band_step(int path, const ProgSmem &P, const flo
 // issues the copy of band b + 2 into its stage.  Bound by issue slots and the
 // MUFU pipe (each about half busy) and by the waits for them, so warps help:
 // 256 x 256, 8 genes, 592 models x 100 steps, kernel ms with 16 warps and a
-// barrier per band 54.3, 20 warps 53.0, 20 warps without the barrier 50.4.
-// In a 50-step sample 16 warps took 1.10x as long without the barrier, 24
-// warps (72 registers, bands of 6 rows) 1.30x.
+// barrier per band 54.3, 20 warps 53.0; without the barrier 16 warps 54.6, 18
+// warps 54.7, 20 warps 50.5.  24 warps (72 registers, bands of 6 rows) took
+// 1.30x as long in a 50-step sample.
 // mphase holds each stage's
 // next wait parity across steps; `counts` are the stages' finished warps (0
 // between steps) and the copies issued for each in this step.
